@@ -51,71 +51,115 @@ __device__ __forceinline__ void epilogue_store(double v, int r, int c, double *C
     C[off] = out;
 }
 
+// One BM x BN output tile over the K slice blockIdx.z.  The FP64 pipe retires
+// two FMA per clock per SM, so a tile's FMAs, not its loads, bound it: the
+// micro-tile is only as large as the load count asks (1 x 1 at 16 x 16), the
+// next K step's operands are loaded into registers while the current one is
+// multiplied from a two-stage shared buffer (one block barrier per step), and
+// what the masks or the matrix's edge leave out is not multiplied:
+// the K range is cut to what triangular masks leave nonzero, a warp whose
+// outputs all lie outside the matrix skips its FMAs, and with upper_only a
+// tile below the diagonal returns at once.  Against the same kernel on fixed
+// 32 x 32 tiles with 256-deep K slices and unpipelined loads: the 617 products
+// of a 1413 x 692 recursive QR 22.1 -> 7.1 ms, the 133 of 4000 x 1000 (tiles
+// of 256) 21.6 -> 16.1 ms, the upper 64 x 64 Gram of 262,144 rows 2.23 -> 1.4 ms.
 template <int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+__global__ void __launch_bounds__(256)
     k_gemm(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e,
            double *part)
 {
-    constexpr int RT = BM / TM;  // threads along rows
-    constexpr int NTH = (BM / TM) * (BN / TN);
-    __shared__ double As[BK][BM];
-    __shared__ double Bs[BK][BN];
-    const int tid = threadIdx.x;
-    const int tr = tid % RT, tc = tid / RT;
+    constexpr int RT = BM / TM, CT = BN / TN;  // threads along rows, columns
+    constexpr int NTH = 256;
+    static_assert(RT * CT == NTH, "one micro-tile per thread");
+    constexpr int LA = BM * BK / NTH, LB = BN * BK / NTH;
+    // rows of As and Bs are padded to an odd length: a transposed operand's
+    // stores walk a column of them
+    __shared__ double As[2][BK][BM + 1];
+    __shared__ double Bs[2][BK][BN + 1];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // a warp covers 8 row threads x 4 column threads
+    const int tr = (lane & 7) + 8 * (warp % (RT / 8)), tc = (lane >> 3) + 4 * (warp / (RT / 8));
     const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
-    const int kbeg = blockIdx.z * kchunk;
-    const int kend = min(K, kbeg + kchunk);
+    if (e.upper_only && row0 > col0 + BN - 1) return;
+    int kbeg = blockIdx.z * kchunk;
+    int kend = min(K, kbeg + kchunk);
+    // rows [row0, row0 + BM) of op(A) and columns [col0, col0 + BN) of op(B)
+    // are zero outside [kbeg, kend) under the stored operand's triangular mask
+    {
+        const bool lowA = A.mask == M_UNIT_LOWER || A.mask == M_LOWER, upA = A.mask == M_UPPER || A.mask == M_UNIT_UPPER;
+        const bool lowB = B.mask == M_UNIT_LOWER || B.mask == M_LOWER, upB = B.mask == M_UPPER || B.mask == M_UNIT_UPPER;
+        if (A.trans == NT ? lowA : upA) kend = min(kend, row0 + BM);
+        if (A.trans == NT ? upA : lowA) kbeg = max(kbeg, row0 / BK * BK);
+        if (B.trans == NT ? upB : lowB) kend = min(kend, col0 + BN);
+        if (B.trans == NT ? lowB : upB) kbeg = max(kbeg, col0 / BK * BK);
+    }
+    const bool live = row0 + 8 * (warp % (RT / 8)) < M && col0 + 4 * (warp / (RT / 8)) < N;
     double acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0;
 
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        for (int idx = tid; idx < BM * BK; idx += NTH) {
-            int r, k;
-            if (A.trans == NT) {
-                r = idx % BM;
-                k = idx / BM;
-            } else {
-                k = idx % BK;
-                r = idx / BK;
-            }
-            int gr = row0 + r, gk = k0 + k;
-            As[k][r] = (gr < M && gk < kend) ? op_elem(A, gr, gk) : 0.0;
+    double ra[LA], rb[LB];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < LA; u++) {
+            const int idx = tid + u * NTH;
+            const int r = A.trans == NT ? idx % BM : idx / BK, k = A.trans == NT ? idx / BM : idx % BK;
+            const int gr = row0 + r, gk = k0 + k;
+            ra[u] = (gr < M && gk < kend) ? op_elem(A, gr, gk) : 0.0;
         }
-        for (int idx = tid; idx < BN * BK; idx += NTH) {
-            int c, k;
-            if (B.trans == NT) {
-                k = idx % BK;
-                c = idx / BK;
-            } else {
-                c = idx % BN;
-                k = idx / BN;
-            }
-            int gc = col0 + c, gk = k0 + k;
-            Bs[k][c] = (gc < N && gk < kend) ? op_elem(B, gk, gc) : 0.0;
+#pragma unroll
+        for (int u = 0; u < LB; u++) {
+            const int idx = tid + u * NTH;
+            const int c = B.trans == NT ? idx / BK : idx % BN, k = B.trans == NT ? idx % BK : idx / BN;
+            const int gc = col0 + c, gk = k0 + k;
+            rb[u] = (gc < N && gk < kend) ? op_elem(B, gk, gc) : 0.0;
         }
+    };
+    load(kbeg);
+    int buf = 0;
+    for (int k0 = kbeg; k0 < kend; k0 += BK, buf ^= 1) {
+#pragma unroll
+        for (int u = 0; u < LA; u++) {
+            const int idx = tid + u * NTH;
+            if (A.trans == NT)
+                As[buf][idx / BM][idx % BM] = ra[u];
+            else
+                As[buf][idx % BK][idx / BK] = ra[u];
+        }
+#pragma unroll
+        for (int u = 0; u < LB; u++) {
+            const int idx = tid + u * NTH;
+            if (B.trans == NT)
+                Bs[buf][idx % BK][idx / BK] = rb[u];
+            else
+                Bs[buf][idx / BN][idx % BN] = rb[u];
+        }
+        // one barrier per step: the buffer written two steps later was last
+        // read before the barrier of the step between
         __syncthreads();
+        if (k0 + BK < kend) load(k0 + BK);
+        if (live) {
 #pragma unroll
-        for (int k = 0; k < BK; k++) {
-            double a[TM], b[TN];
+            for (int k = 0; k < BK; k++) {
+                double a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < TM; i++) a[i] = As[k][tr + i * RT];
+                for (int i = 0; i < TM; i++) a[i] = As[buf][k][tr + i * RT];
 #pragma unroll
-            for (int j = 0; j < TN; j++) b[j] = Bs[k][tc + j * (BN / TN)];
+                for (int j = 0; j < TN; j++) b[j] = Bs[buf][k][tc + j * CT];
 #pragma unroll
-            for (int i = 0; i < TM; i++)
+                for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < TN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            }
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++) {
-            int r = row0 + tr + i * RT, c = col0 + tc + j * (BN / TN);
+            int r = row0 + tr + i * RT, c = col0 + tc + j * CT;
             if (r < M && c < N) {
                 if (part)
                     part[(size_t)blockIdx.z * M * N + (size_t)r + (size_t)c * M] = acc[i][j];
@@ -125,15 +169,27 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         }
 }
 
+// Sum of the K slices' partial products in slice order, eight loads in flight
+// per thread.
 __global__ void k_splitk_reduce(int M, int N, int splits, const double *part, double *C, int ldc,
                                 GemmEpi e)
 {
     size_t total = (size_t)M * N;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
+        const int r = (int)(idx % M), c = (int)(idx / M);
+        if (e.upper_only && r > c) continue;
         double s = 0.0;
-        for (int z = 0; z < splits; z++) s += part[(size_t)z * total + idx];
-        int r = (int)(idx % M), c = (int)(idx / M);
+        const double *p = part + idx;
+        int z = 0;
+        for (; z + 8 <= splits; z += 8, p += 8 * total) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = p[(size_t)u * total];
+#pragma unroll
+            for (int u = 0; u < 8; u++) s += v[u];
+        }
+        for (; z < splits; z++, p += total) s += *p;
         epilogue_store(s, r, c, C, ldc, e);
     }
 }
@@ -143,18 +199,72 @@ static int num_sm() { return sm_count(); }
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Tile and K split of an M x N x K product.  The FP64 pipe makes every tile
+// cost BM BN kchunk / 2 clocks of its SM whatever its shape, so the plan with
+// the least work on the busiest SM wins: small tiles and fine K slices when
+// the output has few tiles, 64 x 64 when it has many (fewer loads).  A split
+// adds the reduction launch (~3 us) and splits / 2 clocks per output.  A 32 x
+// 350 x 1316 product: 106 us on 66 CTAs (32 x 32 x 264, FP64 pipe 21 % busy),
+// its FMAs take 23 us on all SMs.
+struct GemmPlan {
+    int tile, splits, kchunk;
+};
+
+static GemmPlan gemm_plan(int M, int N, int K, long long part_len, bool upper_only)
+{
+    const double sm = num_sm();
+    const long long out = (long long)M * N;
+    GemmPlan best{32, 1, K > 0 ? K : 1};
+    double best_t = 1e300;
+    for (int t = 16; t <= 64; t *= 2) {
+        if (t < 64 && ceil_div(N, t) > 65535) continue;  // grid.y limit
+        double tiles = (double)ceil_div(M, t) * ceil_div(N, t);
+        // upper_only: the tiles below the diagonal return at once
+        if (upper_only) {
+            const double d = ceil_div(M < N ? M : N, t);
+            tiles -= 0.5 * d * (d - 1) + (double)(ceil_div(M, t) - d) * ceil_div(N, t);
+        }
+        // clocks of a K step of 16 that the pipe does not cover: the loads'
+        // latency and the barrier
+        const double step = 700.0;
+        for (int per = 0; per <= 8; per++) {
+            // about `per` CTAs on every SM (0: no split)
+            int splits = 1;
+            if (per > 0) {
+                splits = (int)(per * sm / tiles);
+                if (splits > K / 32) splits = K / 32;
+                if (splits > 128) splits = 128;
+                if ((long long)splits * out > part_len) splits = (int)(part_len / out);
+                if (splits < 2) continue;
+            }
+            int kchunk = K > 0 ? K : 1;
+            if (splits > 1) {
+                kchunk = ceil_div(ceil_div(K, splits), 16) * 16;
+                splits = ceil_div(K, kchunk);
+                if (splits < 2) continue;
+            }
+            const double ctas = tiles * splits;
+            const double waves = ceil(ctas / sm);
+            const double work = 0.5 * t * t * kchunk;  // clocks of one CTA alone on its SM
+            // co-resident CTAs share the pipe and hide each other's latency
+            const double lat = ceil_div(kchunk, 16) * step + 1500.0;
+            double time = waves * work > lat ? waves * work + 0.1 * lat : lat + 0.1 * waves * work;
+            if (splits > 1) time += 6000.0 + 0.5 * splits * out / sm;
+            // wider tiles load less per FMA: prefer them when equal
+            time *= t == 16 ? 1.06 : (t == 32 ? 1.02 : 1.0);
+            if (time < best_t) {
+                best_t = time;
+                best = GemmPlan{t, splits, kchunk};
+            }
+        }
+    }
+    return best;
+}
+
 int gemm_splits(int M, int N, int K, long long part_len)
 {
-    if (M <= 0 || N <= 0 || K <= 512) return 1;
-    const int BM = (M * (long long)N >= 64LL * 64 * 2 * num_sm()) ? 64 : 32;
-    long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BM);
-    if (tiles >= 2 * num_sm()) return 1;
-    int s = ceil_div(K, 256);
-    s = s < ceil_div(4 * num_sm(), tiles) ? s : ceil_div(4 * num_sm(), tiles);
-    if (s > 128) s = 128;
-    long long fit = part_len / ((long long)M * N);
-    if (s > fit) s = (int)fit;
-    return s < 2 ? 1 : s;
+    if (M <= 0 || N <= 0) return 1;
+    return gemm_plan(M, N, K, part_len, false).splits;
 }
 
 void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e,
@@ -167,33 +277,27 @@ void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const G
         return;
     }
     cudaStream_t st = stream();
-    int splits = part ? gemm_splits(M, N, K, part_len) : 1;
-    const bool big = (M * (long long)N >= 64LL * 64 * 2 * num_sm());
-    int kchunk = K > 0 ? K : 1;
-    if (splits > 1) {
-        kchunk = ceil_div(ceil_div(K, splits), 16) * 16;
-        splits = ceil_div(K, kchunk);
-    }
-    double *p = splits > 1 ? part : nullptr;
+    const GemmPlan p = gemm_plan(M, N, K, part ? part_len : 0, e.upper_only != 0);
+    double *pp = p.splits > 1 ? part : nullptr;
+    dim3 grid(ceil_div(M, p.tile), ceil_div(N, p.tile), p.splits);
     trace_begin();
-    if (big) {
-        dim3 grid(ceil_div(M, 64), ceil_div(N, 64), splits);
-        k_gemm<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p);
-    } else {
-        dim3 grid(ceil_div(M, 32), ceil_div(N, 32), splits);
-        k_gemm<32, 32, 16, 2, 2><<<grid, 256, 0, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p);
-    }
+    if (p.tile == 64)
+        k_gemm<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
+    else if (p.tile == 32)
+        k_gemm<32, 32, 16, 2, 2><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
+    else
+        k_gemm<16, 16, 32, 1, 1><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
     note_launch(tag);
-    if (splits > 1) splitk_reduce(M, N, splits, part, C, ldc, e);
+    if (p.splits > 1) splitk_reduce(M, N, p.splits, part, C, ldc, e);
 }
 
 void splitk_reduce(int M, int N, int splits, const double *part, double *C, int ldc, const GemmEpi &e)
 {
     long long total = (long long)M * N;
-    int blocks = ceil_div(total, 256);
-    if (blocks > 4 * num_sm()) blocks = 4 * num_sm();
+    int blocks = ceil_div(total, 128);
+    if (blocks > 8 * num_sm()) blocks = 8 * num_sm();
     trace_begin();
-    k_splitk_reduce<<<blocks, 256, 0, stream()>>>(M, N, splits, part, C, ldc, e);
+    k_splitk_reduce<<<blocks, 128, 0, stream()>>>(M, N, splits, part, C, ldc, e);
     note_launch("splitk_reduce");
 }
 
