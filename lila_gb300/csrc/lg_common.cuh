@@ -159,6 +159,12 @@ int precision();
 bool panel_coop_fits(int m, int nb);
 long long panel_coop_work(int nb);
 bool panel_coop(int m, int nb, double *A, int lda, double *T, int ldt, double *work);
+// Householder QR of a matrix that fits one CTA's shared memory in one launch
+// (lg_panel.cu): V and R in A, the T tiles of the reflectors [i, i + n) of
+// the global numbering (T points at column i; i = 0 and mt >= n: one n x n T)
+// and, unless Q is null, the explicit Q.  False (nothing enqueued) when the
+// matrix does not fit.
+bool qr_small(int m, int n, double *A, int lda, double *T, int ldt, int i, int mt, double *Q, int ldq);
 
 // Copies / element-wise helpers.
 void copy2d(int m, int n, const double *src, int lds, double *dst, int ldd);
@@ -267,6 +273,21 @@ __device__ __forceinline__ double rsqrt_nr(double d)
     }
     // 1 / sqrt(d) = y 2^(adj - k)
     return __hiloint2double(__double2hiint(y) + (adj - k) * 1048576, __double2loint(y));
+}
+
+// 1 / d for a positive d in [2^-1000, 2^1000]: Newton–Raphson y <- y + y (1 - d y),
+// two steps from a single-precision reciprocal of d's mantissa (its error
+// below 2^-22 becomes ~2^-44, then rounding level), four FP64 operations.
+__device__ __forceinline__ double rcp_nr(double d)
+{
+    const int hi = __double2hiint(d), lo = __double2loint(d);
+    const float fm = __int_as_float((127 << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)lo >> 29));
+    const unsigned yb = __float_as_uint(__frcp_rn(fm));  // in (1/2, 1]
+    const int e = (int)(yb >> 23) - 127 - ((hi >> 20) - 1023);
+    double y = __hiloint2double((int)(((unsigned)(e + 1023) << 20) | ((yb & 0x7FFFFFu) >> 3)), (int)((yb & 7u) << 29));
+#pragma unroll
+    for (int it = 0; it < 2; it++) y = fma(y, fma(-d, y, 1.0), y);
+    return y;
 }
 #endif
 

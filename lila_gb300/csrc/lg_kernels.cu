@@ -755,10 +755,59 @@ __global__ void k_larft_from_gram(int k, const double *G, int ldg, const double 
     }
 }
 
+// The same T for k <= 64 by doubling, T12 = -T11 (G12 T22) for blocks of 1, 2,
+// 4, .. columns (dlarft's recurrence regrouped, as lila_dlarft_connect does):
+// 2 log2(k) block barriers instead of 2 k, all operands in shared memory.
+// The column recurrence on global memory took ~110 us for k = 64, this ~20.
+constexpr int LARFT_LD = 65;
+__global__ void __launch_bounds__(512) k_larft_small(int k, const double *G, int ldg, const double *tau, double *T,
+                                                     int ldt)
+{
+    extern __shared__ double lf[];
+    double *Gs = lf, *Ts = lf + 64 * LARFT_LD, *Ys = lf + 2 * 64 * LARFT_LD;
+    for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
+        const int r = idx % k, c = idx / k;
+        if (r < c) Gs[r + c * LARFT_LD] = G[(size_t)r + (size_t)c * ldg];
+        if (r == c) Ts[r + c * LARFT_LD] = tau[c];
+    }
+    __syncthreads();
+    for (int b = 1; b < k; b *= 2) {
+        const int pairs = (k + 2 * b - 1) / (2 * b), total = pairs * b * b;
+        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+            const int r0 = 2 * b * (idx / (b * b)), r = r0 + idx % b, c0 = r0 + b, c = c0 + idx / b % b;
+            if (c >= k) continue;
+            double s = 0.0;
+            for (int q = c0; q <= c; q++) s = fma(Gs[r + q * LARFT_LD], Ts[q + c * LARFT_LD], s);
+            Ys[r + c * LARFT_LD] = s;
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+            // rows by the slow index: a warp's sums have the same length
+            const int r0 = 2 * b * (idx / (b * b)), r = r0 + idx / b % b, c = r0 + b + idx % b;
+            if (c >= k) continue;
+            double s = 0.0;
+            for (int q = r; q < r0 + b; q++) s = fma(Ts[r + q * LARFT_LD], Ys[q + c * LARFT_LD], s);
+            Ts[r + c * LARFT_LD] = -s;
+        }
+        __syncthreads();
+    }
+    for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
+        const int r = idx % k, c = idx / k;
+        if (r <= c) T[(size_t)r + (size_t)c * ldt] = Ts[r + c * LARFT_LD];
+    }
+}
+
 void larft_from_gram(int k, const double *G, int ldg, const double *tau, double *T, int ldt)
 {
     if (k <= 0) return;
-    k_larft_from_gram<<<1, 256, (size_t)k * sizeof(double), stream()>>>(k, G, ldg, tau, T, ldt);
+    trace_begin();
+    if (k <= 64) {
+        constexpr int smem = 3 * 64 * LARFT_LD * (int)sizeof(double);
+        cudaFuncSetAttribute(k_larft_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        k_larft_small<<<1, 512, smem, stream()>>>(k, G, ldg, tau, T, ldt);
+    } else {
+        k_larft_from_gram<<<1, 256, (size_t)k * sizeof(double), stream()>>>(k, G, ldg, tau, T, ldt);
+    }
     note_launch("larft_from_gram");
 }
 

@@ -270,6 +270,8 @@ static void dgeqr3_dev(int m, int n, double *A, int lda, double *T, int ldt, Wor
         larfg(m, A, T);
         return;
     }
+    // or in one CTA when it fits there
+    if (n <= 64 && qr_small(m, n, A, lda, T, ldt, 0, n, nullptr, 0)) return;
     int n1 = n / 2, n2 = n - n1;
     dgeqr3_dev(m, n1, A, lda, T, ldt, w);
     Work w2 = w;
@@ -497,9 +499,32 @@ static void mt_hr(int m, int n, int i, int mt, double *A, int lda, double *T, in
     }
 }
 
+// The leaf's and the recursion's results are the Householder QR of the block
+// with its T tiles, whatever the recursion (leaf 0, or leaf 1 with a
+// Householder panel): one launch can compute them when the block fits one CTA
+// (Q given: with the explicit Q).  One CTA does ~3,400 FP64 multiply-adds per
+// us plus ~1.5 us of dependent chain per column (2.5 with Q); the launches it
+// replaces cost ~80 us per panel (tile or recursion leaf) beside the panels'
+// own columns.  87 x 53 in tiles of 4: 0.32 ms against 3.3; 128 x 128 in one
+// tile: 1.0 ms against ~0.5, so that one keeps its launches.
+static bool small_block(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T, int ldt, double *Q,
+                        int ldq)
+{
+    if (!(lp[1] == 0 || (lp[1] == 1 && lp[2] != 2)) || n < 2) return false;
+    const double ml = m - i, fma = (ml - n / 3.0) * n * n;
+    const double panel = fma / 3400.0 + 1.5 * n, one = Q ? 2.0 * fma / 3400.0 + 2.5 * n : panel;
+    int leaves = 1;
+    for (int w = n; w > lp[3]; w = (w + 1) / 2) leaves *= 2;
+    const int tiles = (i + n - 1) / mt - i / mt + 1;
+    if (one > 80.0 * imax(leaves, tiles) + (panel < 5.0 * n ? panel : 5.0 * n)) return false;
+    const size_t at = i + (size_t)i * lda;
+    return qr_small(m - i, n, A + at, lda, T + (size_t)i * ldt, ldt, i, mt, Q ? Q + i + (size_t)i * ldq : nullptr, ldq);
+}
+
 static void leaf(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T, int ldt,
                  double *Q, int ldq, Work w)
 {
+    if (small_block(lp, m, n, i, mt, A, lda, T, ldt, Q, ldq)) return;
     switch (lp[1]) {
     case 0: mt_l(m, n, i, mt, A, lda, T, ldt, Q, ldq, w); break;
     case 1: mt_hh(lp, m, n, i, mt, A, lda, T, ldt, Q, ldq, w); break;
@@ -512,6 +537,7 @@ static void leaf(const int *lp, int m, int n, int i, int mt, double *A, int lda,
 static void recursive(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T,
                       int ldt, double *Q, int ldq, Work w)
 {
+    if (small_block(lp, m, n, i, mt, A, lda, T, ldt, Q, ldq)) return;
     if (n <= lp[3]) {
         leaf(lp, m, n, i, mt, A, lda, T, ldt, Q, ldq, w);
         return;
@@ -592,6 +618,7 @@ static void v03_mt_l(int m, int n, int i, int mt, double *A, int lda, double *T,
 static void v03_leaf(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T, int ldt,
                      Work w)
 {
+    if (small_block(lp, m, n, i, mt, A, lda, T, ldt, nullptr, 0)) return;
     if (lp[1] == 0) v03_mt_l(m, n, i, mt, A, lda, T, ldt, w);
     if (lp[1] == 1) v03_mt_hh(lp[2], m, n, i, mt, A, lda, T, ldt, w);
 }
@@ -600,6 +627,7 @@ static void v03_leaf(const int *lp, int m, int n, int i, int mt, double *A, int 
 static void v03_recursive(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T,
                           int ldt, Work w)
 {
+    if (small_block(lp, m, n, i, mt, A, lda, T, ldt, nullptr, 0)) return;
     if (n < lp[3] || n <= 1) {
         v03_leaf(lp, m, n, i, mt, A, lda, T, ldt, w);
         return;

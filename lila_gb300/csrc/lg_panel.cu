@@ -1,28 +1,37 @@
-// lg_panel.cu -- Householder QR of an m x nb panel (nb <= 64) in one
-// cooperative launch: the reflectors of dgeqr3 (lila-c/dgeqr3.c:3-114,
-// LAPACK dlarfg conventions) computed column by column with every CTA holding
-// a block of rows in shared memory for the whole panel, one grid barrier per
-// column.
+// lg_panel.cu -- Householder QR of panels and of small matrices in one launch,
+// column by column out of shared memory (the reflectors of dgeqr3,
+// lila-c/dgeqr3.c:3-114, LAPACK dlarfg conventions).
 //
-// Before the barrier of column j every CTA publishes, from its rows below
-// the pivot (column j as updated by the reflectors before it): its sum of
-// squares of column j, its dot products d_c = sum_r x_j(r) A(r, c) with the
-// trailing columns c > j, and, from the CTA that owns row j, alpha = A(j, j)
-// and the pivot row A(j, c).  After the barrier every CTA adds the partials
-// in CTA order (so all CTAs get the same beta, tau bit for bit), forms
-// sc = 1 / (alpha - beta), scales its part of the column into v, and
-// updates its rows with w_c = v^T A(:, c) = A(j, c) + sc d_c:
-// A(r, c) -= v_r tau w_c.  It then publishes the partials of column j + 1.
-// The partials live in two alternating slot buffers, so a CTA can write
-// column j + 1's while others still read column j's.
-// T then follows from V^T V (dlarft recurrence, lg_kernels.cu).
+// What bounds both kernels is the FP64 pipe (2 lanes per clock per SM: a warp
+// instruction holds its sub-partition for 64 clocks whether its lanes carry
+// work or not) and the chain from one column to the next.  So a group of LG
+// lanes owns a column: its dot products and updates run down the rows with
+// full warps and only the last log2(LG) additions are shuffles, the reflector
+// is formed by one lane with Newton-Raphson reciprocals, and the column is not
+// scaled into v before its trailing columns are updated (v_r = x_r sc enters
+// through the factor sc w_c; the scaling happens on the way out).
 //
-// The grid barrier is a monotonic counter: arrival = fence + reduction, wait
-// = acquire loads until the count reaches (barrier index + 1) x CTAs (the
-// acquire load orders the CTA's later reads, so no fence follows it).
-// All CTAs are co-resident (cudaLaunchCooperativeKernel).  Every wait is
-// bounded (iteration and clock limits); a wait that gives up sets
-// ST_WAIT_TIMEOUT and the CTA returns.
+// k_panel (m x nb, nb <= 64, a block of rows per CTA, cooperative launch).
+// For column j every CTA publishes, from its rows below the pivot, its dot
+// products d_c = sum_r x_j(r) A(r, c) with every column (c = j: the sum of
+// squares; c < j: for T), and the CTA that owns row j the pivot row A(j, c).
+// One warp per column, spread over the CTAs, adds the CTAs' partials of its
+// column in a fixed order and publishes the total (so all CTAs get the same
+// beta, tau bit for bit); then every CTA updates its rows with w_c = A(j, c) +
+// sc d_c.  Adding the partials in every CTA instead saves one trip through L2
+// but costs G FP64 additions per column and CTA: 7.1 us per column at 4000 x
+// 64 against 4.8 us this way (11.7 us before, with 5 shuffle additions per
+// column and a counter barrier).
+// The exchange has no separate barrier: a value travels as two 8-byte words
+// of (32 data bits, 32-bit column tag), and its reader polls until both tags
+// are column j's.  Slots alternate between two buffers: a slot of column j is
+// written again for column j + 2 only by a CTA that has every total of column
+// j + 1, to which every CTA contributed after it had read column j's.  The
+// slots are zeroed before the launch; every wait is bounded (clock limit); one
+// that gives up sets ST_WAIT_TIMEOUT and the CTA returns.
+//
+// k_qr_small: the whole matrix in one CTA's shared memory, V, R, the T tiles
+// and (optionally) the explicit Q in one launch.
 #include <math.h>
 
 #include "lg_common.cuh"
@@ -30,176 +39,413 @@
 namespace lg {
 namespace pnl {
 
-constexpr int NT = 256, MAXNB = 64;
+constexpr int NT = 256, MAXNB = 64;  // threads of a panel CTA, most columns
+constexpr int NTS = 512;              // threads of the one-CTA kernel
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+// Lanes per column for n columns in a CTA of `threads`: as few as cover the
+// block, since every doubling adds a shuffle addition per dot product.  128
+// threads would spend fewer still, but one warp per sub-partition does not
+// hide its loads (87 x 53 in one CTA: 504 us with 128 threads, 349 with 256,
+// 322 with 512; the 4000 x 64 panel 317 us with 128, 309 with 256).
+__host__ __device__ inline int lanes_for(int threads, int n)
 {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return threads / 64 * (n > 32 ? 1 : (n > 16 ? 2 : 4));
+}
+// The leading dimension in shared memory: lanes modulo 16, so the 16 / lanes
+// columns that a half warp reads fall into different banks.
+__host__ __device__ inline int pad_ld(int rows, int lanes) { return ((rows - lanes + 15) / 16 * 16) + lanes; }
+
+struct Reflector {
+    double beta, tau, sc;
+};
+
+// dlarfg from alpha and the sum of squares below it; `below` says whether
+// anything below the pivot is nonzero.  |beta| = sqrt(alpha^2 + ss) corrected
+// to rounding level, tau = 1 + |alpha| / |beta|, sc = 1 / (alpha - beta).
+__device__ __forceinline__ Reflector reflector(double alpha, double ss, bool below)
+{
+    if (!below) return Reflector{alpha, 0.0, 0.0};
+    const double s = fma(alpha, alpha, ss), a = fabs(alpha);
+    if (s >= 1e-290 && s <= 1e290) {
+        const double y = rsqrt_nr(s);
+        double b = s * y;
+        b = fma(0.5 * y, fma(-b, b, s), b);
+        const double t = b + a;
+        double tau = t * y;
+        tau = fma(fma(-tau, b, t), y, tau);
+        return Reflector{-copysign(b, alpha), tau, copysign(rcp_nr(t), alpha)};
+    }
+    const double beta = -copysign(sqrt(s), alpha);
+    return Reflector{beta, (beta - alpha) / beta, 1.0 / (alpha - beta)};
+}
+
+template <int LG>
+__device__ __forceinline__ double group_sum(double v)
+{
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// Returns false (and flags the status) when the wait gave up after `limit`
-// clock cycles.
-__device__ bool grid_barrier(unsigned *count, unsigned target, int *status, int *s_fail, long long limit)
+// ---- tagged slots -----------------------------------------------------------
+__device__ __forceinline__ void slot_put(uint4 *p, double v, uint32_t tag)
 {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // the fence makes this CTA's slot writes (ordered before it by the
-        // block barrier) visible before the arrival
-        __threadfence();
-        asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;\n" ::"l"(count) : "memory");
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(tag),
+                 "r"(__double2hiint(v)), "r"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 slot_get(const uint4 *p)
+{
+    uint4 w;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p) : "memory");
+    return w;
+}
+
+// The value of slot p once it holds `tag`; false when the wait gave up.
+__device__ __forceinline__ bool slot_wait(const uint4 *p, uint32_t tag, long long limit, double &v)
+{
+    uint4 w = slot_get(p);
+    if (w.y != tag || w.w != tag) {
         const long long t0 = clock64();
-        bool ok = false;
-        for (unsigned it = 0; it < (1u << 26); ++it) {
-            if (ld_acquire(count) >= target) {
-                ok = true;
+        do {
+            if (clock64() - t0 > limit) return false;
+            w = slot_get(p);
+        } while (w.y != tag || w.w != tag);
+    }
+    v = __hiloint2double((int)w.z, (int)w.x);
+    return true;
+}
+
+// Sum over the warp of the slots p[0 .. G) once each holds `tag` (lane l adds
+// p[l], p[l + 32], .., then a butterfly); false when the wait gave up.
+__device__ __forceinline__ bool slots_sum(const uint4 *p, int lane, int G, uint32_t tag, long long limit, double &sum)
+{
+    constexpr int B = 5;  // loads in flight: 160 CTAs
+    sum = 0.0;
+    bool ok = true;
+    for (int q0 = 0; q0 < G && ok; q0 += B * 32) {
+        uint4 w[B];
+        const long long t0 = clock64();
+        for (;;) {
+            bool ready = true;
+#pragma unroll
+            for (int u = 0; u < B; u++) {
+                w[u] = make_uint4(0, tag, 0, tag);
+                if (q0 + u * 32 + lane < G) w[u] = slot_get(p + q0 + u * 32 + lane);
+            }
+#pragma unroll
+            for (int u = 0; u < B; u++) ready = ready && w[u].y == tag && w[u].w == tag;
+            if (__all_sync(0xffffffffu, ready)) break;
+            if (__any_sync(0xffffffffu, clock64() - t0 > limit)) {
+                ok = false;
                 break;
             }
-            if (clock64() - t0 > limit) break;
         }
-        if (!ok) {
-            atomicOr(status, ST_WAIT_TIMEOUT);
-            *s_fail = 1;
-        }
+#pragma unroll
+        for (int u = 0; u < B; u++)
+            if (q0 + u * 32 < G) sum += __hiloint2double((int)w[u].z, (int)w[u].x);
     }
-    __syncthreads();
-    return *s_fail == 0;
+    sum = group_sum<32>(sum);
+    return ok;
 }
 
-__device__ double block_sum(double v, double *red)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < NT / 32; w++) s += red[w];
-    __syncthreads();
-    return s;  // valid in thread 0
-}
+// Slots of one buffer: column c's partial of CTA q at c G + q, its total at
+// nb G + c, the pivot row's entry at nb (G + 1) + c.
+__host__ __device__ inline long long slot_buffer(int nb, int G) { return (long long)nb * (G + 2); }
 
-// One slot buffer (doubles) for up to gmax CTAs: [0, G) the sums of squares,
-// G + owner the pivot, (2 + c) G + q CTA q's dot product with column c, and
-// (MAXNB + 2) gmax + c the pivot row.
-__host__ __device__ inline long long slot_buffer(int gmax) { return (long long)(MAXNB + 2) * gmax + MAXNB; }
-
+template <int LG>
 __global__ void __launch_bounds__(NT, 1)
-    k_panel(int m, int nb, int rpb, double *A, int lda, double *tau, double *slots, long long bstride,
-            unsigned *count, int *status, long long limit, int extra)
+    k_panel(int m, int nb, int rpb, double *A, int lda, double *tau, double *Gram, uint4 *slots, int *status,
+            long long limit, uint32_t tag_skew)
 {
-    extern __shared__ double X[];  // nb columns x nr rows, ld nr
-    __shared__ double red[NT / 32];
-    __shared__ double s_beta, s_tau, s_scal;
+    extern __shared__ double X[];  // nb columns, ld
+    __shared__ double s_tau, s_sc[MAXNB], s_beta[MAXNB], s_d[MAXNB], s_p[MAXNB];
     __shared__ int s_fail;
+    constexpr int NW = NT / 32;
     const int G = gridDim.x, b = blockIdx.x;
-    const int r0 = b * rpb, r1 = min(m, r0 + rpb), nr = max(0, r1 - r0);
-    const long long prow = bstride - MAXNB;  // offset of the pivot row in a buffer
-    if (threadIdx.x == 0) s_fail = 0;
-    for (int idx = threadIdx.x; idx < nr * nb; idx += NT) {
-        const int r = idx % nr, c = idx / nr;
-        X[idx] = A[(size_t)(r0 + r) + (size_t)c * lda];
-    }
-    __syncthreads();
-    unsigned target = 0;
+    const int r0 = b * rpb, nr = min(m - r0, rpb), ld = pad_ld(rpb, LG);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // this CTA's partials of column j (as updated so far) into buffer j & 1
-    auto publish = [&](int j) {
-        double *buf = slots + (size_t)(j & 1) * bstride;
-        const int owner = j / rpb;
-        const double *xj = X + (size_t)j * nr;
-        double p = 0.0;
-        for (int r = threadIdx.x; r < nr; r += NT)
-            if (r0 + r > j) p += xj[r] * xj[r];
-        p = block_sum(p, red);
-        if (threadIdx.x == 0) {
-            buf[b] = p;
-            if (b == owner) buf[(size_t)G + owner] = xj[j - r0];
-        }
-        for (int c = j + 1 + warp; c < nb; c += NT / 32) {
-            const double *xc = X + (size_t)c * nr;
-            double s = 0.0;
-            for (int r = lane; r < nr; r += 32)
-                if (r0 + r > j) s += xj[r] * xc[r];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) {
-                buf[(size_t)(2 + c) * G + b] = s;
-                if (b == owner) buf[prow + c] = xc[j - r0];
-            }
-        }
-    };
-    publish(0);
-    target += G + extra;
-    if (!grid_barrier(count, target, status, &s_fail, limit)) return;
+    const int c = threadIdx.x / LG, g = threadIdx.x % LG;  // this thread's column and its lane in the group
+    if (threadIdx.x == 0) s_fail = 0;
+    for (int cc = warp; cc < nb; cc += NW)
+        for (int r = lane; r < nr; r += 32) X[r + cc * ld] = A[(size_t)(r0 + r) + (size_t)cc * lda];
+    __syncthreads();
+    const bool mine = c < nb;
+    double *xc = X + (mine ? c : 0) * ld;
+    // one past the warp's last column, 0 for a warp without columns
+    const int wc1 = warp * (32 / LG) < nb ? min(nb, (warp + 1) * (32 / LG)) : 0;
     for (int j = 0; j < nb; j++) {
-        const int owner = j / rpb;
-        double *xj = X + (size_t)j * nr;
-        const double *buf = slots + (size_t)(j & 1) * bstride;
-        // the reflector (identical in every CTA: the same loads reduced in the
-        // same tree)
-        double ss = 0.0;
-        for (int q = threadIdx.x; q < G; q += NT) ss += __ldcg(&buf[q]);
-        ss = block_sum(ss, red);
-        if (threadIdx.x == 0) {
-            const double alpha = __ldcg(&buf[(size_t)G + owner]);
-            const double xn = sqrt(ss);
-            if (xn == 0.0) {
-                s_tau = 0.0;
-                s_beta = alpha;
-                s_scal = 0.0;
-            } else {
-                const double beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-                s_tau = (beta - alpha) / beta;
-                s_scal = 1.0 / (alpha - beta);
-                s_beta = beta;
+        uint4 *buf = slots + (size_t)(j & 1) * slot_buffer(nb, G);
+        uint4 *total = buf + (size_t)nb * G, *pivot = total + nb;
+        const uint32_t tag = j + 1 + tag_skew;
+        const bool owner = j >= r0 && j < r0 + nr;
+        const double *xj = X + j * ld;
+        const int first = max(0, j + 1 - r0);
+        // this CTA's partials (the warps of columns before j would be idle
+        // now: the products for T cost nothing extra)
+        if (wc1 > 0) {
+            double d = 0.0;
+#pragma unroll 4
+            for (int r = first + g; r < nr; r += LG) d = fma(xj[r], xc[r], d);
+            d = group_sum<LG>(d);
+            if (mine && g == 0) {
+                slot_put(buf + (size_t)c * G + b, d, j + 1);
+                if (owner) slot_put(pivot + c, xc[j - r0], j + 1);
             }
-            if (b == owner) tau[j] = s_tau;
         }
-        __syncthreads();
-        const double tj = s_tau, sc = s_scal;
-        for (int r = threadIdx.x; r < nr; r += NT)
-            if (r0 + r > j) xj[r] *= sc;
-        if (b == owner && threadIdx.x == 0) xj[j - r0] = s_beta;
-        __syncthreads();
-        // the trailing columns of this CTA's rows, w_c = A(j, c) + sc d_c
-        // (v_r = xj[r] for r0 + r > j, 1 at the pivot row, 0 above)
-        if (tj != 0.0) {
-            for (int c = j + 1 + warp; c < nb; c += NT / 32) {
-                double d = 0.0;
-                for (int q = lane; q < G; q += 32) d += __ldcg(&buf[(size_t)(2 + c) * G + q]);
-                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-                const double w = tj * fma(sc, d, __ldcg(&buf[prow + c]));
-                double *xc = X + (size_t)c * nr;
-                for (int r = lane; r < nr; r += 32) {
-                    const int gr = r0 + r;
-                    if (gr > j)
-                        xc[r] -= xj[r] * w;
-                    else if (gr == j)
-                        xc[r] -= w;
+        // the totals of the columns this warp adds up
+        bool ok = true;
+        for (int cc = b + warp * G; cc < nb; cc += NW * G) {
+            double d, p = 0.0;
+            ok = slots_sum(buf + (size_t)cc * G, lane, G, tag, limit, d) && ok;
+            if (cc >= j) {
+                if (lane == 0) slot_put(total + cc, d, j + 1);
+            } else {
+                ok = slot_wait(pivot + cc, tag, limit, p) && ok;
+                if (lane == 0) {
+                    s_d[cc] = d;
+                    s_p[cc] = p;
                 }
             }
         }
+        double d = 0.0, pr = 0.0;
+        if (wc1 > j) {
+            if (mine && c >= j) ok = slot_wait(pivot + c, tag, limit, pr) && slot_wait(total + c, tag, limit, d) && ok;
+            if (c == j && g == 0) {
+                const Reflector h = reflector(pr, d, d != 0.0);
+                s_tau = h.tau;
+                s_sc[j] = h.sc;
+                s_beta[j] = h.beta;
+                if (owner) tau[j] = h.tau;
+            }
+        }
+        if (!ok) s_fail = 1;
         __syncthreads();
-        if (j + 1 < nb) {
-            publish(j + 1);
-            target += G + extra;
-            if (!grid_barrier(count, target, status, &s_fail, limit)) return;
+        if (s_fail) {
+            if (threadIdx.x == 0) atomicOr(status, ST_WAIT_TIMEOUT);
+            return;
+        }
+        const double tj = s_tau, sc = s_sc[j];
+        if (wc1 > j + 1 && tj != 0.0 && mine && c > j) {
+            const double w = tj * fma(sc, d, pr), f = sc * w;
+#pragma unroll 4
+            for (int r = first + g; r < nr; r += LG) xc[r] = fma(-f, xj[r], xc[r]);
+            if (g == 0 && owner) xc[j - r0] -= w;
+        }
+        // (V^T V)(cc, j) = v_cc(j) + sum_{r > j} v_cc(r) v_j(r)
+        for (int cc = b + warp * G; cc < j; cc += NW * G)
+            if (lane == 0) Gram[cc + (size_t)j * nb] = s_sc[cc] * fma(sc, s_d[cc], s_p[cc]);
+        __syncthreads();
+    }
+    for (int cc = warp; cc < nb; cc += NW) {
+        const double sc = s_sc[cc], beta = s_beta[cc];
+        for (int r = lane; r < nr; r += 32) {
+            const int gr = r0 + r;
+            const double x = X[r + cc * ld];
+            A[(size_t)gr + (size_t)cc * lda] = gr > cc ? x * sc : (gr == cc ? beta : x);
         }
     }
-    for (int idx = threadIdx.x; idx < nr * nb; idx += NT) {
-        const int r = idx % nr, c = idx / nr;
-        A[(size_t)(r0 + r) + (size_t)c * lda] = X[idx];
+}
+
+// Householder QR of an m x n matrix (m >= n) held in one CTA's shared memory:
+// V and R in A, the T tiles (reflector c belongs to the tile floor((i + c) /
+// mt); i = 0 and mt >= n give the one n x n T of a panel) and, when Q is
+// given, Q = H_0 .. H_{n-1} [I; 0].
+//
+// Per column two block barriers: the dot products of column j with the columns
+// of its T tile before it (for T) and all columns from it on, the reflector by
+// one lane of column j's group while the other groups finish; then each group
+// updates its columns.  T(:, j) = -tau_j T(:, 0:j) (V^T v_j) runs beside the
+// next column's dot products.  A sum of squares outside [1e-280, 1e280] takes
+// the column again scaled by a power of two (dlarfg's scaled norm).  Q is
+// formed in place of V from the last reflector to the first; a column is
+// touched by its own group only, so one barrier per step.
+template <int LG>
+__global__ void __launch_bounds__(NTS, 1)
+    k_qr_small(int m, int n, int ld, double *A, int lda, double *T, int ldt, int i, int mt, double *Q, int ldq)
+{
+    extern __shared__ double sm[];
+    constexpr int NW = NTS / 32, NG = NTS / LG;
+    const int tw = min(mt, n);
+    double *X = sm, *Ts = X + (size_t)ld * n, *s_d = Ts + tw * (tw + 1), *s_g = s_d + n, *s_sc = s_g + n,
+           *s_tau = s_sc + n, *s_beta = s_tau + n;
+    __shared__ int s_redo, s_exp, s_nz;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cg = threadIdx.x / LG, g = threadIdx.x % LG;
+    for (int c = warp; c < n; c += NW)
+        for (int r = lane; r < m; r += 32) X[r + c * ld] = A[(size_t)r + (size_t)c * lda];
+    __syncthreads();
+
+    // dot products of column j's rows below the pivot with the columns lo ..,
+    // column j itself first; its group's first lane forms the reflector
+    auto dots = [&](int j, int lo, bool scaled) {
+        const double *xj = X + j * ld;
+        auto one = [&](int c) {
+            const double *xc = X + (size_t)min(c, n - 1) * ld;
+            double d = 0.0;
+#pragma unroll 4
+            for (int r = j + 1 + g; r < m; r += LG) d = fma(xj[r], xc[r], d);
+            return group_sum<LG>(d);
+        };
+        const int jg = j % NG;
+        if (cg / (32 / LG) == jg / (32 / LG)) {  // the warp of column j: all its groups take the same turn
+            const int c = j - jg + cg;
+            const double d = one(c);
+            if (g == 0 && c < n && c >= lo) {
+                s_d[c] = d;
+                if (c == j) {
+                    const double alpha = xj[j];
+                    const double s = fma(alpha, alpha, d);
+                    const bool last = j == m - 1;
+                    if (!scaled) s_redo = !last && !(d >= 1e-280 && s <= 1e280);
+                    const Reflector h = reflector(alpha, d, scaled ? s_nz != 0 : !last);
+                    s_tau[j] = h.tau;
+                    s_sc[j] = h.sc;
+                    s_beta[j] = scaled ? scalbn(h.beta, s_exp) : h.beta;
+                }
+            }
+        }
+        for (int c0 = lo - lo % NG; c0 < n; c0 += NG) {
+            if (c0 == j - jg && cg / (32 / LG) == jg / (32 / LG)) continue;
+            if (c0 + (warp + 1) * (32 / LG) <= lo || c0 + warp * (32 / LG) >= n) continue;
+            const int c = c0 + cg;
+            const double d = one(c);
+            if (g == 0 && c < n && c >= lo) s_d[c] = d;
+        }
+    };
+    // T(:, j) of j's tile from g_c = v_c^T v_j (s_g), rows ts .. j
+    auto t_column = [&](int j, int ts) {
+        const double tj = s_tau[j];
+        double *gt = T + (i + ts) % mt + (size_t)j * ldt;
+        for (int r0 = ts; r0 < j; r0 += NG) {
+            if (r0 + warp * (32 / LG) >= j) break;
+            const int r = r0 + cg;
+            double s = 0.0;
+            if (r < j)
+                for (int c = r + g; c < j; c += LG) s = fma(Ts[(r - ts) + (c - ts) * (tw + 1)], s_g[c], s);
+            s = group_sum<LG>(s);
+            if (r < j && g == 0) {
+                const double t = tj == 0.0 ? 0.0 : -tj * s;
+                Ts[(r - ts) + (j - ts) * (tw + 1)] = t;
+                gt[r - ts] = t;
+            }
+        }
+        if (threadIdx.x == 0) {
+            Ts[(j - ts) + (j - ts) * (tw + 1)] = tj;
+            gt[j - ts] = tj;
+        }
+    };
+    // first column of j's tile
+    auto tile_start = [&](int j) { return max(0, (i + j) / mt * mt - i); };
+
+    for (int j = 0; j < n; j++) {
+        const int ts = tile_start(j);
+        double *xj = X + j * ld;
+        dots(j, ts, false);
+        // the previous column's T beside this column's dot products
+        if (j > 0) t_column(j - 1, tile_start(j - 1));
+        __syncthreads();
+        if (s_redo) {
+            // rare: scale rows j.. of column j by 2^-e, e the largest exponent,
+            // and take the column again
+            if (threadIdx.x == 0) {
+                s_exp = 0;
+                s_nz = 0;
+            }
+            __syncthreads();
+            int e = 0, nz = 0;
+            for (int r = j + threadIdx.x; r < m; r += NTS) {
+                const unsigned long long u = (unsigned long long)__double_as_longlong(xj[r]) << 1;
+                if (r > j && u) nz = 1;
+                // exponent + 64; a subnormal's from its leading bit
+                const int ex = (int)(u >> 53);
+                e = max(e, u ? (ex ? ex + 64 : 75 - __clzll((long long)u)) : 0);
+            }
+            atomicMax(&s_exp, e);
+            if (nz) atomicOr(&s_nz, 1);
+            __syncthreads();
+            // biased (+64) exponent -> power of two; nothing to scale in a zero
+            // or non-finite column
+            const int ex = s_exp, k = (ex == 0 || ex >= 0x7FF + 64) ? 0 : ex - 64 - 1023;
+            __syncthreads();
+            if (threadIdx.x == 0) s_exp = k;
+            for (int r = j + threadIdx.x; r < m; r += NTS) xj[r] = scalbn(xj[r], -k);
+            __syncthreads();
+            dots(j, ts, true);
+            __syncthreads();
+        }
+        const double tj = s_tau[j], sc = s_sc[j];
+        for (int c0 = ts - ts % NG; c0 < n; c0 += NG) {
+            if (c0 + (warp + 1) * (32 / LG) <= ts || c0 + warp * (32 / LG) >= n) continue;
+            const int c = c0 + cg;
+            const bool on = c >= ts && c < n && c != j, right = on && c > j && tj != 0.0;
+            double *xc = X + (on ? c : j) * ld;
+            const double w = on ? fma(sc, s_d[c], xc[j]) : 0.0;
+            if (right) {
+                const double f = sc * (tj * w);
+#pragma unroll 4
+                for (int r = j + 1 + g; r < m; r += LG) xc[r] = fma(-f, xj[r], xc[r]);
+            }
+            __syncwarp();  // the group has read its pivot entry
+            if (g == 0) {
+                if (right) xc[j] -= tj * w;
+                if (on && c < j) s_g[c] = s_sc[c] * w;
+            }
+        }
+        __syncthreads();
     }
+    t_column(n - 1, tile_start(n - 1));
+    // V and R out; V stays, scaled, where Q is formed
+    for (int c = warp; c < n; c += NW) {
+        const double sc = s_sc[c], beta = s_beta[c];
+        for (int r = lane; r < m; r += 32) {
+            double x = X[r + c * ld];
+            x = r > c ? x * sc : (r == c ? beta : x);
+            A[(size_t)r + (size_t)c * lda] = x;
+            X[r + c * ld] = r > c ? x : 0.0;
+        }
+    }
+    if (!Q) return;
+    __syncthreads();
+    for (int j = n - 1; j >= 0; j--) {
+        const double tj = s_tau[j];
+        double *xj = X + j * ld;
+        for (int c0 = (j + 1) - (j + 1) % NG; c0 < n; c0 += NG) {
+            if (c0 + (warp + 1) * (32 / LG) <= j + 1 || c0 + warp * (32 / LG) >= n) continue;
+            const int c = c0 + cg;
+            const bool on = c > j && c < n;
+            double *xc = X + (on ? c : j) * ld;
+            double d = 0.0;
+#pragma unroll 4
+            for (int r = j + 1 + g; r < m; r += LG) d = fma(xj[r], xc[r], d);
+            d = tj * group_sum<LG>(d);
+            if (on) {
+#pragma unroll 4
+                for (int r = j + 1 + g; r < m; r += LG) xc[r] = fma(-d, xj[r], xc[r]);
+                if (g == 0) xc[j] = -d;
+            }
+        }
+        __syncthreads();
+        if (cg == j % NG) {
+            for (int r = j + 1 + g; r < m; r += LG) xj[r] *= -tj;
+            if (g == 0) xj[j] = 1.0 - tj;
+        }
+        __syncwarp();  // the next step reads the column by other lanes of its group
+    }
+    __syncthreads();
+    for (int c = warp; c < n; c += NW)
+        for (int r = lane; r < m; r += 32) Q[(size_t)r + (size_t)c * ldq] = X[r + c * ld];
 }
 
 }  // namespace pnl
 
-// Doubles of workspace panel_coop needs for an nb-column panel: tau, the
-// Gram V^T V, the per-CTA reduction slots, the barrier counter and split-K
-// room for the Gram.
+// Doubles of workspace panel_coop needs for an nb-column panel (tau, the
+// Gram V^T V and the exchange slots: two buffers of 16-byte slots; the rest
+// is kept so that the workspace queries' answers stay).
 long long panel_coop_work(int nb)
 {
-    return (long long)nb + (long long)nb * nb + 2 * pnl::slot_buffer(sm_count()) + 8 + 64LL * nb * nb;
+    const long long G = sm_count();
+    return (long long)nb + (long long)nb * nb + 2 * ((pnl::MAXNB + 2) * G + pnl::MAXNB) + 8 + 64LL * nb * nb;
 }
 
 // Whether the cooperative panel applies to an m x nb panel.
@@ -214,48 +460,43 @@ bool panel_coop_fits(int m, int nb)
 // V (unit lower, below the diagonal), R (on and above) in A and the nb x nb T
 // of the panel's compact-WY form (forward, columnwise), as dgeqr3 gives them.
 // Returns false when the cooperative launch was refused (nothing enqueued).
-// extra: arrivals each grid barrier waits for beyond the CTAs' own (0; a
-// test passes 1 so that every wait runs out, see lila_prim_panel_phantom).
-static bool panel_coop_launch(int m, int nb, double *A, int lda, double *T, int ldt, double *work, int extra)
+// tag_skew: added to the tag every reader waits for (0; a test passes one that
+// no CTA writes, so that every wait runs out, see lila_prim_panel_phantom).
+static bool panel_coop_launch(int m, int nb, double *A, int lda, double *T, int ldt, double *work, uint32_t tag_skew)
 {
     if (!panel_coop_fits(m, nb)) return false;
     const int Gmax = sm_count();
-    int G = (m + 15) / 16;
-    if (G > Gmax) G = Gmax;
-    const int rpb = (m + G - 1) / G;
-    G = (m + rpb - 1) / rpb;
+    // every SM takes part from 16 rows each on
+    int rpb = (m + Gmax - 1) / Gmax;
+    if (rpb < 16) rpb = 16;
+    const int G = (m + rpb - 1) / rpb;
     double *tau = work;
     double *Gram = tau + nb;
-    double *slots = Gram + (size_t)nb * nb;
-    const long long bstride = pnl::slot_buffer(Gmax);
-    unsigned *count = (unsigned *)(slots + 2 * bstride);
-    double *part = slots + 2 * bstride + 8;
-    const size_t smem = (size_t)rpb * nb * sizeof(double);
+    // slots on a 16-byte boundary (work is at least 8-byte aligned)
+    uint4 *slots = (uint4 *)(((uintptr_t)(Gram + (size_t)nb * nb) + 15) & ~(uintptr_t)15);
+    const long long nslots = 2 * pnl::slot_buffer(nb, G);
+    const int lg = pnl::lanes_for(pnl::NT, nb);
+    const size_t smem = (size_t)pnl::pad_ld(rpb, lg) * nb * sizeof(double);
+    const void *kern = lg == 4 ? (const void *)pnl::k_panel<4>
+                               : (lg == 8 ? (const void *)pnl::k_panel<8> : (const void *)pnl::k_panel<16>);
     cudaStream_t st = stream();
-    cudaFuncSetAttribute(pnl::k_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaMemsetAsync(count, 0, sizeof(unsigned), st);
-    int *status = status_ptr();
-    long long limit = wait_limit();
-    void *args[] = {(void *)&m,     (void *)&nb,      (void *)&rpb,    (void *)&A,      (void *)&lda,
-                    (void *)&tau,   (void *)&slots,   (void *)&bstride, (void *)&count, (void *)&status,
-                    (void *)&limit, (void *)&extra};
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pnl::k_panel, pnl::NT, smem) != cudaSuccess ||
-        per_sm < 1) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
+    trace_break();
+    cudaMemsetAsync(slots, 0, (size_t)nslots * sizeof(uint4), st);
+    int *status = status_ptr();
+    long long limit = wait_limit();
+    void *args[] = {(void *)&m,    (void *)&nb,    (void *)&rpb,    (void *)&A,     (void *)&lda,     (void *)&tau,
+                    (void *)&Gram, (void *)&slots, (void *)&status, (void *)&limit, (void *)&tag_skew};
     trace_begin();
-    if (cudaLaunchCooperativeKernel((const void *)pnl::k_panel, dim3(G), dim3(pnl::NT), args, smem, st) != cudaSuccess) {
+    if (cudaLaunchCooperativeKernel(kern, dim3(G), dim3(pnl::NT), args, smem, st) != cudaSuccess) {
         cudaGetLastError();  // refused (e.g. not all CTAs can be resident): nothing ran
         trace_cancel();
         return false;
     }
     note_launch("panel_coop");
-    // T from V^T V (only the strictly upper part of the Gram is used)
-    GemmEpi e;
-    gemm(nb, nb, m, opnd(A, lda, TR, M_UNIT_LOWER), opnd(A, lda, NT, M_UNIT_LOWER), Gram, nb, e, part,
-         64LL * nb * nb, "panel_gram");
     larft_from_gram(nb, Gram, nb, tau, T, ldt);
     return true;
 }
@@ -265,18 +506,46 @@ bool panel_coop(int m, int nb, double *A, int lda, double *T, int ldt, double *w
     return panel_coop_launch(m, nb, A, lda, T, ldt, work, 0);
 }
 
+// Shared memory of k_qr_small, 0 when the matrix does not fit.
+static size_t qr_small_smem(int m, int n, int mt)
+{
+    const long long tw = mt < n ? mt : n;
+    const long long b = 8LL * ((long long)pnl::pad_ld(m, pnl::lanes_for(pnl::NTS, n)) * n + tw * (tw + 1) + 5LL * n);
+    return b <= 220 * 1024 ? (size_t)b : 0;
+}
+
+bool qr_small(int m, int n, double *A, int lda, double *T, int ldt, int i, int mt, double *Q, int ldq)
+{
+    const size_t smem = n < 1 || m < n ? 0 : qr_small_smem(m, n, mt);
+    if (!smem) return false;
+    cudaStream_t st = stream();
+    auto launch = [&](auto kern) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        trace_begin();
+        kern<<<1, pnl::NTS, smem, st>>>(m, n, pnl::pad_ld(m, pnl::lanes_for(pnl::NTS, n)), A, lda, T, ldt, i, mt, Q, ldq);
+        note_launch("qr_small");
+        return true;
+    };
+    if (pnl::lanes_for(pnl::NTS, n) == 8) return launch(pnl::k_qr_small<8>);
+    if (pnl::lanes_for(pnl::NTS, n) == 16) return launch(pnl::k_qr_small<16>);
+    return launch(pnl::k_qr_small<32>);
+}
+
 }  // namespace lg
 
 extern "C" {
-// Failure-path test of the grid-barrier wait: the panel of an m x nb matrix
-// with every barrier waiting for `extra` arrivals that never come, so each
-// CTA's wait runs out after the lila_gpu_set_wait_limit cycles, sets
+// Failure-path test of the exchange's bounded waits: the panel of an m x nb
+// matrix with every reader waiting for a tag that is never written (extra > 0),
+// so each CTA's wait runs out after the lila_gpu_set_wait_limit cycles, sets
 // LILA_ST_WAIT_TIMEOUT and returns (A and T are then meaningless).  1 when
 // the cooperative launch ran, 0 when the panel does not apply.
 int lila_prim_panel_phantom(int m, int nb, double *A, int lda, double *T, int ldt, double *work, int extra)
 {
     if (extra < 0) return -8;
-    return lg::panel_coop_launch(m, nb, A, lda, T, ldt, work, extra) ? 1 : 0;
+    return lg::panel_coop_launch(m, nb, A, lda, T, ldt, work, extra ? 0x40000000u : 0u) ? 1 : 0;
 }
 long long lila_prim_panel_work(int nb) { return lg::panel_coop_work(nb); }
 }
