@@ -1,6 +1,7 @@
 // lg_batched.cu -- thousands of independent least-squares problems
 // min ||A_t x - b_t|| (A_t m_t x n_t, m_t >= n_t, nrhs right-hand sides) in
-// one persistent launch.
+// one persistent launch (and one of clusters beside it when a few large
+// instances would outlast the rest).
 //
 // Per instance the algorithm is the reference's least-squares driver
 // (least-squares/main_ls_qr3.c:94-119): Householder QR of A, Q^T applied to
@@ -15,302 +16,571 @@
 #include <algorithm>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "lg_common.cuh"
 #include "../../include/lila_gpu.h"
 
 namespace lg {
 namespace bat {
 
+namespace cg = cooperative_groups;
+
 struct Inst {
     int m, n, lda, ldb;
 };
 
-constexpr int CW = 8;  // columns updated per pass
+constexpr int NB = 8;    // panel width
+constexpr int UW = 4;    // trailing columns of one warp's pass
+constexpr int TIERS = 3; // launches by team: clusters of 8 and of 4 CTAs, single CTAs
+__host__ __device__ constexpr int tier_ctas(int tier) { return tier == 0 ? 8 : (tier == 1 ? 4 : 1); }
+constexpr int MAXG = 34; // column groups exchanged at a time in a cluster (n + nrhs <= 136 in one go)
 
-template <int TH>
-__device__ double bsum(double v, double *red)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = l < TH / 32 ? red[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (l == 0) red[32] = v;
-    }
-    __syncthreads();
-    return red[32];
-}
+// Blocked Householder least squares of one instance by a CTA (CS = 1) or by a
+// cluster of CS CTAs, each on its own block of rows.
+//
+// Bound: the FP64 pipe (2 lanes per clock per SM, 64 clocks of a sub-partition
+// per warp instruction whatever its lanes carry).  So no FP64 instruction is
+// spent on what is not a product of the algorithm where that can be avoided:
+//  * a panel of NB columns takes one pass over its rows per column: the pass
+//    scales v, updates the panel's later columns and accumulates the next
+//    column's products with all panel columns (those before it give T), the
+//    eight sums reduced by a transposing butterfly (9 additions per warp, not
+//    40); plain sums of squares (no maximum, no division per element), a
+//    column whose squares leave the FP64 range is taken again scaled by a
+//    power of two;
+//  * a warp owns UW trailing columns: W = V^T C over all rows needs no other
+//    warp, its 32 sums land one per lane (31 additions, not 160), W := T^T W
+//    by shuffles, C -= V W, without a block barrier;
+//  * the back substitution runs one warp per right-hand side from registers
+//    with the reciprocals of R's diagonal formed beforehand.
+// 5,000 uneven instances (m 64..4096, n 8..128): 195 -> 140 ms (920 GFLOP/s,
+// 73 % of the DFMA peak); 400 took 47 ms in the previous form (one column's
+// dot products per pass over the block, five shuffle additions per accumulator
+// in every warp, scaled norms by division, one CTA per instance).
+//
+// In a cluster each CTA publishes its partial sums in every CTA's shared
+// memory (distributed shared memory) and one cluster barrier later all add
+// them in CTA order; the trailing W of column group q is added up and
+// multiplied by T^T in CTA q mod CS.  Slots alternate with the column so that
+// one barrier per column is enough.
+template <int TH, int CS>
+struct Shared {
+    static constexpr int NW = TH / 32;
+    double red[NW][NB];          // per warp sums of a column's products
+    double x[2][CS][NB];         // per CTA sums, written by every CTA of the cluster
+    double piv[2][NB], own[NB];  // the pivot row's panel entries; as its owner has them
+    double w[NB], f[NB], g[NB];  // update factors of the panel columns, V^T v
+    double T[NB][NB], tau[NB];
+    double sc, beta;
+    double wb[NW][NB * UW];
+    double part[CS > 1 ? MAXG : 1][NB * UW], wt[CS > 1 ? MAXG : 1][NB * UW];
+    int emax[CS], nz[CS];
+    int exp2, below, redo, idx;
+};
 
-template <int TH>
-__device__ double bmax(double v, double *red)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = l < TH / 32 ? red[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (l == 0) red[32] = v;
-    }
-    __syncthreads();
-    return red[32];
-}
-
-// column c of the combined [A | B] operand of an instance
 __device__ __forceinline__ double *colp(double *A, int lda, double *B, int ldb, int n, int c)
 {
     return c < n ? A + (size_t)c * lda : B + (size_t)(c - n) * ldb;
 }
 
-constexpr int NB = 8;   // panel width of the blocked factorization
-constexpr int UW = 4;   // trailing columns per block-reflector pass
-
-// Blocked Householder least squares per instance: panels of NB columns are
-// factored column by column (each reflector applied to the rest of its
-// panel), then the panel's block reflector I - V T V^T (T by the dlarft
-// recurrence from V^T V) is applied to the trailing columns of A and to B,
-// UW columns per pass: W = V^T C, W = T^T W, C -= V W.  The trailing matrix
-// is read and written once per panel instead of once per column.
-template <int TH>
-__global__ void __launch_bounds__(TH)
-    k_gels(int count, int nrhs, const Inst *inst, double *const *Aptr, double *const *Bptr, const int *order,
-           int *counter, int *info)
+template <int CS>
+__device__ __forceinline__ void team_sync()
 {
-    __shared__ double red[33 * CW];
-    __shared__ double s_w[CW];
-    __shared__ double s_tau, s_scale, s_beta;
-    __shared__ double s_taus[NB], s_G[NB * NB], s_T[NB * NB], s_W[NB * UW];
-    __shared__ double s_red[TH / 32][NB * (NB - 1) / 2 > NB * UW ? NB * (NB - 1) / 2 : NB * UW];
-    __shared__ int s_idx;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (;;) {
-        if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1);
+    if (CS > 1)
+        cg::this_cluster().sync();
+    else
         __syncthreads();
-        const int idx = s_idx;
-        __syncthreads();
-        if (idx >= count) break;
-        const int t = order[idx];
-        const Inst I = inst[t];
-        double *A = Aptr[t], *B = Bptr[t];
-        const int m = I.m, n = I.n;
-        const int ncol = n + nrhs;
-        int bad = 0;
-        for (int j0 = 0; j0 < n; j0 += NB) {
-            const int jb = min(NB, n - j0);
-            // ---- panel: reflectors j0 .. j0 + jb - 1 on the panel's own columns
-            for (int k = j0; k < j0 + jb; k++) {
-                double *ck = A + (size_t)k * I.lda;
-                // Householder vector of A(k:m, k) (LAPACK dlarfg convention)
-                double mx = 0.0;
-                for (int r = k + 1 + threadIdx.x; r < m; r += TH) mx = fmax(mx, fabs(ck[r]));
-                const double scale = bmax<TH>(mx, red);
-                double part = 0.0;
-                if (scale > 0.0)
-                    for (int r = k + 1 + threadIdx.x; r < m; r += TH) {
-                        const double q = ck[r] / scale;
-                        part += q * q;
-                    }
-                const double ssq = bsum<TH>(part, red);
-                if (threadIdx.x == 0) {
-                    const double alpha = ck[k];
-                    if (scale == 0.0) {
-                        s_tau = 0.0;
-                        s_beta = alpha;
-                    } else {
-                        const double beta = -copysign(hypot(alpha, scale * sqrt(ssq)), alpha);
-                        s_tau = (beta - alpha) / beta;
-                        s_scale = 1.0 / (alpha - beta);
-                        s_beta = beta;
-                    }
-                    s_taus[k - j0] = s_tau;
-                }
-                __syncthreads();
-                const double tk = s_tau;
-                if (tk != 0.0)
-                    for (int r = k + 1 + threadIdx.x; r < m; r += TH) ck[r] *= s_scale;
-                __syncthreads();
-                if (threadIdx.x == 0) ck[k] = s_beta;
-                const int pend = j0 + jb;  // panel columns k + 1 .. pend - 1
-                if (tk == 0.0 || k + 1 >= pend) {
-                    __syncthreads();
-                    continue;
-                }
-                const int nc = pend - (k + 1);  // <= NB - 1 <= CW
-                double acc[CW];
+}
+
+// `p` of this CTA's shared memory in CTA `rank` of the cluster.
+template <int CS, typename V>
+__device__ __forceinline__ V *remote(V *p, int rank)
+{
+    return CS > 1 ? cg::this_cluster().map_shared_rank(p, rank) : p;
+}
+
+// Eight sums over the warp: lane l returns sum number l / 4.
+__device__ __forceinline__ double reduce8(double (&a)[NB], int lane)
+{
 #pragma unroll
-                for (int j = 0; j < CW; j++) acc[j] = 0.0;
-                for (int r = k + 1 + threadIdx.x; r < m; r += TH) {
-                    const double v = ck[r];
+    for (int h = NB / 2, o = 16; h > 0; h /= 2, o /= 2)
 #pragma unroll
-                    for (int j = 0; j < CW; j++)
-                        if (j < nc) acc[j] += v * A[(size_t)r + (size_t)(k + 1 + j) * I.lda];
-                }
+        for (int i = 0; i < h; i++) {
+            const double send = (lane & o) ? a[i] : a[i + h], keep = (lane & o) ? a[i + h] : a[i];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    double v = a[0];
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v;
+}
+
+// 32 sums over the warp: lane l returns sum number l.
+__device__ __forceinline__ double reduce32(double (&a)[NB * UW], int lane)
+{
 #pragma unroll
-                for (int j = 0; j < CW; j++)
-                    for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-                if (lane == 0)
+    for (int h = 16; h > 0; h /= 2)
 #pragma unroll
-                    for (int j = 0; j < CW; j++) red[j * 33 + warp] = acc[j];
-                __syncthreads();
-                if (threadIdx.x < nc) {
-                    double sw = 0.0;
-                    for (int q = 0; q < TH / 32; q++) sw += red[threadIdx.x * 33 + q];
-                    sw += A[(size_t)k + (size_t)(k + 1 + threadIdx.x) * I.lda];  // v_k = 1
-                    s_w[threadIdx.x] = tk * sw;
-                }
-                __syncthreads();
-                for (int r = k + threadIdx.x; r < m; r += TH) {
-                    const double v = r == k ? 1.0 : ck[r];
+        for (int i = 0; i < h; i++) {
+            const double send = (lane & h) ? a[i] : a[i + h], keep = (lane & h) ? a[i + h] : a[i];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    return a[0];
+}
+
+template <int TH, int CS>
+struct Solver {
+    using S = Shared<TH, CS>;
+    static constexpr int NW = TH / 32;
+    S &s;
+    double *A, *B;
+    int m, n, lda, ldb, nrhs;
+    int rank, lo, hi;  // this CTA's rows [lo, hi)
+    int tid, warp, lane;
+
+    __device__ Solver(S &sh) : s(sh) {}
+
+    // a pivot-row entry; in a cluster the owner's warp 0 passes it on (reflect)
+    __device__ __forceinline__ void put_pivot(int par, int c, double v)
+    {
+        if (CS > 1)
+            s.own[c] = v;
+        else
+            s.piv[par][c] = v;
+    }
+
+    // products of column kk of the panel at j0 (rows below its pivot) with the
+    // panel's columns; the pivot row into slot par
+    __device__ void dots(int j0, int jb, int kk, int par, double (&acc)[NB])
+    {
+        const int k = j0 + kk;
+        const double *P = A + (size_t)j0 * lda, *xk = A + (size_t)k * lda;
 #pragma unroll
-                    for (int j = 0; j < CW; j++)
-                        if (j < nc) A[(size_t)r + (size_t)(k + 1 + j) * I.lda] -= s_w[j] * v;
-                }
-                __syncthreads();
+        for (int c = 0; c < NB; c++) acc[c] = 0.0;
+        for (int r = lo + (max(k - lo, 0)) / TH * TH + tid; r < hi; r += TH) {
+            if (r < k) continue;
+            if (r == k) {
+#pragma unroll
+                for (int c = 0; c < NB; c++)
+                    if (c < jb) put_pivot(par, c, P[(size_t)r + (size_t)c * lda]);
+                continue;
             }
-            if (j0 + jb >= ncol) continue;
-            // ---- T of the panel from G = V^T V (strictly upper part)
-            // v_i(r) = A(r, j0 + i) below the diagonal, 1 on it, 0 above
-            {
-                double g[NB * (NB - 1) / 2];
+            const double y = xk[r];
 #pragma unroll
-                for (int q = 0; q < NB * (NB - 1) / 2; q++) g[q] = 0.0;
-                for (int r = j0 + 1 + threadIdx.x; r < m; r += TH) {
-                    double v[NB];
+            for (int c = 0; c < NB; c++)
+                if (c < jb) acc[c] = fma(y, P[(size_t)r + (size_t)c * lda], acc[c]);
+        }
+    }
+
+    // the pass of column KK: v, the update of the panel's later columns and
+    // the products of column KK + 1
+    template <int KK>
+    __device__ void pass(int j0, int jb, int par, double (&acc)[NB])
+    {
+        const int k = j0 + KK;
+        double *P = A + (size_t)j0 * lda;
+        const double sc = s.sc, beta = s.beta;
+        double f[NB];
 #pragma unroll
-                    for (int i = 0; i < NB; i++) {
-                        const int d = j0 + i;
-                        v[i] = (i < jb) ? (r > d ? A[(size_t)r + (size_t)d * I.lda] : (r == d ? 1.0 : 0.0)) : 0.0;
-                    }
-                    int q = 0;
+        for (int c = KK + 1; c < NB; c++) f[c] = s.f[c];
+        const bool next = KK + 1 < jb;
 #pragma unroll
-                    for (int a2 = 0; a2 < NB; a2++)
+        for (int c = 0; c < NB; c++) acc[c] = 0.0;
+        for (int r = lo + (max(k - lo, 0)) / TH * TH + tid; r < hi; r += TH) {
+            if (r < k) continue;
+            double *row = P + r;
+            if (r == k) {
+                row[(size_t)KK * lda] = beta;
 #pragma unroll
-                        for (int b2 = a2 + 1; b2 < NB; b2++) g[q++] += v[a2] * v[b2];
-                }
-#pragma unroll
-                for (int q = 0; q < NB * (NB - 1) / 2; q++) {
-                    double x = g[q];
-                    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                    if (lane == 0) s_red[warp][q] = x;
-                }
-                __syncthreads();
-                if (threadIdx.x < NB * (NB - 1) / 2) {
-                    double x = 0.0;
-                    for (int w = 0; w < TH / 32; w++) x += s_red[w][threadIdx.x];
-                    // pair index -> (a2, b2)
-                    int q = threadIdx.x, a2 = 0;
-                    while (q >= NB - 1 - a2) {
-                        q -= NB - 1 - a2;
-                        a2++;
-                    }
-                    s_G[a2 + NB * (a2 + 1 + q)] = x;
-                }
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    for (int i = 0; i < jb; i++) {
-                        const double ti = s_taus[i];
-                        for (int r = 0; r < i; r++) {
-                            double x = 0.0;
-                            for (int p2 = r; p2 < i; p2++) x += s_T[r + NB * p2] * s_G[p2 + NB * i];
-                            s_T[r + NB * i] = -ti * x;
-                        }
-                        s_T[i + NB * i] = ti;
-                    }
-                }
-                __syncthreads();
+                for (int c = KK + 1; c < NB; c++)
+                    if (c < jb) row[(size_t)c * lda] -= s.w[c];
+                continue;
             }
-            // ---- block reflector on the trailing columns of A and on B
-            for (int c0 = j0 + jb; c0 < ncol; c0 += UW) {
-                const int nc = min(UW, ncol - c0);
-                double w[NB][UW];
+            double a[NB];
 #pragma unroll
-                for (int i = 0; i < NB; i++)
+            for (int c = 0; c < NB; c++) a[c] = (c < jb && (next || c == KK)) ? row[(size_t)c * lda] : 0.0;
+            const double x = a[KK];
+            a[KK] = x * sc;
+            row[(size_t)KK * lda] = a[KK];
+            if (!next) continue;
 #pragma unroll
-                    for (int j = 0; j < UW; j++) w[i][j] = 0.0;
-                for (int r = j0 + threadIdx.x; r < m; r += TH) {
-                    double v[NB];
-#pragma unroll
-                    for (int i = 0; i < NB; i++) {
-                        const int d = j0 + i;
-                        v[i] = (i < jb) ? (r > d ? A[(size_t)r + (size_t)d * I.lda] : (r == d ? 1.0 : 0.0)) : 0.0;
-                    }
-#pragma unroll
-                    for (int j = 0; j < UW; j++)
-                        if (j < nc) {
-                            const double cv = colp(A, I.lda, B, I.ldb, n, c0 + j)[r];
-#pragma unroll
-                            for (int i = 0; i < NB; i++) w[i][j] += v[i] * cv;
-                        }
+            for (int c = KK + 1; c < NB; c++)
+                if (c < jb) {
+                    a[c] = fma(-f[c], x, a[c]);
+                    row[(size_t)c * lda] = a[c];
                 }
+            constexpr int K1 = KK + 1 < NB ? KK + 1 : KK;
+            if (r == k + 1) {
 #pragma unroll
-                for (int i = 0; i < NB; i++)
+                for (int c = 0; c < NB; c++)
+                    if (c < jb) put_pivot(par, c, a[c]);
+            } else {
+                const double y = a[K1];
 #pragma unroll
-                    for (int j = 0; j < UW; j++) {
-                        double x = w[i][j];
-                        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                        if (lane == 0) s_red[warp][i * UW + j] = x;
-                    }
-                __syncthreads();
-                if (threadIdx.x < NB * UW) {
-                    double x = 0.0;
-                    for (int q = 0; q < TH / 32; q++) x += s_red[q][threadIdx.x];
-                    red[threadIdx.x] = x;  // W(i, j), i = idx / UW
-                }
-                __syncthreads();
-                if (threadIdx.x < NB * UW) {  // W := T^T W
-                    const int i = threadIdx.x / UW, j = threadIdx.x % UW;
-                    double x = 0.0;
-                    for (int p2 = 0; p2 <= i && p2 < jb; p2++) x += s_T[p2 + NB * i] * red[p2 * UW + j];
-                    s_W[i * UW + j] = (i < jb) ? x : 0.0;
-                }
-                __syncthreads();
-                for (int r = j0 + threadIdx.x; r < m; r += TH) {
-                    double v[NB];
-#pragma unroll
-                    for (int i = 0; i < NB; i++) {
-                        const int d = j0 + i;
-                        v[i] = (i < jb) ? (r > d ? A[(size_t)r + (size_t)d * I.lda] : (r == d ? 1.0 : 0.0)) : 0.0;
-                    }
-#pragma unroll
-                    for (int j = 0; j < UW; j++)
-                        if (j < nc) {
-                            double x = 0.0;
-#pragma unroll
-                            for (int i = 0; i < NB; i++) x += v[i] * s_W[i * UW + j];
-                            colp(A, I.lda, B, I.ldb, n, c0 + j)[r] -= x;
-                        }
-                }
-                __syncthreads();
+                for (int c = 0; c < NB; c++)
+                    if (c < jb) acc[c] = fma(y, a[c], acc[c]);
             }
         }
-        // back substitution R x = y, x over B(0:n, :)
-        for (int k = n - 1; k >= 0; k--) {
-            const double d = A[(size_t)k + (size_t)k * I.lda];
-            if (threadIdx.x < nrhs) {
-                double *bk = B + (size_t)threadIdx.x * I.ldb;
-                if (d == 0.0 || !isfinite(d)) {
-                    bad = k + 1;
-                    bk[k] = NAN;
+    }
+
+    // sums of acc over the team, then the reflector of column kk (by warp 0);
+    // on return (block barrier passed) s.sc, s.beta, s.w, s.f, s.tau[kk], T's
+    // column kk and s.redo are set
+    __device__ void reflect(int j0, int jb, int kk, int par, double (&acc)[NB], bool scaled)
+    {
+        // a warp without rows spends no additions
+        const double mine = lo + 32 * warp < hi ? reduce8(acc, lane) : 0.0;
+        if ((lane & 3) == 0) s.red[warp][lane >> 2] = mine;
+        __syncthreads();
+        const int c = lane >> 2, q = lane & 3;
+        double d = 0.0;
+        if (warp == 0) {
+            for (int u = q; u < NW; u += 4) d += s.red[u][c];
+            d += __shfl_xor_sync(0xffffffffu, d, 1);
+            d += __shfl_xor_sync(0xffffffffu, d, 2);
+        }
+        if (CS > 1) {
+            if (warp == 0) {
+                const bool owner = j0 + kk >= lo && j0 + kk < hi;
+                for (int u = q; u < CS; u += 4) {
+                    *remote<CS>(&s.x[par][rank][c], u) = d;
+                    if (owner) *remote<CS>(&s.piv[par][c], u) = s.own[c];
+                }
+            }
+            team_sync<CS>();
+            if (warp == 0) {
+                d = 0.0;
+                for (int u = q; u < CS; u += 4) d += s.x[par][u][c];
+                d += __shfl_xor_sync(0xffffffffu, d, 1);
+                d += __shfl_xor_sync(0xffffffffu, d, 2);
+            }
+        }
+        if (warp == 0) {
+            const double p = s.piv[par][c];
+            const double alpha = __shfl_sync(0xffffffffu, p, 4 * kk), ss = __shfl_sync(0xffffffffu, d, 4 * kk);
+            const int k = j0 + kk;
+            const bool last = k == m - 1;
+            const double sq = fma(alpha, alpha, ss);
+            const bool redo = !scaled && !last && !(ss >= 1e-280 && sq <= 1e280);
+            const bool below = scaled ? s.below != 0 : !last;
+            double beta = alpha, tau = 0.0, sc = 0.0;
+            if (below) {
+                if (sq >= 1e-290 && sq <= 1e290) {
+                    // |beta| = sqrt(sq) corrected to rounding level, tau = 1 +
+                    // |alpha| / |beta|, sc = 1 / (alpha - beta)
+                    const double y = rsqrt_nr(sq);
+                    double nb = sq * y;
+                    nb = fma(0.5 * y, fma(-nb, nb, sq), nb);
+                    const double t = nb + fabs(alpha);
+                    tau = t * y;
+                    tau = fma(fma(-tau, nb, t), y, tau);
+                    beta = -copysign(nb, alpha);
+                    sc = copysign(rcp_nr(t), alpha);
                 } else {
-                    bk[k] /= d;
+                    beta = -copysign(sqrt(sq), alpha);
+                    tau = (beta - alpha) / beta;
+                    sc = 1.0 / (alpha - beta);
                 }
             }
-            __syncthreads();
-            for (int idx2 = threadIdx.x; idx2 < k * nrhs; idx2 += TH) {
-                const int r = idx2 % k, j = idx2 / k;
-                double *bj = B + (size_t)j * I.ldb;
-                bj[r] -= A[(size_t)r + (size_t)k * I.lda] * bj[k];
+            // A(k, c) + sc d_c: v^T of the column for c > kk, V^T v for c < kk
+            const double e = fma(sc, d, p), w = tau * e;
+            if (q == 0) {
+                s.w[c] = w;
+                s.f[c] = sc * w;
+                s.g[c] = e;
             }
-            __syncthreads();
+            if (lane == 0) {
+                s.sc = sc;
+                s.beta = scaled ? scalbn(beta, s.exp2) : beta;
+                s.tau[kk] = tau;
+                s.redo = redo;
+            }
+            __syncwarp();
+            // T(:, kk) = -tau T(:, 0:kk) g
+            if (lane < NB) {
+                double t = 0.0;
+                for (int u = lane; u < kk; u++) t = fma(s.T[lane][u], s.g[u], t);
+                s.T[lane][kk] = lane < kk ? (tau == 0.0 ? 0.0 : -tau * t) : (lane == kk ? tau : 0.0);
+            }
         }
-        if (threadIdx.x == 0) info[t] = bad;
         __syncthreads();
     }
+
+    // rare: scale rows k.. of column k by a power of two taken from their
+    // largest exponent
+    __device__ void rescale(int k)
+    {
+        double *x = A + (size_t)k * lda;
+        if (tid == 0) s.emax[rank] = s.nz[rank] = 0;
+        __syncthreads();
+        int e = 0, nz = 0;
+        for (int r = lo + tid; r < hi; r += TH) {
+            if (r < k) continue;
+            const unsigned long long u = (unsigned long long)__double_as_longlong(x[r]) << 1;
+            if (r > k && u) nz = 1;
+            const int ex = (int)(u >> 53);  // exponent + 64; a subnormal's from its leading bit
+            e = max(e, u ? (ex ? ex + 64 : 75 - __clzll((long long)u)) : 0);
+        }
+        atomicMax(&s.emax[rank], e);
+        if (nz) atomicOr(&s.nz[rank], 1);
+        __syncthreads();
+        if (CS > 1) {
+            const int te = s.emax[rank], tn = s.nz[rank];
+            __syncthreads();
+            if (tid < CS) {
+                *remote<CS>(&s.emax[rank], tid) = te;
+                *remote<CS>(&s.nz[rank], tid) = tn;
+            }
+            team_sync<CS>();
+        }
+        int ex = 0, any = 0;
+        for (int u = 0; u < CS; u++) {
+            ex = max(ex, s.emax[u]);
+            any |= s.nz[u];
+        }
+        const int sh = (ex == 0 || ex >= 0x7FF + 64) ? 0 : ex - 64 - 1023;
+        for (int r = lo + tid; r < hi; r += TH)
+            if (r >= k) x[r] = scalbn(x[r], -sh);
+        team_sync<CS>();  // all have read emax and nz
+        if (tid == 0) {
+            s.exp2 = sh;
+            s.below = any;
+        }
+        __syncthreads();
+    }
+
+    template <int KK>
+    __device__ void columns(int j0, int jb, double (&acc)[NB])
+    {
+        if (KK >= jb) return;
+        const int k = j0 + KK;
+        reflect(j0, jb, KK, k & 1, acc, false);
+        if (s.redo) {
+            rescale(k);
+            dots(j0, jb, KK, k & 1, acc);
+            reflect(j0, jb, KK, k & 1, acc, true);
+        }
+        pass<KK>(j0, jb, (k + 1) & 1, acc);
+        if constexpr (KK + 1 < NB) columns<KK + 1>(j0, jb, acc);
+    }
+
+    // V(r, 0..7) of the panel: rows above j0 + 7 need the unit lower mask
+    __device__ __forceinline__ void load_v(int j0, int jb, int r, bool top, double (&v)[NB])
+    {
+        const double *row = A + (size_t)j0 * lda + r;
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            v[i] = i < jb ? row[(size_t)i * lda] : 0.0;
+            if (top) v[i] = (i >= jb || r < j0 + i) ? 0.0 : (r == j0 + i ? 1.0 : v[i]);
+        }
+    }
+
+    // W(i, j) of one column group over this CTA's rows, sum i UW + j in lane i UW + j
+    __device__ double group_w(int j0, int jb, int c0, int nc)
+    {
+        double acc[NB * UW];
+#pragma unroll
+        for (int u = 0; u < NB * UW; u++) acc[u] = 0.0;
+        const double *col[UW];
+#pragma unroll
+        for (int j = 0; j < UW; j++) col[j] = colp(A, lda, B, ldb, n, c0 + min(j, nc - 1));
+        for (int r0 = lo + max(j0 - lo, 0) / 32 * 32; r0 < hi; r0 += 32) {
+            const int r = r0 + lane;
+            if (r >= hi) continue;
+            double v[NB];
+            load_v(j0, jb, r, r0 < j0 + NB, v);
+#pragma unroll
+            for (int j = 0; j < UW; j++) {
+                const double cv = r >= j0 ? col[j][r] : 0.0;
+#pragma unroll
+                for (int i = 0; i < NB; i++) acc[i * UW + j] = fma(v[i], cv, acc[i * UW + j]);
+            }
+        }
+        __syncwarp();
+        return reduce32(acc, lane);
+    }
+
+    // T^T W, W's entries one per lane
+    __device__ __forceinline__ double times_t(double w)
+    {
+        const int i = lane / UW, j = lane % UW;
+        double x = 0.0;
+#pragma unroll
+        for (int p = 0; p < NB; p++) x = fma(s.T[p][i], __shfl_sync(0xffffffffu, w, p * UW + j), x);
+        return x;
+    }
+
+    // C -= V W of one column group over this CTA's rows
+    __device__ void group_update(int j0, int jb, int c0, int nc, const double *w)
+    {
+        double ww[NB * UW];
+#pragma unroll
+        for (int u = 0; u < NB * UW; u++) ww[u] = w[u];
+        double *col[UW];
+#pragma unroll
+        for (int j = 0; j < UW; j++) col[j] = colp(A, lda, B, ldb, n, c0 + min(j, nc - 1));
+        for (int r0 = lo + max(j0 - lo, 0) / 32 * 32; r0 < hi; r0 += 32) {
+            const int r = r0 + lane;
+            if (r < j0 || r >= hi) continue;
+            double v[NB];
+            load_v(j0, jb, r, r0 < j0 + NB, v);
+#pragma unroll
+            for (int j = 0; j < UW; j++) {
+                if (j >= nc) break;
+                double x = col[j][r];
+#pragma unroll
+                for (int i = 0; i < NB; i++) x = fma(-v[i], ww[i * UW + j], x);
+                col[j][r] = x;
+            }
+        }
+        __syncwarp();
+    }
+
+    __device__ void trailing(int j0, int jb)
+    {
+        const int ncol = n + nrhs, first = j0 + jb, groups = (ncol - first + UW - 1) / UW;
+        if (CS == 1) {
+            for (int q = warp; q < groups; q += NW) {
+                const int c0 = first + UW * q, nc = min(UW, ncol - c0);
+                s.wb[warp][lane] = times_t(group_w(j0, jb, c0, nc));
+                __syncwarp();
+                group_update(j0, jb, c0, nc, s.wb[warp]);
+            }
+            return;
+        }
+        for (int g0 = 0; g0 < groups; g0 += MAXG) {
+            const int ng = min(MAXG, groups - g0);
+            for (int q = warp; q < ng; q += NW) {
+                const int c0 = first + UW * (g0 + q);
+                s.part[q][lane] = group_w(j0, jb, c0, min(UW, ncol - c0));
+            }
+            team_sync<CS>();
+            for (int q = rank + CS * warp; q < ng; q += CS * NW) {
+                double w = 0.0;
+#pragma unroll
+                for (int u = 0; u < CS; u++) w += *remote<CS>(&s.part[q][lane], u);
+                w = times_t(w);
+#pragma unroll
+                for (int u = 0; u < CS; u++) *remote<CS>(&s.wt[q][lane], u) = w;
+            }
+            team_sync<CS>();
+            for (int q = warp; q < ng; q += NW) {
+                const int c0 = first + UW * (g0 + q);
+                group_update(j0, jb, c0, min(UW, ncol - c0), s.wt[q]);
+            }
+        }
+    }
+
+    // R x = y for one right-hand side by one warp, x over B(0:n, j); returns
+    // k + 1 of the smallest k with a zero or non-finite R(k, k), 0 if none
+    __device__ int back_substitute(int j)
+    {
+        double *b = B + (size_t)j * ldb;
+        int bad = 0;
+        // row blocks of 32 from the bottom: the block's own triangle from
+        // registers, then the rows above it
+        for (int q = (n - 1) / 32; q >= 0; q--) {
+            const int r = 32 * q + lane, nk = min(32, n - 32 * q);
+            const bool on = r < n;
+            double y = on ? b[r] : 0.0;
+            const double d = on ? A[(size_t)r + (size_t)r * lda] : 1.0;
+            const double ad = fabs(d);
+            const bool plain = ad >= 1e-290 && ad <= 1e290;
+            const double inv = plain ? copysign(rcp_nr(ad), d) : 1.0 / d;
+            const bool is_bad = d == 0.0 || !isfinite(d);
+            const unsigned bm = __ballot_sync(0xffffffffu, on && is_bad);
+            if (bm) bad = 32 * q + __ffs(bm);
+            double col = nk > 1 && r < n ? A[(size_t)r + (size_t)(32 * q + nk - 1) * lda] : 0.0;
+            for (int k = nk - 1; k >= 0; k--) {
+                const double cur = col;
+                if (k > 0 && on) col = A[(size_t)r + (size_t)(32 * q + k - 1) * lda];
+                // lane k: y / d, the quotient corrected by one residual step
+                double x = y * inv;
+                if (plain) x = fma(fma(-x, d, y), inv, x);
+                if (!plain) x = is_bad ? NAN : y / d;
+                x = __shfl_sync(0xffffffffu, x, k);
+                if (lane == k) y = x;
+                if (lane < k) y = fma(-cur, x, y);
+            }
+            if (on) b[r] = y;
+            // rows above: b(0:32 q) -= R(0:32 q, block) x
+            for (int rr = lane; rr < 32 * q; rr += 32) {
+                double z = b[rr];
+                for (int k = 0; k < nk; k++) {
+                    // x_k from lane k: every lane takes part (32 q is a multiple of 32)
+                    const double xk = __shfl_sync(0xffffffffu, y, k);
+                    z = fma(-A[(size_t)rr + (size_t)(32 * q + k) * lda], xk, z);
+                }
+                b[rr] = z;
+            }
+            __syncwarp();
+        }
+        return bad;
+    }
+
+    __device__ void solve(const Inst &I, double *a, double *b, int nr, int *info)
+    {
+        m = I.m;
+        n = I.n;
+        lda = I.lda;
+        ldb = I.ldb;
+        A = a;
+        B = b;
+        nrhs = nr;
+        const int rows = ((m + CS - 1) / CS + 31) / 32 * 32;  // whole warps, coalesced
+        lo = min(m, rank * rows);
+        hi = min(m, lo + rows);
+        for (int j0 = 0; j0 < n; j0 += NB) {
+            const int jb = min(NB, n - j0);
+            for (int u = tid; u < NB * NB; u += TH) s.T[u / NB][u % NB] = 0.0;
+            double acc[NB];
+            dots(j0, jb, 0, j0 & 1, acc);
+            columns<0>(j0, jb, acc);
+            __syncthreads();
+            trailing(j0, jb);
+            __syncthreads();
+        }
+        team_sync<CS>();
+        for (int j = rank + CS * warp; j < nrhs; j += CS * NW) {
+            const int bad = back_substitute(j);
+            if (j == 0 && lane == 0) *info = bad;
+        }
+        team_sync<CS>();
+    }
+};
+
+// Persistent: teams of CS CTAs take instances order[*from .. *to) from the
+// tier's counter, largest first (null: from the first, to the last).  A tier's
+// launch starts beside the one
+// before it (programmatic launch) and ends after it.
+template <int TH, int CS>
+__global__ void __launch_bounds__(TH, TH <= 256 ? 512 / TH : 1)
+    k_gels(int count, int nrhs, const Inst *inst, double *const *Aptr, double *const *Bptr, const int *order,
+           int *counter, const int *from, const int *to, int *info)
+{
+    __shared__ Shared<TH, CS> s;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    Solver<TH, CS> v(s);
+    v.tid = threadIdx.x;
+    v.warp = threadIdx.x >> 5;
+    v.lane = threadIdx.x & 31;
+    v.rank = CS > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    const int first = from ? *from : 0, last = to ? *to : count;
+    if (CS > 1) team_sync<CS>();  // every CTA of the cluster runs before its memory is written
+    for (;;) {
+        if (v.rank == 0 && threadIdx.x == 0) {
+            const int idx = atomicAdd(counter, 1);
+            for (int u = 0; u < CS; u++) *remote<CS>(&s.idx, u) = idx;
+        }
+        team_sync<CS>();
+        const int at = first + s.idx;
+        if (at >= last) break;
+        const int t = order[at];
+        v.solve(inst[t], Aptr[t], Bptr[t], nrhs, info + t);
+    }
+    if (CS > 1) team_sync<CS>();  // no CTA leaves while its memory may still be written
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace bat
@@ -319,8 +589,10 @@ struct BatchMeta {
     int count, nrhs;
     bat::Inst *inst;
     double **Aptr, **Bptr;
-    int *order, *counter;
+    int *order, *counter;  // counter[0 .. TIERS): the launches' queues, then TIERS + 1 bounds of their instances
 };
+
+constexpr double kTier8 = 1.0, kTier4 = 0.16;  // of the work per SM
 
 static long long batch_bytes(int count)
 {
@@ -348,18 +620,68 @@ static BatchMeta carve_meta(void *work, int count)
 // launch configuration (threads, CTAs per SM), chosen by lila_gpu_gels_autotune
 static int g_gels_threads = 256, g_gels_per_sm = 2;
 
+// One tier's launch over order[*from .. *to): as many clusters as are resident
+// at once (the next tier starts beside it only when all its CTAs have
+// started).  False (nothing enqueued) when the device refuses such clusters.
+template <int TH, int CS>
+static bool launch_tier(const BatchMeta &b, int nrhs, int *info, int tier, const int *from, const int *to, bool beside)
+{
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(sm_count() * g_gels_per_sm);
+    cfg.blockDim = dim3(TH);
+    cfg.stream = stream();
+    cfg.attrs = at;
+    if (CS > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs++].val.clusterDim = {CS, 1, 1};
+        int n = 0;
+        cfg.gridDim = dim3(CS);
+        if (cudaOccupancyMaxActiveClusters(&n, bat::k_gels<TH, CS>, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return false;
+        }
+        cfg.gridDim = dim3(CS * n);
+    }
+    if (beside) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cudaLaunchKernelEx(&cfg, bat::k_gels<TH, CS>, b.count, nrhs, (const bat::Inst *)b.inst,
+                           (double *const *)b.Aptr, (double *const *)b.Bptr, (const int *)b.order, b.counter + tier,
+                           from, to, info) == cudaSuccess)
+        return true;
+    if (CS > 1) cudaGetLastError();  // the single CTAs take these instances
+    return false;
+}
+
 static void launch_gels(const BatchMeta &b, int nrhs, int *info)
 {
-    cudaStream_t st = stream();
-    cudaMemsetAsync(b.counter, 0, sizeof(int), st);
-    const int grid = sm_count() * g_gels_per_sm;
+    cudaMemsetAsync(b.counter, 0, bat::TIERS * sizeof(int), stream());
+    trace_break();
     trace_begin();
+    // the instances that would keep one SM busy long after the others go to
+    // clusters (prepare bounds the tiers; none in a batch of over 32 per SM;
+    // always CTAs of 256 threads); what a refused cluster launch leaves goes
+    // to the single CTAs
+    const int *bound = b.counter + bat::TIERS, *from = nullptr;
+    if (b.count <= 32 * sm_count() && launch_tier<256, 8>(b, nrhs, info, 0, bound, bound + 1, false)) {
+        from = bound + 1;
+        note_launch("gels_batched_clusters");
+        trace_begin();
+        if (launch_tier<256, 4>(b, nrhs, info, 1, bound + 1, bound + 2, true)) {
+            from = bound + 2;
+            note_launch("gels_batched_clusters");
+            trace_begin();
+        }
+    }
+    const bool beside = from != nullptr;
     if (g_gels_threads == 128)
-        bat::k_gels<128><<<grid, 128, 0, st>>>(b.count, nrhs, b.inst, b.Aptr, b.Bptr, b.order, b.counter, info);
+        launch_tier<128, 1>(b, nrhs, info, 2, from, nullptr, beside);
     else if (g_gels_threads == 512)
-        bat::k_gels<512><<<grid, 512, 0, st>>>(b.count, nrhs, b.inst, b.Aptr, b.Bptr, b.order, b.counter, info);
+        launch_tier<512, 1>(b, nrhs, info, 2, from, nullptr, beside);
     else
-        bat::k_gels<256><<<grid, 256, 0, st>>>(b.count, nrhs, b.inst, b.Aptr, b.Bptr, b.order, b.counter, info);
+        launch_tier<256, 1>(b, nrhs, info, 2, from, nullptr, beside);
     note_launch("gels_batched");
 }
 
@@ -389,8 +711,30 @@ int lila_dgels_batched_prepare(int count, const int *m, const int *n, int nrhs, 
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return (double)inst[a].m * inst[a].n * inst[a].n > (double)inst[b].m * inst[b].n * inst[b].n;
     });
+    // An instance's team: a cluster of 8 CTAs when its FMAs exceed what the
+    // whole batch spread over all SMs leaves for one, a cluster of 4 from a
+    // sixth of that, provided its columns carry enough rows to pay for the
+    // cluster's exchange; smaller teams waste fewer FP64 slots on reductions.
+    // 500 instances (m up to 4096, n up to 128; 10 ms of FMAs on all SMs): one
+    // CTA each 34 ms (the largest takes that long alone), clusters of 8 or one
+    // 20.6 ms, these tiers 18.7 ms; 60 instances 33.6, 4.6 and 5.2 ms.  An
+    // eighth instead of a sixth gains 5 % there and loses 4 % at 2,000
+    // instances, a quarter the other way round.
+    auto fma = [&](int t) { return (double)inst[t].m * inst[t].n * (inst[t].n + 2.0 * nrhs); };
+    double total = 0.0;
+    for (int t = 0; t < count; t++) total += fma(t);
+    const double share[bat::TIERS - 1] = {kTier8, kTier4};
+    int head[2 * bat::TIERS + 1] = {};
+    for (int tier = 0, at = 0; tier < bat::TIERS - 1; tier++) {
+        while (at < count && fma(order[at]) > share[tier] * total / sm_count() &&
+               (long long)inst[order[at]].m * inst[order[at]].n >= 16384)
+            at++;
+        head[bat::TIERS + tier + 1] = at;
+    }
+    head[2 * bat::TIERS] = count;
     BatchMeta b = carve_meta(work, count);
     cudaStream_t st = stream();
+    cudaMemcpyAsync(b.counter, head, sizeof head, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b.inst, inst.data(), sizeof(bat::Inst) * count, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b.Aptr, A, sizeof(double *) * count, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b.Bptr, B, sizeof(double *) * count, cudaMemcpyHostToDevice, st);
