@@ -18,7 +18,7 @@
 
 #include <cooperative_groups.h>
 
-#include "lg_common.cuh"
+#include "lg_house.cuh"
 #include "../../include/lila_gpu.h"
 
 namespace lg {
@@ -261,28 +261,9 @@ struct Solver {
             const double alpha = __shfl_sync(0xffffffffu, p, 4 * kk), ss = __shfl_sync(0xffffffffu, d, 4 * kk);
             const int k = j0 + kk;
             const bool last = k == m - 1;
-            const double sq = fma(alpha, alpha, ss);
-            const bool redo = !scaled && !last && !(ss >= 1e-280 && sq <= 1e280);
-            const bool below = scaled ? s.below != 0 : !last;
-            double beta = alpha, tau = 0.0, sc = 0.0;
-            if (below) {
-                if (sq >= 1e-290 && sq <= 1e290) {
-                    // |beta| = sqrt(sq) corrected to rounding level, tau = 1 +
-                    // |alpha| / |beta|, sc = 1 / (alpha - beta)
-                    const double y = rsqrt_nr(sq);
-                    double nb = sq * y;
-                    nb = fma(0.5 * y, fma(-nb, nb, sq), nb);
-                    const double t = nb + fabs(alpha);
-                    tau = t * y;
-                    tau = fma(fma(-tau, nb, t), y, tau);
-                    beta = -copysign(nb, alpha);
-                    sc = copysign(rcp_nr(t), alpha);
-                } else {
-                    beta = -copysign(sqrt(sq), alpha);
-                    tau = (beta - alpha) / beta;
-                    sc = 1.0 / (alpha - beta);
-                }
-            }
+            const bool redo = !scaled && !last && !house_in_range(alpha, ss);
+            const Reflector h = house_reflector(alpha, ss, scaled ? s.below != 0 : !last);
+            const double sc = h.sc, tau = h.tau;
             // A(k, c) + sc d_c: v^T of the column for c > kk, V^T v for c < kk
             const double e = fma(sc, d, p), w = tau * e;
             if (q == 0) {
@@ -292,7 +273,7 @@ struct Solver {
             }
             if (lane == 0) {
                 s.sc = sc;
-                s.beta = scaled ? scalbn(beta, s.exp2) : beta;
+                s.beta = scaled ? scalbn(h.beta, s.exp2) : h.beta;
                 s.tau[kk] = tau;
                 s.redo = redo;
             }
@@ -317,10 +298,9 @@ struct Solver {
         int e = 0, nz = 0;
         for (int r = lo + tid; r < hi; r += TH) {
             if (r < k) continue;
-            const unsigned long long u = (unsigned long long)__double_as_longlong(x[r]) << 1;
-            if (r > k && u) nz = 1;
-            const int ex = (int)(u >> 53);  // exponent + 64; a subnormal's from its leading bit
-            e = max(e, u ? (ex ? ex + 64 : 75 - __clzll((long long)u)) : 0);
+            const int xe = house_exponent(x[r]);
+            if (r > k && xe) nz = 1;
+            e = max(e, xe);
         }
         atomicMax(&s.emax[rank], e);
         if (nz) atomicOr(&s.nz[rank], 1);
@@ -339,7 +319,7 @@ struct Solver {
             ex = max(ex, s.emax[u]);
             any |= s.nz[u];
         }
-        const int sh = (ex == 0 || ex >= 0x7FF + 64) ? 0 : ex - 64 - 1023;
+        const int sh = house_shift(ex);
         for (int r = lo + tid; r < hi; r += TH)
             if (r >= k) x[r] = scalbn(x[r], -sh);
         team_sync<CS>();  // all have read emax and nz

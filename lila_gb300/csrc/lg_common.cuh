@@ -238,56 +238,37 @@ int mixed_leaf_entry(int m, int n, int i, int mt, double *A, int lda, double *T,
                      double *work, long long lwork, int variant);
 
 #ifdef __CUDACC__
-// 1 / sqrt(d) for a positive finite d: Newton–Raphson on f(y) = y^-2 - d,
-// y <- y + y (1 - d y^2) / 2, two steps from the single-precision estimate
-// rsqrtf of d scaled into [1, 4) by an even power of two (the seed's relative
-// error below 2^-21 becomes ~2^-42, then rounding level; the result is
-// within about 1.5 ulp).  The scalings and conversions are exact exponent
-// and bit moves, so the pivot chain holds six FP64 operations.
-__device__ __forceinline__ double rsqrt_nr(double d)
+// 1 / sqrt(d) for a positive normal d: one third-order (Householder) step on
+// f(y) = y^-2 - d, y <- y + y (r / 2 + 3 r^2 / 8), r = 1 - d y^2, from the
+// hardware estimate rsqrt.approx.ftz.f64 (relative error e about 2^-20: the step
+// leaves 5 e^3 / 2, below 2^-57, then rounding level).  Five FP64 operations,
+// each 64 clocks of a dependent chain; a single-precision seed moved in and out
+// of the FP64 format cost as much again in integer instructions.
+__device__ __forceinline__ double rsqrt_normal(double d)
 {
-    int hi = __double2hiint(d);
-    int lo = __double2loint(d);
-    int adj = 0;
-    if (((hi >> 20) & 0x7FF) == 0) {  // subnormal: scale by 2^64 first
-        const double s = d * 0x1p64;
-        hi = __double2hiint(s);
-        lo = __double2loint(s);
-        adj = 32;
-    }
-    const int e = ((hi >> 20) & 0x7FF) - 1023;
-    const int k = e >> 1;  // floor(e / 2)
-    const int hm = hi - 2 * k * 1048576;  // dm = d 2^-2k in [1, 4)
-    const double dm = __hiloint2double(hm, lo);
-    // dm as a float (mantissa truncated to 23 bits), its rsqrtf, and that as a double
-    const float fm = __int_as_float((((hm >> 20) - 1023 + 127) << 23) | ((hm & 0xFFFFF) << 3) |
-                                    (int)((unsigned)lo >> 29));
-    const unsigned yb = __float_as_uint(rsqrtf(fm));
-    double y = __hiloint2double((int)((((yb >> 23) - 127 + 1023) << 20) | ((yb & 0x7FFFFFu) >> 3)),
-                                (int)((yb & 7u) << 29));
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const double t = dm * y;
-        const double r = fma(-t, y, 1.0);
-        y = fma(0.5 * y, r, y);
-    }
-    // 1 / sqrt(d) = y 2^(adj - k)
-    return __hiloint2double(__double2hiint(y) + (adj - k) * 1048576, __double2loint(y));
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double r = fma(-(d * y), y, 1.0);
+    return fma(y, r * fma(0.375, r, 0.5), y);
 }
 
-// 1 / d for a positive d in [2^-1000, 2^1000]: Newton–Raphson y <- y + y (1 - d y),
-// two steps from a single-precision reciprocal of d's mantissa (its error
-// below 2^-22 becomes ~2^-44, then rounding level), four FP64 operations.
+// The same for any positive finite d: a subnormal one (rare, kept out of line:
+// the compiler would issue its scalings for every d) is scaled by 2^64 first.
+static __device__ __noinline__ double rsqrt_subnormal(double d) { return rsqrt_normal(d * 0x1p64) * 0x1p32; }
+__device__ __forceinline__ double rsqrt_nr(double d)
+{
+    return (__double2hiint(d) >> 20) == 0 ? rsqrt_subnormal(d) : rsqrt_normal(d);
+}
+
+// 1 / d for a positive d in [2^-1000, 2^1000]: one third-order step y <- y + y
+// (e + e^2), e = 1 - d y, from rcp.approx.ftz.f64 (e^3 below 2^-57, then
+// rounding level), three FP64 operations.
 __device__ __forceinline__ double rcp_nr(double d)
 {
-    const int hi = __double2hiint(d), lo = __double2loint(d);
-    const float fm = __int_as_float((127 << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)lo >> 29));
-    const unsigned yb = __float_as_uint(__frcp_rn(fm));  // in (1/2, 1]
-    const int e = (int)(yb >> 23) - 127 - ((hi >> 20) - 1023);
-    double y = __hiloint2double((int)(((unsigned)(e + 1023) << 20) | ((yb & 0x7FFFFFu) >> 3)), (int)((yb & 7u) << 29));
-#pragma unroll
-    for (int it = 0; it < 2; it++) y = fma(y, fma(-d, y, 1.0), y);
-    return y;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 #endif
 

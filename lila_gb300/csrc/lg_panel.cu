@@ -34,7 +34,7 @@
 // and (optionally) the explicit Q in one launch.
 #include <math.h>
 
-#include "lg_common.cuh"
+#include "lg_house.cuh"
 
 namespace lg {
 namespace pnl {
@@ -54,38 +54,6 @@ __host__ __device__ inline int lanes_for(int threads, int n)
 // The leading dimension in shared memory: lanes modulo 16, so the 16 / lanes
 // columns that a half warp reads fall into different banks.
 __host__ __device__ inline int pad_ld(int rows, int lanes) { return ((rows - lanes + 15) / 16 * 16) + lanes; }
-
-struct Reflector {
-    double beta, tau, sc;
-};
-
-// dlarfg from alpha and the sum of squares below it; `below` says whether
-// anything below the pivot is nonzero.  |beta| = sqrt(alpha^2 + ss) corrected
-// to rounding level, tau = 1 + |alpha| / |beta|, sc = 1 / (alpha - beta).
-__device__ __forceinline__ Reflector reflector(double alpha, double ss, bool below)
-{
-    if (!below) return Reflector{alpha, 0.0, 0.0};
-    const double s = fma(alpha, alpha, ss), a = fabs(alpha);
-    if (s >= 1e-290 && s <= 1e290) {
-        const double y = rsqrt_nr(s);
-        double b = s * y;
-        b = fma(0.5 * y, fma(-b, b, s), b);
-        const double t = b + a;
-        double tau = t * y;
-        tau = fma(fma(-tau, b, t), y, tau);
-        return Reflector{-copysign(b, alpha), tau, copysign(rcp_nr(t), alpha)};
-    }
-    const double beta = -copysign(sqrt(s), alpha);
-    return Reflector{beta, (beta - alpha) / beta, 1.0 / (alpha - beta)};
-}
-
-template <int LG>
-__device__ __forceinline__ double group_sum(double v)
-{
-#pragma unroll
-    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // ---- tagged slots -----------------------------------------------------------
 __device__ __forceinline__ void slot_put(uint4 *p, double v, uint32_t tag)
@@ -159,7 +127,7 @@ __global__ void __launch_bounds__(NT, 1)
             long long limit, uint32_t tag_skew)
 {
     extern __shared__ double X[];  // nb columns, ld
-    __shared__ double s_tau, s_sc[MAXNB], s_beta[MAXNB], s_d[MAXNB], s_p[MAXNB];
+    __shared__ double s_tau, s_f, s_sc[MAXNB], s_beta[MAXNB], s_d[MAXNB], s_p[MAXNB];
     __shared__ int s_fail;
     constexpr int NW = NT / 32;
     const int G = gridDim.x, b = blockIdx.x;
@@ -212,8 +180,9 @@ __global__ void __launch_bounds__(NT, 1)
         if (wc1 > j) {
             if (mine && c >= j) ok = slot_wait(pivot + c, tag, limit, pr) && slot_wait(total + c, tag, limit, d) && ok;
             if (c == j && g == 0) {
-                const Reflector h = reflector(pr, d, d != 0.0);
+                const Reflector h = house_reflector(pr, d, d != 0.0);
                 s_tau = h.tau;
+                s_f = h.tau * h.sc;
                 s_sc[j] = h.sc;
                 s_beta[j] = h.beta;
                 if (owner) tau[j] = h.tau;
@@ -227,10 +196,10 @@ __global__ void __launch_bounds__(NT, 1)
         }
         const double tj = s_tau, sc = s_sc[j];
         if (wc1 > j + 1 && tj != 0.0 && mine && c > j) {
-            const double w = tj * fma(sc, d, pr), f = sc * w;
+            const double e = fma(sc, d, pr), f = s_f * e;
 #pragma unroll 4
             for (int r = first + g; r < nr; r += LG) xc[r] = fma(-f, xj[r], xc[r]);
-            if (g == 0 && owner) xc[j - r0] -= w;
+            if (owner && g == 0) xc[j - r0] = fma(-tj, e, pr);
         }
         // (V^T V)(cc, j) = v_cc(j) + sum_{r > j} v_cc(r) v_j(r)
         for (int cc = b + warp * G; cc < j; cc += NW * G)
@@ -269,6 +238,7 @@ __global__ void __launch_bounds__(NTS, 1)
     const int tw = min(mt, n);
     double *X = sm, *Ts = X + (size_t)ld * n, *s_d = Ts + tw * (tw + 1), *s_g = s_d + n, *s_sc = s_g + n,
            *s_tau = s_sc + n, *s_beta = s_tau + n;
+    __shared__ double s_f;
     __shared__ int s_redo, s_exp, s_nz;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cg = threadIdx.x / LG, g = threadIdx.x % LG;
@@ -295,11 +265,12 @@ __global__ void __launch_bounds__(NTS, 1)
                 s_d[c] = d;
                 if (c == j) {
                     const double alpha = xj[j];
-                    const double s = fma(alpha, alpha, d);
                     const bool last = j == m - 1;
-                    if (!scaled) s_redo = !last && !(d >= 1e-280 && s <= 1e280);
-                    const Reflector h = reflector(alpha, d, scaled ? s_nz != 0 : !last);
+                    if (!scaled) s_redo = !last && !house_in_range(alpha, d);
+                    const Reflector h = house_reflector(alpha, d, scaled ? s_nz != 0 : !last);
                     s_tau[j] = h.tau;
+                    s_f = h.tau * h.sc;
+                    if (scaled || !s_redo) X[j + j * ld] = h.u;  // u's pivot entry, until V goes out
                     s_sc[j] = h.sc;
                     s_beta[j] = scaled ? scalbn(h.beta, s_exp) : h.beta;
                 }
@@ -355,18 +326,14 @@ __global__ void __launch_bounds__(NTS, 1)
             __syncthreads();
             int e = 0, nz = 0;
             for (int r = j + threadIdx.x; r < m; r += NTS) {
-                const unsigned long long u = (unsigned long long)__double_as_longlong(xj[r]) << 1;
-                if (r > j && u) nz = 1;
-                // exponent + 64; a subnormal's from its leading bit
-                const int ex = (int)(u >> 53);
-                e = max(e, u ? (ex ? ex + 64 : 75 - __clzll((long long)u)) : 0);
+                const int x = house_exponent(xj[r]);
+                if (r > j && x) nz = 1;
+                e = max(e, x);
             }
             atomicMax(&s_exp, e);
             if (nz) atomicOr(&s_nz, 1);
             __syncthreads();
-            // biased (+64) exponent -> power of two; nothing to scale in a zero
-            // or non-finite column
-            const int ex = s_exp, k = (ex == 0 || ex >= 0x7FF + 64) ? 0 : ex - 64 - 1023;
+            const int k = house_shift(s_exp);
             __syncthreads();
             if (threadIdx.x == 0) s_exp = k;
             for (int r = j + threadIdx.x; r < m; r += NTS) xj[r] = scalbn(xj[r], -k);
@@ -380,17 +347,14 @@ __global__ void __launch_bounds__(NTS, 1)
             const int c = c0 + cg;
             const bool on = c >= ts && c < n && c != j, right = on && c > j && tj != 0.0;
             double *xc = X + (on ? c : j) * ld;
-            const double w = on ? fma(sc, s_d[c], xc[j]) : 0.0;
-            if (right) {
-                const double f = sc * (tj * w);
-#pragma unroll 4
-                for (int r = j + 1 + g; r < m; r += LG) xc[r] = fma(-f, xj[r], xc[r]);
-            }
+            const double e = on ? fma(sc, s_d[c], xc[j]) : 0.0;
             __syncwarp();  // the group has read its pivot entry
-            if (g == 0) {
-                if (right) xc[j] -= tj * w;
-                if (on && c < j) s_g[c] = s_sc[c] * w;
+            if (right) {
+                const double f = s_f * e;
+#pragma unroll 4
+                for (int r = j + g; r < m; r += LG) xc[r] = fma(-f, xj[r], xc[r]);
             }
+            if (on && c < j && g == 0) s_g[c] = s_sc[c] * e;
         }
         __syncthreads();
     }
