@@ -271,8 +271,10 @@ void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const G
           double *part, long long part_len, const char *tag)
 {
     if (M <= 0 || N <= 0) return;
-    // large products go to the tensor cores in split-precision mode
-    if (precision() == 1 && M >= 64 && N >= 64 && K >= 64 && (double)M * N * K >= 134217728.0) {
+    // large products go to the tensor cores in split-precision mode: from 2^25
+    // multiply-adds, where both take the same time (128 x 128 x 3000: FP64 95 us,
+    // split 72; 3000 x 64 x 128: 48 and 47; 128 x 64 x 3000: 54 and 70)
+    if (precision() == 1 && M >= 64 && N >= 64 && K >= 64 && (double)M * N * K >= 33554432.0) {
         ozgemm(M, N, K, A, B, C, ldc, e, part, part_len, "ozgemm");
         return;
     }

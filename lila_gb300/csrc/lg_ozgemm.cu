@@ -77,6 +77,28 @@ __device__ __forceinline__ unsigned long long opb(const Operand &B, int N, int k
     return B.trans == NT ? masked_bits(B.p, B.ld, B.mask, k, c) : masked_bits(B.p, B.ld, B.mask, c, k);
 }
 
+// The K range [lo, hi) of [kbeg, kend) in which the rows (columns) [x0, x0 + nx)
+// of op(A) (op(B)) are stored values: inside the matrix and off the mask's
+// zeros and ones.  `rowwise`: the stored row index is x, not k (op(A) of an
+// untransposed A, op(B) of a transposed B).  There the loads need no test per
+// element: with one, splitting a value took ~100 instructions, two thirds of
+// them for its load.
+struct PlainRange {
+    int lo, hi;
+};
+__device__ __forceinline__ PlainRange plain_range(int mask, bool rowwise, bool inside, int x0, int nx, int kbeg, int kend)
+{
+    PlainRange p{kbeg, kend};
+    if (!inside) p.hi = kbeg;
+    if (mask == M_FULL) return p;
+    const bool lower = mask == M_UNIT_LOWER || mask == M_LOWER;
+    if (lower == rowwise)  // k below every x
+        p.hi = min(p.hi, x0);
+    else  // k above every x
+        p.lo = max(p.lo, x0 + nx);
+    return p;
+}
+
 // Digits of 4 consecutive K values (half hf of a unit) -> 8-byte stores.
 __device__ __forceinline__ void store_half(uint8_t *base, uint32_t slice_bytes, int idx, int kg, int hf,
                                            const uint32_t (&w01)[NS], const uint32_t (&w23)[NS])
@@ -132,7 +154,7 @@ __device__ __forceinline__ double dfma_nospec(double a, double b, double c)
 }
 
 __device__ __forceinline__ void epi_store(double v, int r, int c, double *C, int ldc, const GemmEpi &e,
-                                          const EpiMode &md)
+                                          const EpiMode &md, bool use_c, double cval)
 {
     if (e.upper_only && r > c) return;
     double out;
@@ -144,7 +166,7 @@ __device__ __forceinline__ void epi_store(double v, int r, int c, double *C, int
         out = dmul_nospec(e.alpha, v);
     if (e.add_diag && r == c) out = dadd_nospec(out, 1.0);
     const size_t off = (size_t)r + (size_t)c * (size_t)ldc;
-    if (md.use_beta && r >= e.zero_rows) out = dfma_nospec(e.beta, C[off], out);
+    if (use_c) out = dfma_nospec(e.beta, cval, out);
     C[off] = out;
 }
 
@@ -283,13 +305,69 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
         bk = bu >> 6;
     }
     unsigned long long ra[8], rb[4];
+    const PlainRange pa = plain_range(A.mask, A.trans == NT, row0 + BM <= M, row0, BM, kbeg, kend);
+    const PlainRange pb = plain_range(B.mask, B.trans == TR, col0 + BN <= N, col0, BN, kbeg, kend);
+    // two values per load where they are contiguous along K and 16-byte aligned
+    const bool va = ((uintptr_t)A.p & 15) == 0 && (A.ld & 1) == 0 && (kbeg & 1) == 0;
+    const bool vb = ((uintptr_t)B.p & 15) == 0 && (B.ld & 1) == 0 && (kbeg & 1) == 0;
     auto load_stage = [&](int ch2) {
         const int k1 = kbeg + ch2 * KC;
-        const bool live = ch2 < nch;
+        if (ch2 >= nch) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) ra[j] = live ? opa(A, M, row0 + ar, k1 + ak * 8 + j, kend) : 0ull;
+            for (int j = 0; j < 8; j++) ra[j] = 0ull;
 #pragma unroll
-        for (int j = 0; j < 4; j++) rb[j] = live ? opb(B, N, k1 + bk * 8 + 4 * bh + j, col0 + bc, kend) : 0ull;
+            for (int j = 0; j < 4; j++) rb[j] = 0ull;
+            return;
+        }
+        const int ka = k1 + ak * 8, kb = k1 + bk * 8 + 4 * bh;
+        if (k1 >= pa.lo && k1 + KC <= pa.hi) {
+            const unsigned long long *q = (const unsigned long long *)A.p;
+            if (A.trans == NT) {
+                q += (size_t)(row0 + ar) + (size_t)ka * A.ld;
+#pragma unroll
+                for (int j = 0; j < 8; j++) ra[j] = q[(size_t)j * A.ld];
+            } else {
+                q += (size_t)ka + (size_t)(row0 + ar) * A.ld;
+                if (va) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const ulonglong2 t = ((const ulonglong2 *)q)[j];
+                        ra[2 * j] = t.x;
+                        ra[2 * j + 1] = t.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) ra[j] = q[j];
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) ra[j] = opa(A, M, row0 + ar, ka + j, kend);
+        }
+        if (k1 >= pb.lo && k1 + KC <= pb.hi) {
+            const unsigned long long *q = (const unsigned long long *)B.p;
+            if (B.trans == NT) {
+                q += (size_t)kb + (size_t)(col0 + bc) * B.ld;
+                if (vb) {
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const ulonglong2 t = ((const ulonglong2 *)q)[j];
+                        rb[2 * j] = t.x;
+                        rb[2 * j + 1] = t.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) rb[j] = q[j];
+                }
+            } else {
+                q += (size_t)(col0 + bc) + (size_t)kb * B.ld;
+#pragma unroll
+                for (int j = 0; j < 4; j++) rb[j] = q[(size_t)j * B.ld];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) rb[j] = opb(B, N, kb + j, col0 + bc, kend);
+        }
     };
     // the first stage's operands and the precomputed scales are loaded before
     // the barrier, so their latency overlaps the wait for the previous tile
@@ -304,20 +382,29 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
     // ---- scaling groups over [kbeg, kend): the largest biased exponent of
     // every row of op(A) and every column of op(B); lanes run along the
     // stored contiguous dimension
+    // (inside the plain range from the high words alone, without a test per
+    // element)
+    auto high = [](const double *q, size_t at) { return ((const int *)(q + at))[1] & 0x7FFFFFFF; };
     if (rexp) {
         // precomputed
     } else if (A.trans == NT) {
         const int r = tid & 127;
-        int mx = 0;
+        int mx = 0, hi = 0;
+        for (int k = kbeg + (tid >> 7); k < min(kend, pa.lo); k += 4) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
+        for (int k = max(pa.lo, pa.hi) + (tid >> 7); k < kend; k += 4) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
+        const double *q = A.p + row0 + r;
 #pragma unroll 8
-        for (int k = kbeg + (tid >> 7); k < kend; k += 4) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
-        atomicMax(&s_rexp[r], mx);
+        for (int k = pa.lo + (tid >> 7); k < pa.hi; k += 4) hi = max(hi, high(q, (size_t)k * A.ld));
+        atomicMax(&s_rexp[r], max(mx, hi >> 20));
     } else {
         for (int r = warp; r < BM; r += OZT / 32) {
-            int mx = 0;
-#pragma unroll 4
-            for (int k = kbeg + lane; k < kend; k += 32) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
-            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            int mx = 0, hi = 0;
+            for (int k = kbeg + lane; k < min(kend, pa.lo); k += 32) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
+            for (int k = max(pa.lo, pa.hi) + lane; k < kend; k += 32) mx = max(mx, oz::bexp(opa(A, M, row0 + r, k, kend)));
+            const double *q = A.p + (size_t)(row0 + r) * A.ld;
+#pragma unroll 8
+            for (int k = pa.lo + lane; k < pa.hi; k += 32) hi = max(hi, high(q, k));
+            mx = __reduce_max_sync(0xffffffffu, max(mx, hi >> 20));
             if (lane == 0) s_rexp[r] = mx;
         }
     }
@@ -325,18 +412,24 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
         // precomputed
     } else if (B.trans == NT) {
         for (int c = warp; c < BN; c += OZT / 32) {
-            int mx = 0;
-#pragma unroll 4
-            for (int k = kbeg + lane; k < kend; k += 32) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
-            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            int mx = 0, hi = 0;
+            for (int k = kbeg + lane; k < min(kend, pb.lo); k += 32) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
+            for (int k = max(pb.lo, pb.hi) + lane; k < kend; k += 32) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
+            const double *q = B.p + (size_t)(col0 + c) * B.ld;
+#pragma unroll 8
+            for (int k = pb.lo + lane; k < pb.hi; k += 32) hi = max(hi, high(q, k));
+            mx = __reduce_max_sync(0xffffffffu, max(mx, hi >> 20));
             if (lane == 0) s_cexp[c] = mx;
         }
     } else {
         const int c = tid & 63;
-        int mx = 0;
+        int mx = 0, hi = 0;
+        for (int k = kbeg + (tid >> 6); k < min(kend, pb.lo); k += 8) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
+        for (int k = max(pb.lo, pb.hi) + (tid >> 6); k < kend; k += 8) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
+        const double *q = B.p + col0 + c;
 #pragma unroll 8
-        for (int k = kbeg + (tid >> 6); k < kend; k += 8) mx = max(mx, oz::bexp(opb(B, N, k, col0 + c, kend)));
-        atomicMax(&s_cexp[c], mx);
+        for (int k = pb.lo + (tid >> 6); k < pb.hi; k += 8) hi = max(hi, high(q, (size_t)k * B.ld));
+        atomicMax(&s_cexp[c], max(mx, hi >> 20));
     }
     __syncthreads();
     if (tid < BM && s_rexp[tid] == 0x7FF) atomicOr(status, ST_NONFINITE);
@@ -419,24 +512,36 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
         const int r = 32 * q + lane, gr = row0 + r;
         const int er = s_rexp[r];
         if (gr < M) {
+            // eight outputs at a time, C's values (beta) loaded together before
+            // the first is used
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const int c = 16 * h + j, gc = col0 + c;
-                if (gc >= N) continue;
-                const int ec = s_cexp[c];
-                double v;
-                if (er == 0x7FF || ec == 0x7FF)
-                    v = __longlong_as_double(0x7FF8000000000000ll);
-                else if (!(er && ec))
-                    v = 0.0;
-                else if (fast)
-                    v = oz::assemble_fast(acc_hi[j], acc_lo[j], (er - 1022) + (ec - 1022) - 63);
-                else
-                    v = oz::assemble(acc_hi[j], acc_lo[j], (er - 1022) + (ec - 1022) - 63);
-                if (part)
-                    part[(size_t)gr + (size_t)gc * M] = v;
-                else
-                    epi_store(v, gr, gc, C, ldc, e, md);
+            for (int jb = 0; jb < 16; jb += 8) {
+                double cv[8];
+                const bool use = !part && md.use_beta && gr >= e.zero_rows;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int gc = col0 + 16 * h + jb + j;
+                    if (use && gc < N && !(e.upper_only && gr > gc)) cv[j] = C[(size_t)gr + (size_t)gc * ldc];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int c = 16 * h + jb + j, gc = col0 + c;
+                    if (gc >= N) continue;
+                    const int ec = s_cexp[c];
+                    double v;
+                    if (er == 0x7FF || ec == 0x7FF)
+                        v = __longlong_as_double(0x7FF8000000000000ll);
+                    else if (!(er && ec))
+                        v = 0.0;
+                    else if (fast)
+                        v = oz::assemble_fast(acc_hi[jb + j], acc_lo[jb + j], (er - 1022) + (ec - 1022) - 63);
+                    else
+                        v = oz::assemble(acc_hi[jb + j], acc_lo[jb + j], (er - 1022) + (ec - 1022) - 63);
+                    if (part)
+                        part[(size_t)gr + (size_t)gc * M] = v;
+                    else
+                        epi_store(v, gr, gc, C, ldc, e, md, use, cv[j]);
+                }
             }
         }
     }
