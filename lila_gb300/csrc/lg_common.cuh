@@ -97,6 +97,9 @@ void splitk_reduce(int M, int N, int splits, const double *part, double *C, int 
 void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e,
             double *part = nullptr, long long part_len = 0, const char *tag = "ozgemm");
 int ozgemm_splits(int M, int N, int K, long long part_len);
+// Doubles of `part` that let ozgemm split the operands of a block reflector's
+// products (vb columns, m x n block) beforehand; 0 where it would not.
+long long ozgemm_room(long long m, long long n, long long vb);
 // Many independent split-precision GEMMs in one launch: C = alpha op(A) op(B)
 // + beta C per group; d_prefix[g] = tiles of groups 0..g-1 (ozgemm_group_tiles
 // each), total_tiles = all of them; d_tilemap (total_tiles entries) is

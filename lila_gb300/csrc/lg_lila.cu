@@ -194,7 +194,7 @@ static void apply_qt(int m, int n, int k, int i, int mt, const double *A, int ld
         double *Ct = C + a;
         gemm(vb, n, m - a, opnd(V, lda, TR, M_UNIT_LOWER), opnd(Ct, ldc), W1, vb, epi(1, 0), w.p, w.len);
         gemm(vb, n, vb, opnd(Tt, ldt, TR, M_UPPER), opnd(W1, vb), W2, vb, epi(1, 0));
-        gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), Ct, ldc, epi(-1, 1));
+        gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), Ct, ldc, epi(-1, 1), w.p, w.len);
         a = b;
     }
 }
@@ -230,7 +230,7 @@ static void apply_q_bz(int m, int n, int k, int i, int j, int mt, const double *
         gemm(vb, n, vb, opnd(Tt, ldt, NT, M_UPPER), opnd(W1, vb), W2, vb, epi(1, 0));
         GemmEpi e = epi(-1, 1);
         e.zero_rows = vb;
-        gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), X + a, ldq, e);
+        gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), X + a, ldq, e, w.p, w.len);
         b = a;
     }
 }
@@ -864,7 +864,7 @@ int dgeqr3(int m, int n, double *A, int lda, double *T, int ldt)
 int lila_query_dormqrf_w03(int m, int n, int k, int i, int j, int mt, double *A, int lda, double *T,
                            int ldt, double *work, int lwork)
 {
-    return clamp_query(need_apply(n, k, mt, true));
+    return clamp_query(need_apply(n, k, mt, true) + ozgemm_room(m - i, n, imin(mt, k)));
 }
 
 static int check_apply(int m, int n, int k, int i, int j, int mt, int lda, int ldt, long long lwork,
@@ -908,7 +908,7 @@ int lila_dormqrf_z03(int m, int n, int k, int i, int j, int mt, double *A, int l
 int lila_query_dormqrbz_w03(int m, int n, int k, int i, int j, int mt, double *A, int lda,
                             double *Q, int ldq, double *T, int ldt, double *work, int lwork)
 {
-    return clamp_query(need_apply(n, k, mt, true));
+    return clamp_query(need_apply(n, k, mt, true) + ozgemm_room(m - i, n, imin(mt, k)));
 }
 
 int lila_dormqrbz_w03(int m, int n, int k, int i, int j, int mt, double *A, int lda, double *Q,
@@ -1163,7 +1163,8 @@ int lila_query_dgeqrf_w03_recursive(int *lila_param, int m, int n, int i, int mt
                                     int lwork)
 {
     if (bad_lp(lila_param) || mt <= 0) return 0;
-    return clamp_query(need_recursive(lila_param, n, i, mt, true));
+    // the widest update of the recursion: n / 2 reflectors' tiles on the rest
+    return clamp_query(need_recursive(lila_param, n, i, mt, true) + ozgemm_room(m - i, n - n / 2, imin(mt, n / 2)));
 }
 int lila_query_dgeqrf_w03_levelx(int *lila_param, int n_lvl, int i_lvl, int *nb_lvl, int m, int n,
                                  int i, int mt, double *A, int lda, double *T, int ldt, double *Q,
@@ -1172,7 +1173,8 @@ int lila_query_dgeqrf_w03_levelx(int *lila_param, int n_lvl, int i_lvl, int *nb_
     if (bad_lp(lila_param) || mt <= 0 || !nb_lvl || n_lvl <= 0 || i_lvl < 0 || i_lvl >= n_lvl) return 0;
     for (int l = i_lvl; l < n_lvl; l++)
         if (nb_lvl[l] <= 0) return 0;
-    return clamp_query(need_levelx(lila_param, n_lvl, i_lvl, nb_lvl, n, i, mt, true));
+    return clamp_query(need_levelx(lila_param, n_lvl, i_lvl, nb_lvl, n, i, mt, true) +
+                       ozgemm_room(m - i, imin(nb_lvl[i_lvl], n), imin(mt, n)));
 }
 
 int lila_dgeqrf_w03_mt_l(int m, int n, int i, int mt, double *A, int lda, double *T, int ldt,

@@ -201,24 +201,26 @@ __device__ __forceinline__ void flush_acc(uint32_t tbase, int q, int h, long lon
 // bookkeeping carry over from one tile to the next in the persistent kernel.
 struct TileCtx {
     uint8_t *smem;
-    uint64_t *empty_b, *full_b, *tfree;
+    uint64_t *empty_b, *full_b, *tfree, *copy_b;
     int *s_rexp, *s_cexp;
     volatile int *s_abort;
     uint32_t tbase, sbase;
     int g;            // stages run by this CTA so far (buffer g & 1, mbarrier parity (g >> 1) & 1)
     int w;            // flush windows completed so far (tfree parity)
     int last_commit;  // global stage index of the issuer's last commit (-1: none)
+    int last_copy;    // and of thread 0's last bulk copy
 };
 
 __device__ __forceinline__ void ctx_open(TileCtx &x, uint8_t *smem, uint64_t *bars, uint32_t *tmem_base_s,
                                          int *s_rexp, int *s_cexp, int *s_abort)
 {
     const int tid = threadIdx.x, warp = tid >> 5;
-    // bars: empty[NSTAGE], full[NSTAGE], tfree
+    // bars: empty[NSTAGE], full[NSTAGE], tfree, copy[NSTAGE]
     if (tid == 0) {
         for (int b = 0; b < NSTAGE; b++) {
             tc::mbar_init(&bars[b], 1);
             tc::mbar_init(&bars[NSTAGE + b], OZT / 32);
+            tc::mbar_init(&bars[2 * NSTAGE + 1 + b], 1);
         }
         tc::mbar_init(&bars[2 * NSTAGE], OZT / 32);
         tc::fence_mbar_init();
@@ -235,6 +237,7 @@ __device__ __forceinline__ void ctx_open(TileCtx &x, uint8_t *smem, uint64_t *ba
     x.empty_b = bars;
     x.full_b = bars + NSTAGE;
     x.tfree = bars + 2 * NSTAGE;
+    x.copy_b = bars + 2 * NSTAGE + 1;
     x.s_rexp = s_rexp;
     x.s_cexp = s_cexp;
     x.s_abort = s_abort;
@@ -243,6 +246,7 @@ __device__ __forceinline__ void ctx_open(TileCtx &x, uint8_t *smem, uint64_t *ba
     x.g = 0;
     x.w = 0;
     x.last_commit = -1;
+    x.last_copy = -1;
 }
 
 __device__ __forceinline__ void ctx_close(TileCtx &x)
@@ -250,19 +254,33 @@ __device__ __forceinline__ void ctx_close(TileCtx &x)
     // normally every commit has been waited on by the flushes; after an
     // abort wait (bounded) for the issuer's last MMAs before freeing TMEM
     if (x.last_commit >= 0) tc::mbar_wait(&x.empty_b[x.last_commit & 1], (x.last_commit >> 1) & 1);
+    // and for the copies still writing shared memory
+    if (x.last_copy >= 0) tc::mbar_wait(&x.copy_b[x.last_copy & 1], (x.last_copy >> 1) & 1);
     tc::fence_before_sync();
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(x.tbase, 512);
 }
 
+// An operand split beforehand (k_pre_split): the digits of its 128 rows (64
+// columns) and 32 K values of one stage contiguous, in the stage's shared
+// memory layout, tile by tile; dig null: split by the tile itself.
+struct PreSplit {
+    const uint8_t *dig;
+    int stages;  // per tile
+};
+
 // One 128 x 64 output tile at (row0, col0) over K range [kbeg, kend); with
 // `part` set the FP64 partial product goes there (ld M) instead of C.
 // Returns false after a bounded wait gave up (the CTA must stop).
+// PRE: an operand with dig set comes as ready digits by bulk copies (its scales
+// in rexp / cexp).
+template <bool PRE>
 __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col0, int kbeg, int kend,
                                      const Operand &A, const Operand &B, double *C, int ldc, const GemmEpi &e,
                                      double *part, int *status, const int *rexp = nullptr,
-                                     const int *cexp = nullptr)
+                                     const int *cexp = nullptr, PreSplit preA = PreSplit{}, PreSplit preB = PreSplit{})
 {
+    const bool haveA = PRE && preA.dig, haveB = PRE && preB.dig;
     uint8_t *smem = x.smem;
     int *s_rexp = x.s_rexp, *s_cexp = x.s_cexp;
     volatile int *s_abort = x.s_abort;
@@ -320,7 +338,9 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
             return;
         }
         const int ka = k1 + ak * 8, kb = k1 + bk * 8 + 4 * bh;
-        if (k1 >= pa.lo && k1 + KC <= pa.hi) {
+        if (haveA) {
+            // copied
+        } else if (k1 >= pa.lo && k1 + KC <= pa.hi) {
             const unsigned long long *q = (const unsigned long long *)A.p;
             if (A.trans == NT) {
                 q += (size_t)(row0 + ar) + (size_t)ka * A.ld;
@@ -344,7 +364,9 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
 #pragma unroll
             for (int j = 0; j < 8; j++) ra[j] = opa(A, M, row0 + ar, ka + j, kend);
         }
-        if (k1 >= pb.lo && k1 + KC <= pb.hi) {
+        if (haveB) {
+            // copied
+        } else if (k1 >= pb.lo && k1 + KC <= pb.hi) {
             const unsigned long long *q = (const unsigned long long *)B.p;
             if (B.trans == NT) {
                 q += (size_t)kb + (size_t)(col0 + bc) * B.ld;
@@ -442,8 +464,18 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
         if (G >= NSTAGE && !tc::wait_abort_warp(&x.empty_b[buf], ((G - NSTAGE) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) break;
         uint8_t *stA = smem + (size_t)buf * STAGE_BYTES;
         uint8_t *stB = stA + A_BYTES;
+        if (PRE && (haveA || haveB) && tid == 0) {
+            tc::mbar_arrive_expect_tx(&x.copy_b[buf], (haveA ? A_BYTES : 0) + (haveB ? B_BYTES : 0));
+            const size_t st = (size_t)(kbeg / KC + ch);
+            const uint32_t at = sbase + buf * STAGE_BYTES;
+            if (haveA) tc::bulk_load(at, preA.dig + ((size_t)(row0 / BM) * preA.stages + st) * A_BYTES, A_BYTES, &x.copy_b[buf]);
+            if (haveB)
+                tc::bulk_load(at + A_BYTES, preB.dig + ((size_t)(col0 / BN) * preB.stages + st) * B_BYTES, B_BYTES,
+                              &x.copy_b[buf]);
+            x.last_copy = G;
+        }
         // A: 128 rows x 4 groups of 8 K values = 512 units, one per thread
-        {
+        if (!haveA) {
             const int emax = s_rexp[ar];
 #pragma unroll
             for (int hf = 0; hf < 2; hf++) {
@@ -453,7 +485,7 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
             }
         }
         // B: 64 columns x 4 groups x 2 halves = 512 half units, one per thread
-        {
+        if (!haveB) {
             uint32_t w01[NS], w23[NS];
             digits4(rb, s_cexp[bc], w01, w23);
             store_half(stB, B_SLICE, bc, bk, bh, w01, w23);
@@ -465,6 +497,7 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
         const bool window_start = (ch % FLUSH) == 0;
         if (issuer) {
             bool ok = tc::wait_abort(&x.full_b[buf], (G >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
+            if (ok && (haveA || haveB)) ok = tc::wait_abort(&x.copy_b[buf], (G >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
             if (ok && window_start && x.w > 0) ok = tc::wait_abort(x.tfree, (x.w - 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
             if (ok) {
                 tc::fence_after_sync();
@@ -552,7 +585,7 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
 
 #define OZG_SHARED                                          \
     extern __shared__ __align__(1024) uint8_t smem[];      \
-    __shared__ __align__(8) uint64_t bars[2 * NSTAGE + 1]; \
+    __shared__ __align__(8) uint64_t bars[3 * NSTAGE + 1]; \
     __shared__ uint32_t tmem_base_s;                       \
     __shared__ int s_rexp[BM], s_cexp[BN];                 \
     __shared__ int s_abort;                                \
@@ -565,9 +598,98 @@ __global__ void __launch_bounds__(OZT, 1)
 {
     OZG_SHARED;
     const int kbeg = blockIdx.z * kchunk;
-    tile(x, M, N, blockIdx.x * BM, blockIdx.y * BN, kbeg, min(K, kbeg + kchunk), A, B, C, ldc, e,
-         part ? part + (size_t)blockIdx.z * M * N : nullptr, status);
+    tile<false>(x, M, N, blockIdx.x * BM, blockIdx.y * BN, kbeg, min(K, kbeg + kchunk), A, B, C, ldc, e,
+                part ? part + (size_t)blockIdx.z * M * N : nullptr, status);
     ctx_close(x);
+}
+
+// The same with operands split beforehand; rexp / cexp: the split operands'
+// scales, M / N per K slice.
+__global__ void __launch_bounds__(OZT, 1)
+    k_ozgemm_pre(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e, double *part,
+                 int *status, PreSplit preA, PreSplit preB, const int *rexp, const int *cexp)
+{
+    OZG_SHARED;
+    const int kbeg = blockIdx.z * kchunk;
+    tile<true>(x, M, N, blockIdx.x * BM, blockIdx.y * BN, kbeg, min(K, kbeg + kchunk), A, B, C, ldc, e,
+               part ? part + (size_t)blockIdx.z * M * N : nullptr, status,
+               preA.dig ? rexp + (size_t)blockIdx.z * M : nullptr, preB.dig ? cexp + (size_t)blockIdx.z * N : nullptr,
+               preA, preB);
+    ctx_close(x);
+}
+
+// ---- splitting an operand beforehand ---------------------------------------
+// A tile of the output splits its 128 rows of op(A) and 64 columns of op(B)
+// itself, so op(A)'s digits are made once per 64 columns of C and op(B)'s once
+// per 128 rows.  Where that is often, they are made once here and copied: two
+// launches per product (scales, digits) for both operands.
+struct PreJob {
+    Operand X;
+    int rows, isA, tile;  // rows of op(A) or columns of op(B); their tile
+    int *exps;            // rows per K slice, zeroed
+    uint8_t *dig;
+};
+struct PreJobs {
+    PreJob j[2];
+    int K, kchunk;
+};
+
+__device__ __forceinline__ unsigned long long pre_bits(const PreJob &J, int x, int k, int kend)
+{
+    return J.isA ? opa(J.X, J.rows, x, k, kend) : opb(J.X, J.rows, k, x, kend);
+}
+// whether the operand is contiguous along its rows (op(A)) or columns (op(B))
+__device__ __forceinline__ bool along_x(const PreJob &J) { return J.isA ? J.X.trans == NT : J.X.trans == TR; }
+
+constexpr int PRE_KP = 64;   // K values per CTA of the scale pass
+
+__global__ void __launch_bounds__(256) k_pre_scales(PreJobs P)
+{
+    const PreJob J = P.j[blockIdx.z];
+    const int ppc = (P.kchunk + PRE_KP - 1) / PRE_KP, z = blockIdx.y / ppc;
+    const int k0 = z * P.kchunk + (blockIdx.y % ppc) * PRE_KP;
+    const int k1 = min(min(k0 + PRE_KP, (z + 1) * P.kchunk), P.K), x0 = blockIdx.x * 64;
+    if (!J.dig || x0 >= J.rows || k0 >= k1) return;
+    int *out = J.exps + (size_t)z * J.rows;
+    if (along_x(J)) {
+        const int x = x0 + (threadIdx.x & 63);
+        int mx = 0;
+#pragma unroll 4
+        for (int k = k0 + (threadIdx.x >> 6); k < k1; k += 4) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
+        if (x < J.rows && mx) atomicMax(&out[x], mx);
+    } else {
+        for (int x = x0 + (threadIdx.x >> 5); x < min(x0 + 64, J.rows); x += 8) {
+            int mx = 0;
+#pragma unroll 4
+            for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            if ((threadIdx.x & 31) == 0 && mx) atomicMax(&out[x], mx);
+        }
+    }
+}
+
+// 64 rows x 32 K values per CTA (256 units of 8 values, one per thread).
+__global__ void __launch_bounds__(256) k_pre_split(PreJobs P)
+{
+    const PreJob J = P.j[blockIdx.z];
+    const int st = blockIdx.y, k0 = st * KC, z = k0 / P.kchunk, x0 = blockIdx.x * 64;
+    const int pad = (J.rows + J.tile - 1) / J.tile * J.tile;
+    if (!J.dig || x0 >= pad || k0 >= P.K) return;
+    const int kend = min(P.K, (z + 1) * P.kchunk);
+    const int kg = along_x(J) ? threadIdx.x >> 6 : threadIdx.x & 3, xi = along_x(J) ? threadIdx.x & 63 : threadIdx.x >> 2;
+    const int x = x0 + xi, emax = x < J.rows ? J.exps[(size_t)z * J.rows + x] : 0;
+    unsigned long long v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = pre_bits(J, x, k0 + kg * 8 + i, kend);
+    uint32_t a01[NS], a23[NS], b01[NS], b23[NS];
+    digits4(v, emax, a01, a23);
+    digits4(v + 4, emax, b01, b23);
+    const uint32_t slice = J.isA ? A_SLICE : B_SLICE, bytes = J.isA ? A_BYTES : B_BYTES;
+    const int idx = x % J.tile;
+    uint8_t *base = J.dig + ((size_t)(x / J.tile) * ((P.K + KC - 1) / KC) + st) * bytes + (idx >> 3) * SBO + kg * LBO +
+                    (idx & 7) * 16;
+#pragma unroll
+    for (int s = 0; s < NS; s++) *(uint4 *)(base + s * slice) = make_uint4(a01[s], a23[s], b01[s], b23[s]);
 }
 
 // Grouped form: CTA b runs tile b - prefix[g] of group g, prefix[g] <= b <
@@ -595,7 +717,7 @@ __global__ void __launch_bounds__(OZT, 1) k_ozgemm_groups(const OzGroup *groups,
         const OzGroup g = groups[cur.x];
         const int t = cur.y;
         const int tiles_m = (g.M + BM - 1) / BM;
-        if (!tile(x, g.M, g.N, (t % tiles_m) * BM, (t / tiles_m) * BN, 0, g.K, g.A, g.B, g.C, g.ldc, g.e, nullptr,
+        if (!tile<false>(x, g.M, g.N, (t % tiles_m) * BM, (t / tiles_m) * BN, 0, g.K, g.A, g.B, g.C, g.ldc, g.e, nullptr,
                   status, g.rexp, g.cexp))
             break;
         cur = nxt;
@@ -607,25 +729,68 @@ __global__ void __launch_bounds__(OZT, 1) k_ozgemm_groups(const OzGroup *groups,
 
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// One CTA holds an SM (192 KB of shared memory, all of tensor memory), so the
+// K split that minimises waves per slice wins: s with ceil(tiles s / SMs) / s
+// least, a slice of at least 256 K, and a per-slice charge for the partials.
+// 128 x 1024 x 6000: 202 us on 160 CTAs (10 slices, two waves), 139 on 144 (9).
 int ozgemm_splits(int M, int N, int K, long long part_len)
 {
     if (M <= 0 || N <= 0 || K <= 256) return 1;
     const long long tiles = (long long)cdiv(M, ozg::BM) * cdiv(N, ozg::BN);
     const int sms = sm_count();
-    if (tiles >= sms) return 1;
-    int s = cdiv(K, 256);
-    const int want = cdiv(sms, tiles);
-    if (s > want) s = want;
+    int most = cdiv(K, 256);
     const long long fit = part_len / ((long long)M * N);
-    if (s > fit) s = (int)fit;
-    return s < 2 ? 1 : s;
+    if (most > fit) most = (int)fit;
+    if (most > 64) most = 64;
+    int best = 1;
+    double best_t = cdiv(tiles, sms);
+    for (int s = 2; s <= most; s++) {
+        const double t = (double)cdiv(tiles * s, sms) / s + 0.01 * s * tiles / sms;
+        if (t < best_t) {
+            best_t = t;
+            best = s;
+        }
+    }
+    return best;
 }
+
+constexpr double kPreMin = 134217728.0;  // multiply-adds from which operands are split beforehand
+constexpr int kReuse = 4;
 
 void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e, double *part,
             long long part_len, const char *tag)
 {
     if (M <= 0 || N <= 0) return;
     cudaStream_t st = stream();
+    // split an operand beforehand where the output's tiles use it at least
+    // kReuse times and `part` has room for its digits (at the end; the K
+    // slices' partials get the rest)
+    ozg::PreJobs P{};
+    P.j[0] = ozg::PreJob{A, M, 1, ozg::BM, nullptr, nullptr};
+    P.j[1] = ozg::PreJob{B, N, 0, ozg::BN, nullptr, nullptr};
+    dim3 grid(cdiv(M, ozg::BM), cdiv(N, ozg::BN), 1);
+    int *exps = nullptr;
+    size_t nexp = 0;
+    if (part && (double)M * N * K >= kPreMin) {
+        const size_t stages = cdiv(K, ozg::KC);
+        uintptr_t end = (uintptr_t)(part + part_len) & ~(uintptr_t)127;
+        auto take = [&](size_t bytes) -> void * {
+            bytes = (bytes + 127) / 128 * 128;
+            if (end < (uintptr_t)part + bytes) return nullptr;
+            end -= bytes;
+            return (void *)end;
+        };
+        const bool wantA = (int)grid.y >= kReuse, wantB = (int)grid.x >= kReuse;
+        // scales for as many slices as there may be
+        const size_t most = cdiv(K, 256) < 64 ? cdiv(K, 256) : 64;
+        nexp = most * ((wantA ? M : 0) + (size_t)(wantB ? N : 0));
+        exps = (int *)take(nexp * sizeof(int));
+        if (exps && wantA) P.j[0].dig = (uint8_t *)take((size_t)grid.x * stages * ozg::A_BYTES);
+        if (exps && wantB) P.j[1].dig = (uint8_t *)take((size_t)grid.y * stages * ozg::B_BYTES);
+        P.j[0].exps = exps;
+        P.j[1].exps = exps + (wantA ? most * M : 0);
+        if (P.j[0].dig || P.j[1].dig) part_len = ((const double *)end - part);
+    }
     int splits = part ? ozgemm_splits(M, N, K, part_len) : 1;
     int kchunk = K > 0 ? K : 1;
     if (splits > 1) {
@@ -633,12 +798,41 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
         splits = cdiv(K, kchunk);
     }
     double *p = splits > 1 ? part : nullptr;
-    cudaFuncSetAttribute(ozg::k_ozgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
-    dim3 grid(cdiv(M, ozg::BM), cdiv(N, ozg::BN), splits);
-    trace_begin();
-    ozg::k_ozgemm<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr());
+    grid.z = splits;
+    P.K = K;
+    P.kchunk = kchunk;
+    if (P.j[0].dig || P.j[1].dig) {
+        trace_break();
+        cudaMemsetAsync(exps, 0, nexp * sizeof(int), st);
+        const int xb = cdiv(P.j[0].dig && (!P.j[1].dig || M > N) ? cdiv(M, ozg::BM) * ozg::BM : cdiv(N, ozg::BN) * ozg::BN, 64);
+        trace_begin();
+        ozg::k_pre_scales<<<dim3(xb, splits * cdiv(kchunk, ozg::PRE_KP), 2), 256, 0, st>>>(P);
+        note_launch("ozgemm_pre_scales");
+        trace_begin();
+        ozg::k_pre_split<<<dim3(xb, cdiv(K, ozg::KC), 2), 256, 0, st>>>(P);
+        note_launch("ozgemm_pre_split");
+        const ozg::PreSplit sA{P.j[0].dig, cdiv(K, ozg::KC)}, sB{P.j[1].dig, cdiv(K, ozg::KC)};
+        cudaFuncSetAttribute(ozg::k_ozgemm_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
+        trace_begin();
+        ozg::k_ozgemm_pre<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr(), sA, sB,
+                                                            P.j[0].exps, P.j[1].exps);
+    } else {
+        cudaFuncSetAttribute(ozg::k_ozgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
+        trace_begin();
+        ozg::k_ozgemm<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr());
+    }
     note_launch(tag);
     if (splits > 1) splitk_reduce(M, N, splits, part, C, ldc, e);
+}
+
+// Doubles of `part` that the operands split beforehand may take in the two
+// tall products of a block reflector of vb columns applied to an m x n block.
+long long ozgemm_room(long long m, long long n, long long vb)
+{
+    if ((double)m * n * vb < kPreMin) return 0;
+    const long long v = (vb + 127) / 128 * 128 + 32;
+    const long long room = 2 * v * (m + n + 256) + m + n + 256;
+    return room <= (1LL << 27) ? room : 0;
 }
 
 int ozgemm_group_tiles(int M, int N) { return M > 0 && N > 0 ? cdiv(M, ozg::BM) * cdiv(N, ozg::BN) : 0; }

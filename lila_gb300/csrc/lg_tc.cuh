@@ -205,6 +205,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int 
         : "memory");
 }
 
+// Untiled bulk copy of `bytes` (a multiple of 16, both addresses 16-byte
+// aligned) from global into shared memory; completes on mbar.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint64_t *mbar)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+        "l"((unsigned long long)(uintptr_t)src), "r"(bytes), "r"(smem_u32(mbar))
+        : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tmap(const void *tmap)
 {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)(uintptr_t)tmap) : "memory");
