@@ -267,14 +267,25 @@ int gemm_splits(int M, int N, int K, long long part_len)
     return gemm_plan(M, N, K, part_len, false).splits;
 }
 
+// Whether a product goes to the tensor cores in split precision: its time there
+// (38 us of latency, then 0.175 us per million multiply-adds of the padded 128 x
+// 64 x 32 tiles) against the FP64 pipe's (10 us, 1.65 us per million).  128 x 64
+// x 3000: FP64 54 us, split 44; 3000 x 128 x 64: 50 and 35; 128 x 256 x 512: 38
+// and 44; 128 x 3000 x 6000: 3,795 and 403.  Thin tiles count at their padded
+// size: 34 reflectors on 6000 x 3000 take the FP64 pipe 970 us.
+static bool split_pays(int M, int N, int K)
+{
+    if (precision() != 1 || M < 16 || N < 16 || K < 16) return false;
+    const double fma = 1e-6 * M * N * K;
+    const double pad = 1e-6 * (128.0 * ceil_div(M, 128)) * (64.0 * ceil_div(N, 64)) * (32.0 * ceil_div(K, 32));
+    return 38.0 + 0.175 * pad < 10.0 + 1.65 * fma;
+}
+
 void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e,
           double *part, long long part_len, const char *tag)
 {
     if (M <= 0 || N <= 0) return;
-    // large products go to the tensor cores in split-precision mode: from 2^25
-    // multiply-adds, where both take the same time (128 x 128 x 3000: FP64 95 us,
-    // split 72; 3000 x 64 x 128: 48 and 47; 128 x 64 x 3000: 54 and 70)
-    if (precision() == 1 && M >= 64 && N >= 64 && K >= 64 && (double)M * N * K >= 33554432.0) {
+    if (split_pays(M, N, K)) {
         ozgemm(M, N, K, A, B, C, ldc, e, part, part_len, "ozgemm");
         return;
     }

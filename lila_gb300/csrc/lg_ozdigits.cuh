@@ -108,14 +108,13 @@ __device__ __forceinline__ double assemble_fast(long long hi, long long lo, int 
     return __longlong_as_double(b + ((long long)(sc + 9) << 52));
 }
 
-// The same value as assemble_fast, bit for bit, with the int64 -> double
+// The same value as assemble_fast (J its 63-bit sum), bit for bit, with the int64 -> double
 // rounding done by integer instructions (no FP64-pipe conversion): |J| is
 // normalised by its leading-zero count, rounded to 53 bits (nearest, ties to
 // even) and placed in the exponent and fraction fields; a carry out of the
 // rounding moves into the exponent field by itself.
-__device__ __forceinline__ double assemble_int(long long hi, long long lo, int sc)
+__device__ __forceinline__ double assemble_j(long long J, int sc)
 {
-    const long long J = hi * (1LL << 19) + (lo >> 9);
     if (J == 0) return 0.0;
     const unsigned long long sign = (unsigned long long)J & 0x8000000000000000ull;
     unsigned long long a = J < 0 ? 0ull - (unsigned long long)J : (unsigned long long)J;
@@ -132,6 +131,11 @@ __device__ __forceinline__ double assemble_int(long long hi, long long lo, int s
     // (be - 1) << 52 plus mant (whose bit 52 is the implicit one) is the
     // exponent and fraction field; a carry (mant = 2^53) lands in the exponent
     return __longlong_as_double((long long)(sign | ((((unsigned long long)(long long)(be - 1)) << 52) + mant)));
+}
+
+__device__ __forceinline__ double assemble_int(long long hi, long long lo, int sc)
+{
+    return assemble_j(hi * (1LL << 19) + (lo >> 9), sc);
 }
 
 // (hi * 2^28 + lo) * 2^sc rounded to nearest even double; integer-only.

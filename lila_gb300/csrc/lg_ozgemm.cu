@@ -121,13 +121,14 @@ __device__ __forceinline__ void digits4(const unsigned long long *v, int emax, u
 // narrow, so per-output FP64 compares and products are avoided.
 struct EpiMode {
     int amode;     // 1: alpha = 1, 2: alpha = -1 (a sign flip), 0: general
-    bool use_beta;
+    bool use_beta, beta_one;
 };
 __device__ __forceinline__ EpiMode epi_mode(const GemmEpi &e)
 {
     EpiMode m;
     m.amode = e.alpha == 1.0 ? 1 : (e.alpha == -1.0 ? 2 : 0);
     m.use_beta = e.beta != 0.0;
+    m.beta_one = e.beta == 1.0;
     return m;
 }
 
@@ -195,6 +196,106 @@ __device__ __forceinline__ void flush_acc(uint32_t tbase, int q, int h, long lon
                     acc_lo[8 * hc + j] += x;
             }
         }
+}
+
+// The digit products of one stage (32 K) at shared address `at`: order d = s +
+// t of slices s of A and t of B into TMEM block d; `fresh` overwrites.
+__device__ __forceinline__ void issue_stage(uint32_t tbase, uint32_t at, bool fresh)
+{
+    const uint64_t da = tc::desc_nosw(at, LBO, SBO);
+    const uint64_t db = tc::desc_nosw(at + A_BYTES, LBO, SBO);
+#pragma unroll
+    for (int ks = 0; ks < KC / 16; ks++) {
+        const uint64_t koff = (uint64_t)(ks * 2 * LBO) >> 4;
+#pragma unroll
+        for (int sl = 0; sl < NS; sl++) {
+            const int ntot = 64 * (NS - sl);
+            const uint64_t ad = da + koff + ((uint64_t)(sl * A_SLICE) >> 4);
+            const uint32_t acc = (fresh && ks == 0 && sl == 0) ? 0u : 1u;
+            const int n1 = ntot < 256 ? ntot : 256;
+            tc::mma_bf16(tbase + 64 * sl, ad, db + koff, tc::idesc_bf16_f32(128, n1), acc);
+            if (ntot > 256)
+                tc::mma_bf16(tbase + 64 * sl + 256, ad, db + koff + ((uint64_t)(32 * SBO) >> 4),
+                             tc::idesc_bf16_f32(128, ntot - 256), acc);
+        }
+    }
+}
+
+// This thread's 16 outputs (row gr, columns gc0 ..) from their int64 sums; er
+// and cexp(j) are the scales.  Up to 256 K values (two flush windows) |hi| stays
+// below 2^43, where the short integer assembly keeps every bit down to 2^-54 of
+// the group scale.  Eight outputs at a time, C's values (beta) loaded together
+// before the first is used.  status: flags non-finite column scales (null: the
+// caller has).
+//
+// MODE keeps the FP64 pipe out of what does not need it (an FP64 instruction
+// whose predicate is off still holds it: with alpha, add_diag and beta tested per
+// output the tile spent six per output): 0 plus or minus the product, 1 C plus or
+// minus the product (one addition), 2 everything else.
+// val(j, sc): output j's sum times 2^sc; `loaded`: cval holds C's values already.
+template <int MODE, typename V, typename F>
+__device__ __forceinline__ void store_outputs_mode(V &&val, int gr, int gc0, int M, int N, int er, const GemmEpi &e,
+                                                   const EpiMode &md, double *C, int ldc, double *part, F &&cexp,
+                                                   int *status, bool loaded, const double (&cval)[16])
+{
+    const long long flip = md.amode == 2 ? (long long)0x8000000000000000ull : 0ll;
+    const bool use = MODE != 0 && !part && md.use_beta && gr >= e.zero_rows;
+#pragma unroll
+    for (int jb = 0; jb < 16; jb += 8) {
+        double cv[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int gc = gc0 + jb + j;
+            cv[j] = cval[jb + j];
+            if (!loaded && use && gc < N && !(e.upper_only && gr > gc)) cv[j] = C[(size_t)gr + (size_t)gc * ldc];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int gc = gc0 + jb + j;
+            if (gc >= N) continue;
+            const int ec = cexp(jb + j);
+            if (status && ec == 0x7FF) atomicOr(status, ST_NONFINITE);
+            double v;
+            if (er == 0x7FF || ec == 0x7FF)
+                v = __longlong_as_double(0x7FF8000000000000ll);
+            else if (!(er && ec))
+                v = 0.0;
+            else
+                v = val(jb + j, (er - 1022) + (ec - 1022) - 63);
+            if (MODE == 2) {
+                if (part)
+                    part[(size_t)gr + (size_t)gc * M] = v;
+                else
+                    epi_store(v, gr, gc, C, ldc, e, md, use, cv[j]);
+                continue;
+            }
+            if (MODE == 0 && part) {
+                part[(size_t)gr + (size_t)gc * M] = v;
+                continue;
+            }
+            if (e.upper_only && gr > gc) continue;
+            v = __longlong_as_double(__double_as_longlong(v) ^ flip);
+            if (MODE == 1) {
+                const double sum = cv[j] + v;
+                v = use ? sum : v;  // rows whose C is not read keep the sign of a zero product
+            }
+            C[(size_t)gr + (size_t)gc * ldc] = v;
+        }
+    }
+}
+
+template <typename V, typename F>
+__device__ __forceinline__ void store_outputs(V &&val, int gr, int gc0, int M, int N, int er, const GemmEpi &e,
+                                              const EpiMode &md, double *C, int ldc, double *part, F &&cexp, int *status,
+                                              bool loaded, const double (&cval)[16])
+{
+    if (gr >= M) return;
+    if (part || (md.amode && !e.add_diag && !md.use_beta))
+        store_outputs_mode<0>(val, gr, gc0, M, N, er, e, md, C, ldc, part, cexp, status, loaded, cval);
+    else if (md.amode && !e.add_diag && md.beta_one)
+        store_outputs_mode<1>(val, gr, gc0, M, N, er, e, md, C, ldc, part, cexp, status, loaded, cval);
+    else
+        store_outputs_mode<2>(val, gr, gc0, M, N, er, e, md, C, ldc, part, cexp, status, loaded, cval);
 }
 
 // Per-CTA state of the tile loop: TMEM, the stage mbarriers and their phase
@@ -501,23 +602,7 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
             if (ok && window_start && x.w > 0) ok = tc::wait_abort(x.tfree, (x.w - 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
             if (ok) {
                 tc::fence_after_sync();
-                const uint64_t da = tc::desc_nosw(sbase + buf * STAGE_BYTES, LBO, SBO);
-                const uint64_t db = tc::desc_nosw(sbase + buf * STAGE_BYTES + A_BYTES, LBO, SBO);
-#pragma unroll
-                for (int ks = 0; ks < KC / 16; ks++) {
-                    const uint64_t koff = (uint64_t)(ks * 2 * LBO) >> 4;
-#pragma unroll
-                    for (int sl = 0; sl < NS; sl++) {
-                        const int ntot = 64 * (NS - sl);
-                        const uint64_t ad = da + koff + ((uint64_t)(sl * A_SLICE) >> 4);
-                        const uint32_t acc = (window_start && ks == 0 && sl == 0) ? 0u : 1u;
-                        const int n1 = ntot < 256 ? ntot : 256;
-                        tc::mma_bf16(tbase + 64 * sl, ad, db + koff, tc::idesc_bf16_f32(128, n1), acc);
-                        if (ntot > 256)
-                            tc::mma_bf16(tbase + 64 * sl + 256, ad, db + koff + ((uint64_t)(32 * SBO) >> 4),
-                                         tc::idesc_bf16_f32(128, ntot - 256), acc);
-                    }
-                }
+                issue_stage(tbase, sbase + buf * STAGE_BYTES, window_start);
                 tc::mma_commit(&x.empty_b[buf]);
                 x.last_commit = G;
             }
@@ -540,43 +625,13 @@ __device__ __forceinline__ bool tile(TileCtx &x, int M, int N, int row0, int col
     // Up to 256 K values (two flush windows) |hi| stays below 2^43, where the
     // integer-only assembly keeps every bit down to 2^-54 of the group scale.
     if (!*s_abort) {
+        const int r = 32 * q + lane;
         const bool fast = kend - kbeg <= 256;
-        const EpiMode md = epi_mode(e);
-        const int r = 32 * q + lane, gr = row0 + r;
-        const int er = s_rexp[r];
-        if (gr < M) {
-            // eight outputs at a time, C's values (beta) loaded together before
-            // the first is used
-#pragma unroll
-            for (int jb = 0; jb < 16; jb += 8) {
-                double cv[8];
-                const bool use = !part && md.use_beta && gr >= e.zero_rows;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int gc = col0 + 16 * h + jb + j;
-                    if (use && gc < N && !(e.upper_only && gr > gc)) cv[j] = C[(size_t)gr + (size_t)gc * ldc];
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int c = 16 * h + jb + j, gc = col0 + c;
-                    if (gc >= N) continue;
-                    const int ec = s_cexp[c];
-                    double v;
-                    if (er == 0x7FF || ec == 0x7FF)
-                        v = __longlong_as_double(0x7FF8000000000000ll);
-                    else if (!(er && ec))
-                        v = 0.0;
-                    else if (fast)
-                        v = oz::assemble_fast(acc_hi[jb + j], acc_lo[jb + j], (er - 1022) + (ec - 1022) - 63);
-                    else
-                        v = oz::assemble(acc_hi[jb + j], acc_lo[jb + j], (er - 1022) + (ec - 1022) - 63);
-                    if (part)
-                        part[(size_t)gr + (size_t)gc * M] = v;
-                    else
-                        epi_store(v, gr, gc, C, ldc, e, md, use, cv[j]);
-                }
-            }
-        }
+        const double none[16] = {};
+        store_outputs([&](int j, int sc) {
+            return fast ? oz::assemble_int(acc_hi[j], acc_lo[j], sc) : oz::assemble(acc_hi[j], acc_lo[j], sc);
+        }, row0 + r, col0 + 16 * h, M, N, s_rexp[r], e, epi_mode(e), C, ldc, part,
+                      [&](int j) { return s_cexp[16 * h + j]; }, nullptr, false, none);
     }
     // the next tile's first MMA waits on tfree, so TMEM needs no barrier
     // here; the next tile's first barrier orders the exponent reads above
@@ -616,6 +671,165 @@ __global__ void __launch_bounds__(OZT, 1)
                preA.dig ? rexp + (size_t)blockIdx.z * M : nullptr, preB.dig ? cexp + (size_t)blockIdx.z * N : nullptr,
                preA, preB);
     ctx_close(x);
+}
+
+// Both operands split beforehand, no K slices: nothing is left for the tile's
+// warps but its outputs, so a persistent CTA gives copies and MMAs to one thread
+// of a 17th warp and the other 16 warps only fold tensor memory and assemble.
+// The MMAs of a tile start as soon as the previous tile's sums are in registers:
+// its 8,192 outputs (an int64 -> FP64 conversion and a beta FMA each, ~10,000
+// clocks of the FP64 pipe) are assembled while the next 128 K are multiplied
+// (~12,000 clocks).  16384 x 8192 x 128: 2,674 us with a CTA per tile, which does
+// one after the other, 1,152 this way.
+// ONE: K <= 128, a single window per tile: its sums go straight into one 64-bit
+// integer per output, which leaves registers for C's values, loaded while the
+// tile's MMAs run (4096 x 4864 x 128: 212 -> 185 us).
+template <bool ONE>
+__global__ void __launch_bounds__(OZT + 32, 1)
+    k_ozgemm_pp(int M, int N, int K, double *C, int ldc, GemmEpi e, int *status, PreSplit preA, PreSplit preB,
+                const int *rexp, const int *cexp, int tiles_m, int total)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t copy_b[NSTAGE], empty_b[NSTAGE], acc_b, tfree;
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int s_abort_w;
+    volatile int *s_abort = &s_abort_w;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int b = 0; b < NSTAGE; b++) {
+            tc::mbar_init(&copy_b[b], 1);
+            tc::mbar_init(&empty_b[b], 1);
+        }
+        tc::mbar_init(&acc_b, 1);
+        tc::mbar_init(&tfree, OZT / 32);
+        tc::fence_mbar_init();
+        s_abort_w = 0;
+    }
+    if (warp == 0) {
+        tc::tmem_alloc(&tmem_base_s, 512);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tbase = tmem_base_s, sbase = tc::smem_u32(smem);
+    const int nst = (K + KC - 1) / KC, nwin = (nst + FLUSH - 1) / FLUSH;
+
+    if (warp == OZT / 32) {
+        if (lane == 0) {
+            int made = 0, mt = blockIdx.x, ms = 0;  // stages copied; the next one's tile and stage
+            auto make = [&] {
+                if (mt >= total) return true;
+                const int buf = made & 1;
+                if (made >= NSTAGE && !tc::wait_abort(&empty_b[buf], ((made - NSTAGE) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT))
+                    return false;
+                tc::mbar_arrive_expect_tx(&copy_b[buf], STAGE_BYTES);
+                const uint32_t at = sbase + buf * STAGE_BYTES;
+                tc::bulk_load(at, preA.dig + ((size_t)(mt % tiles_m) * preA.stages + ms) * A_BYTES, A_BYTES, &copy_b[buf]);
+                tc::bulk_load(at + A_BYTES, preB.dig + ((size_t)(mt / tiles_m) * preB.stages + ms) * B_BYTES, B_BYTES,
+                              &copy_b[buf]);
+                made++;
+                if (++ms == nst) {
+                    ms = 0;
+                    mt += gridDim.x;
+                }
+                return true;
+            };
+            int g = 0, w = 0;
+            bool ok = make() && make();
+            for (int t = blockIdx.x; ok && t < total; t += gridDim.x)
+                for (int st = 0; ok && st < nst; st++, g++) {
+                    const int buf = g & 1;
+                    const bool start = st % FLUSH == 0, end = st % FLUSH == FLUSH - 1 || st == nst - 1;
+                    ok = tc::wait_abort(&copy_b[buf], (g >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
+                    if (ok && start && w > 0) ok = tc::wait_abort(&tfree, (w - 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
+                    if (!ok) break;
+                    tc::fence_after_sync();
+                    issue_stage(tbase, sbase + buf * STAGE_BYTES, start);
+                    tc::mma_commit(&empty_b[buf]);
+                    if (end) {
+                        tc::mma_commit(&acc_b);
+                        w++;
+                    }
+                    // refill the other buffer once its MMAs are done
+                    if (g >= 1) ok = make();
+                }
+            // a give-up leaves copies and MMAs in flight: wait (bounded) for them
+            if (!ok) {
+                if (made > 0) tc::mbar_wait(&copy_b[(made - 1) & 1], ((made - 1) >> 1) & 1);
+                if (made > 1) tc::mbar_wait(&copy_b[(made - 2) & 1], ((made - 2) >> 1) & 1);
+                if (g > 0) tc::mbar_wait(&empty_b[(g - 1) & 1], ((g - 1) >> 1) & 1);
+            }
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, h = warp >> 2;
+        const EpiMode md = epi_mode(e);
+        int w = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x) {
+            const int row0 = (t % tiles_m) * BM, col0 = (t / tiles_m) * BN;
+            const int gr = row0 + 32 * q + lane, er = gr < M ? rexp[gr] : 0;
+            const int gc0 = col0 + 16 * h;
+            auto scale = [&](int j) { return gc0 + j < N ? cexp[gc0 + j] : 0; };
+            if (er == 0x7FF) atomicOr(status, ST_NONFINITE);
+            double cv[16] = {};
+            if constexpr (ONE) {
+                const bool use = md.use_beta && gr < M && gr >= e.zero_rows;
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (use && gc0 + j < N && !(e.upper_only && gr > gc0 + j)) cv[j] = C[(size_t)gr + (size_t)(gc0 + j) * ldc];
+                if (!tc::wait_abort_warp(&acc_b, w++ & 1, s_abort, status, ST_WAIT_TIMEOUT)) break;
+                tc::fence_after_sync();
+                long long J[16];
+#pragma unroll
+                for (int hc = 0; hc < 2; hc++) {
+                    long long half[2][8];
+#pragma unroll
+                    for (int g4 = 0; g4 < 2; g4++) {
+                        uint32_t v[4][8];
+#pragma unroll
+                        for (int u = 0; u < 4; u++)
+                            tc::tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * (4 * g4 + u) + 16 * h + 8 * hc), v[u]);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; j++) half[g4][j] = oz::combine4(v[0][j], v[1][j], v[2][j], v[3][j]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; j++) J[8 * hc + j] = half[0][j] * (1LL << 19) + (half[1][j] >> 9);
+                }
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&tfree);
+                store_outputs([&](int j, int sc) { return oz::assemble_j(J[j], sc); }, gr, gc0, M, N, er, e, md, C, ldc,
+                              nullptr, scale, status, true, cv);
+            } else {
+                long long acc_hi[16], acc_lo[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    acc_hi[j] = 0;
+                    acc_lo[j] = 0;
+                }
+                bool ok = true;
+                for (int k = 0; k < nwin; k++, w++) {
+                    ok = tc::wait_abort_warp(&acc_b, w & 1, s_abort, status, ST_WAIT_TIMEOUT);
+                    if (!ok) break;
+                    tc::fence_after_sync();
+                    flush_acc(tbase, q, h, acc_hi, acc_lo);
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&tfree);
+                }
+                if (!ok) break;
+                const bool fast = K <= 256;
+                store_outputs([&](int j, int sc) {
+                    return fast ? oz::assemble_int(acc_hi[j], acc_lo[j], sc) : oz::assemble(acc_hi[j], acc_lo[j], sc);
+                }, gr, gc0, M, N, er, e, md, C, ldc, nullptr, scale, status, false, cv);
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tbase, 512);
 }
 
 // ---- splitting an operand beforehand ---------------------------------------
@@ -731,14 +945,14 @@ static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b)
 
 // One CTA holds an SM (192 KB of shared memory, all of tensor memory), so the
 // K split that minimises waves per slice wins: s with ceil(tiles s / SMs) / s
-// least, a slice of at least 256 K, and a per-slice charge for the partials.
+// least, a slice of at least 128 K (a window of tensor memory), and a per-slice charge for the partials.
 // 128 x 1024 x 6000: 202 us on 160 CTAs (10 slices, two waves), 139 on 144 (9).
 int ozgemm_splits(int M, int N, int K, long long part_len)
 {
     if (M <= 0 || N <= 0 || K <= 256) return 1;
     const long long tiles = (long long)cdiv(M, ozg::BM) * cdiv(N, ozg::BN);
     const int sms = sm_count();
-    int most = cdiv(K, 256);
+    int most = cdiv(K, 128);
     const long long fit = part_len / ((long long)M * N);
     if (most > fit) most = (int)fit;
     if (most > 64) most = 64;
@@ -782,7 +996,7 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
         };
         const bool wantA = (int)grid.y >= kReuse, wantB = (int)grid.x >= kReuse;
         // scales for as many slices as there may be
-        const size_t most = cdiv(K, 256) < 64 ? cdiv(K, 256) : 64;
+        const size_t most = cdiv(K, 128) < 64 ? cdiv(K, 128) : 64;
         nexp = most * ((wantA ? M : 0) + (size_t)(wantB ? N : 0));
         exps = (int *)take(nexp * sizeof(int));
         if (exps && wantA) P.j[0].dig = (uint8_t *)take((size_t)grid.x * stages * ozg::A_BYTES);
@@ -814,7 +1028,15 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
         const ozg::PreSplit sA{P.j[0].dig, cdiv(K, ozg::KC)}, sB{P.j[1].dig, cdiv(K, ozg::KC)};
         cudaFuncSetAttribute(ozg::k_ozgemm_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
         trace_begin();
-        ozg::k_ozgemm_pre<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr(), sA, sB,
+        if (sA.dig && sB.dig && splits == 1) {
+            auto kern = K <= ozg::FLUSH * ozg::KC ? ozg::k_ozgemm_pp<true> : ozg::k_ozgemm_pp<false>;
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
+            const long long total = (long long)grid.x * grid.y;
+            const int ctas = total < sm_count() ? (int)total : sm_count();
+            kern<<<ctas, ozg::OZT + 32, ozg::SMEM, st>>>(M, N, K, C, ldc, e, status_ptr(), sA, sB, P.j[0].exps, P.j[1].exps,
+                                                        (int)grid.x, (int)total);
+        } else
+            ozg::k_ozgemm_pre<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr(), sA, sB,
                                                             P.j[0].exps, P.j[1].exps);
     } else {
         cudaFuncSetAttribute(ozg::k_ozgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
