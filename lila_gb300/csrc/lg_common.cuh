@@ -192,6 +192,12 @@ void trsm_right_lower_unit_trans(int M, int N, double alpha, const double *L, in
 void potrf_upper(int n, double *A, int lda, bool record_breakdown = true);
 // LU without pivoting of (T*S - I) with the sign choice of lila_dorgh2_3.
 void lu_sign(int n, double *T, int ldt, double *S);
+// lu_sign with the tile's other small steps (n <= 64, else false and nothing
+// done): A's upper part times S by rows, T's strict lower part moved into A.
+bool lu_sign_tile(int n, double *T, int ldt, double *S, double *A, int lda);
+// V = Q S U^-1 of M rows into B and Q := Q S, one pass (N <= 64).
+void trsm_right_upper_from(int M, int N, const double *U, int ldu, double *Q, int ldq, double *B, int ldb,
+                           const double *S, const char *tag);
 // Householder vector of a column: LAPACK dlarfg on x(0:m) (alpha = x(0)),
 // tau written to *tau.
 void larfg(int m, double *x, double *tau);

@@ -63,6 +63,7 @@ __device__ __forceinline__ void epilogue_store(double v, int r, int c, double *C
 // 32 x 32 tiles with 256-deep K slices and unpipelined loads: the 617 products
 // of a 1413 x 692 recursive QR 22.1 -> 7.1 ms, the 133 of 4000 x 1000 (tiles
 // of 256) 21.6 -> 16.1 ms, the upper 64 x 64 Gram of 262,144 rows 2.23 -> 1.4 ms.
+constexpr int UPPER_TILES = 2;  // upper_only on a grid without the tiles below the diagonal
 template <int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__(256)
     k_gemm(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e,
@@ -79,7 +80,10 @@ __global__ void __launch_bounds__(256)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // a warp covers 8 row threads x 4 column threads
     const int tr = (lane & 7) + 8 * (warp % (RT / 8)), tc = (lane >> 3) + 4 * (warp / (RT / 8));
-    const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
+    int bx = blockIdx.x, by = blockIdx.y;
+    if (e.upper_only == UPPER_TILES)  // blockIdx.x counts the tiles on and above the diagonal
+        for (by = 0; bx > by; by++) bx -= by + 1;
+    const int row0 = bx * BM, col0 = by * BN;
     if (e.upper_only && row0 > col0 + BN - 1) return;
     int kbeg = blockIdx.z * kchunk;
     int kend = min(K, kbeg + kchunk);
@@ -293,13 +297,21 @@ void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const G
     const GemmPlan p = gemm_plan(M, N, K, part ? part_len : 0, e.upper_only != 0);
     double *pp = p.splits > 1 ? part : nullptr;
     dim3 grid(ceil_div(M, p.tile), ceil_div(N, p.tile), p.splits);
+    GemmEpi ek = e;
+    if (e.upper_only && M == N) {
+        // no CTAs for the tiles below the diagonal: they would leave the others
+        // unevenly spread (64 x 64 x 262,144: 1.42 ms with them, 1.14 without)
+        ek.upper_only = UPPER_TILES;
+        grid.x = grid.x * (grid.x + 1) / 2;
+        grid.y = 1;
+    }
     trace_begin();
     if (p.tile == 64)
-        k_gemm<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
+        k_gemm<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     else if (p.tile == 32)
-        k_gemm<32, 32, 16, 2, 2><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
+        k_gemm<32, 32, 16, 2, 2><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     else
-        k_gemm<16, 16, 32, 1, 1><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, e, pp);
+        k_gemm<16, 16, 32, 1, 1><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     note_launch(tag);
     if (p.splits > 1) splitk_reduce(M, N, p.splits, part, C, ldc, e);
 }
@@ -440,39 +452,52 @@ __global__ void k_trsm_left_lower_unit(int M, int N, const double *L, int ldl, d
     }
 }
 
+// The same for M <= 64, a warp per column: the column's rows two per lane, each
+// solved entry broadcast to the rows below it (M dependent steps of one or two
+// FMAs instead of M^2 / 2 dependent global loads on one thread).
+__global__ void __launch_bounds__(128) k_trsm_left_lower_unit_warp(int M, int N, const double *L, int ldl, double *B,
+                                                                   int ldb)
+{
+    const int lane = threadIdx.x & 31, c = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (c >= N) return;
+    double *b = B + (size_t)c * ldb;
+    double b0 = lane < M ? b[lane] : 0.0, b1 = lane + 32 < M ? b[lane + 32] : 0.0;
+    for (int p = 0; p + 1 < M; p++) {
+        const double l0 = lane > p && lane < M ? L[(size_t)lane + (size_t)p * ldl] : 0.0;
+        const double l1 = lane + 32 > p && lane + 32 < M ? L[(size_t)(lane + 32) + (size_t)p * ldl] : 0.0;
+        const double x = __shfl_sync(0xffffffffu, p < 32 ? b0 : b1, p & 31);
+        b0 = lane > p ? fma(-x, l0, b0) : b0;
+        b1 = lane + 32 > p ? fma(-x, l1, b1) : b1;
+    }
+    if (lane < M) b[lane] = b0;
+    if (lane + 32 < M) b[lane + 32] = b1;
+}
+
 void trsm_left_lower_unit(int M, int N, const double *L, int ldl, double *B, int ldb)
 {
     if (M <= 1 || N <= 0) return;
+    if (M <= 64) {
+        k_trsm_left_lower_unit_warp<<<ceil_div(N, 4), 128, 0, stream()>>>(M, N, L, ldl, B, ldb);
+        note_launch("trsm_left_lower_unit");
+        return;
+    }
     k_trsm_left_lower_unit<<<ceil_div(N, 64), 64, 0, stream()>>>(M, N, L, ldl, B, ldb);
     note_launch("trsm_left_lower_unit");
 }
 
-// Row r of B solves x * U = alpha * S.*b.  U (N x N) is staged in shared
-// memory when it fits; the row's solved prefix is re-read from global memory
-// (coalesced across the threads of a warp, which own consecutive rows).
-template <bool SMEM>
+// Row r of B solves x * U = alpha * S.*b, any N: the row's solved prefix is
+// re-read from global memory (coalesced across the threads of a warp, which own
+// consecutive rows).
 __global__ void k_trsm_right_upper(int M, int N, double alpha, const double *U, int ldu, double *B,
                                    int ldb, const double *S)
 {
-    extern __shared__ double Us[];
-    if (SMEM) {
-        for (int idx = threadIdx.x; idx < N * N; idx += blockDim.x) {
-            int r = idx % N, c = idx / N;
-            Us[idx] = (r <= c) ? U[(size_t)r + (size_t)c * ldu] : 0.0;
-        }
-        __syncthreads();
-    }
     for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < (size_t)M;
          r += (size_t)gridDim.x * blockDim.x) {
         for (int c = 0; c < N; c++) {
             double s = alpha * B[r + (size_t)c * ldb];
             if (S && S[c] == -1.0) s = -s;
-            for (int p = 0; p < c; p++) {
-                double u = SMEM ? Us[p + c * N] : U[(size_t)p + (size_t)c * ldu];
-                s -= B[r + (size_t)p * ldb] * u;
-            }
-            double d = SMEM ? Us[c + c * N] : U[(size_t)c + (size_t)c * ldu];
-            B[r + (size_t)c * ldb] = s / d;
+            for (int p = 0; p < c; p++) s -= B[r + (size_t)p * ldb] * U[(size_t)p + (size_t)c * ldu];
+            B[r + (size_t)c * ldb] = s / U[(size_t)c + (size_t)c * ldu];
         }
     }
 }
@@ -512,6 +537,80 @@ __global__ void __launch_bounds__(128) k_trsm_right_upper_warp(int M, int N, dou
     if (lane + 32 < N) B[(size_t)row + (size_t)(lane + 32) * ldb] = x1;
 }
 
+// The same solve for many rows (N <= 64): a row per thread, held in registers, U
+// broadcast from shared memory, the divisions by U's diagonal as products with
+// its reciprocal corrected by the residual (3 FP64 operations instead of ~10).
+// Bound by the FP64 pipe: N^2 / 2 FMAs per row (0.85 ms for 262,144 x 64).  262,144
+// x 64: 1.26 -> 1.12 ms against rows re-read from global memory; the
+// reconstruction's copy, sign pass and solve 1.44 -> 1.09 ms in one pass.
+// Optionally the source rows come from another matrix (X, ldx), whose columns with
+// S = -1 are then negated in place: the reconstruction's V = Q S U^-1 with Q := Q S
+// in one pass.
+template <bool FROM>
+__global__ void __launch_bounds__(128) k_trsm_right_upper_rows(int M, int N, double alpha, const double *U, int ldu,
+                                                                double *B, int ldb, const double *S, double *X, int ldx)
+{
+    __shared__ __align__(16) double Us[64 * 64];
+    __shared__ double s_d[64], s_inv[64];
+    __shared__ int s_neg[64], s_plain[64];
+    for (int idx = threadIdx.x; idx < 64 * 64; idx += 128) {
+        const int r = idx & 63, c = idx >> 6;
+        Us[idx] = r < c && c < N ? U[(size_t)r + (size_t)c * ldu] : 0.0;
+    }
+    if (threadIdx.x < N) {
+        const double d = U[(size_t)threadIdx.x * (ldu + 1)];
+        s_d[threadIdx.x] = d;
+        s_inv[threadIdx.x] = 1.0 / d;
+        const int ex = (__double2hiint(d) >> 20) & 0x7FF;
+        s_plain[threadIdx.x] = ex > 40 && ex < 2007;  // d and 1 / d normal
+        s_neg[threadIdx.x] = S && S[threadIdx.x] == -1.0;
+    }
+    __syncthreads();
+    for (size_t row = blockIdx.x * (size_t)128 + threadIdx.x; row < (size_t)M; row += (size_t)gridDim.x * 128) {
+        double *b = B + row, *x = FROM ? X + row : b;
+        const int ld = FROM ? ldx : ldb;
+        double v[64];
+#pragma unroll
+        for (int c = 0; c < 64; c++) {
+            v[c] = 0.0;
+            if (c < N) v[c] = x[(size_t)c * ld];
+        }
+        if (alpha != 1.0) {
+#pragma unroll
+            for (int c = 0; c < 64; c++) v[c] *= alpha;
+        }
+#pragma unroll
+        for (int c = 0; c < 64; c++) {
+            if (c >= N) break;
+            if (s_neg[c]) {
+                v[c] = __longlong_as_double(__double_as_longlong(v[c]) ^ (long long)0x8000000000000000ull);
+                if (FROM) x[(size_t)c * ld] = v[c];
+            }
+            double t = v[c];
+#pragma unroll
+            for (int p = 0; p < c; p++) t = fma(-v[p], Us[p + c * 64], t);
+            const double inv = s_inv[c], d = s_d[c];
+            if (s_plain[c]) {
+                v[c] = t * inv;
+                v[c] = fma(fma(-v[c], d, t), inv, v[c]);
+            } else {
+                v[c] = t / d;
+            }
+            b[(size_t)c * ldb] = v[c];
+        }
+    }
+}
+
+// V = Q S U^-1 of M rows into B, Q := Q S (N <= 64).
+void trsm_right_upper_from(int M, int N, const double *U, int ldu, double *Q, int ldq, double *B, int ldb,
+                           const double *S, const char *tag)
+{
+    if (M <= 0 || N <= 0) return;
+    trace_begin();
+    k_trsm_right_upper_rows<true><<<ceil_div(M, 128), 128, 0, stream()>>>(M, N, 1.0, U, ldu, B, ldb, S, Q, ldq);
+    note_launch(tag);
+}
+
 void trsm_right_upper(int M, int N, double alpha, const double *U, int ldu, double *B, int ldb,
                       const double *S, const char *tag)
 {
@@ -523,13 +622,12 @@ void trsm_right_upper(int M, int N, double alpha, const double *U, int ldu, doub
         return;
     }
     int blocks = ceil_div(M, 128);
-    if (blocks > 16 * num_sm()) blocks = 16 * num_sm();
-    size_t sm = (size_t)N * N * sizeof(double);
     trace_begin();
     if (N <= 64) {
-        k_trsm_right_upper<true><<<blocks, 128, sm, stream()>>>(M, N, alpha, U, ldu, B, ldb, S);
+        k_trsm_right_upper_rows<false><<<blocks, 128, 0, stream()>>>(M, N, alpha, U, ldu, B, ldb, S, nullptr, 0);
     } else {
-        k_trsm_right_upper<false><<<blocks, 128, 0, stream()>>>(M, N, alpha, U, ldu, B, ldb, S);
+        if (blocks > 16 * num_sm()) blocks = 16 * num_sm();
+        k_trsm_right_upper<<<blocks, 128, 0, stream()>>>(M, N, alpha, U, ldu, B, ldb, S);
     }
     note_launch(tag);
 }
@@ -547,10 +645,40 @@ __global__ void k_trsm_right_lower_unit_trans(int M, int N, double alpha, const 
     }
 }
 
+// The same for N <= 64, a warp per row (its values two per lane, each solved one
+// broadcast to the later ones), L in shared memory: 64 x 64 in 110 -> 20 us.
+__global__ void __launch_bounds__(256) k_trsm_right_lower_unit_trans_warp(int M, int N, double alpha, const double *L,
+                                                                          int ldl, double *B, int ldb)
+{
+    __shared__ double Ls[64 * 64];
+    for (int idx = threadIdx.x; idx < N * N; idx += 256) {
+        const int r = idx % N, c = idx / N;
+        if (r > c) Ls[r + 64 * c] = L[(size_t)r + (size_t)c * ldl];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= M) return;
+    double *b = B + row;
+    double b0 = lane < N ? alpha * b[(size_t)lane * ldb] : 0.0, b1 = lane + 32 < N ? alpha * b[(size_t)(lane + 32) * ldb] : 0.0;
+    for (int p = 0; p + 1 < N; p++) {
+        const double x = __shfl_sync(0xffffffffu, p < 32 ? b0 : b1, p & 31);
+        if (x == 0.0) continue;  // left of an upper triangular row's diagonal
+        if (lane > p && lane < N) b0 = fma(-x, Ls[lane + 64 * p], b0);
+        if (lane + 32 > p && lane + 32 < N) b1 = fma(-x, Ls[lane + 32 + 64 * p], b1);
+    }
+    if (lane < N) b[(size_t)lane * ldb] = b0;
+    if (lane + 32 < N) b[(size_t)(lane + 32) * ldb] = b1;
+}
+
 void trsm_right_lower_unit_trans(int M, int N, double alpha, const double *L, int ldl, double *B,
                                  int ldb)
 {
     if (M <= 0 || N <= 0) return;
+    if (N <= 64) {
+        k_trsm_right_lower_unit_trans_warp<<<ceil_div(M, 8), 256, 0, stream()>>>(M, N, alpha, L, ldl, B, ldb);
+        note_launch("trsm_right_lower_unit_trans");
+        return;
+    }
     k_trsm_right_lower_unit_trans<<<ceil_div(M, 64), 64, 0, stream()>>>(M, N, alpha, L, ldl, B, ldb);
     note_launch("trsm_right_lower_unit_trans");
 }
@@ -623,6 +751,69 @@ __global__ void k_potrf_upper(int n, double *A, int lda, int *status)
     }
 }
 
+constexpr int SLD = 65;  // leading dimension of the 64 x 64 blocks in shared memory
+
+// The same for n <= 64 in shared memory, the pivot one step ahead: while the
+// other warps subtract row j from the rows after j + 1, warp 0 subtracts it from
+// row j + 1, takes that row's pivot (1 / sqrt by rsqrt_nr) and scales it; one
+// block barrier per step.  64 x 64: 141 us for the kernel above (every step a
+// reduction and columns of dependent global loads), 64 us here.
+__global__ void __launch_bounds__(512) k_potrf_small(int n, double *A, int lda, int *status)
+{
+    extern __shared__ double G[];  // (r, c) at r * SLD + c: a warp's lanes run along a row
+    __shared__ int s_bad;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int idx = threadIdx.x; idx < n * n; idx += 512) {
+        const int r = idx % n, c = idx / n;
+        if (r <= c) G[r * SLD + c] = A[(size_t)r + (size_t)c * lda];
+    }
+    if (threadIdx.x == 0) s_bad = n;
+    __syncthreads();
+    // row j by warp 0: the pivot and the scaling; false on a non-positive pivot
+    auto scale_row = [&](int j) {
+        const double d = G[j * SLD + j];
+        if (!(d > 0.0)) {
+            if (lane == 0) s_bad = j;
+            return;
+        }
+        const double y = rsqrt_nr(d);
+        double root = d * y;
+        root = fma(0.5 * y, fma(-root, root, d), root);
+        __syncwarp();
+        for (int c = j + lane; c < n; c += 32) {
+            const double t = G[j * SLD + c];
+            double u = t * y;
+            u = fma(fma(-u, root, t), y, u);  // t / root to rounding level
+            G[j * SLD + c] = c == j ? root : u;
+        }
+    };
+    if (warp == 0) scale_row(0);
+    __syncthreads();
+    for (int j = 0; j < n; j++) {
+        if (s_bad <= j) break;
+        if (warp == 0) {
+            if (j + 1 < n) {
+                const double l = G[j * SLD + j + 1];
+                for (int c = j + 1 + lane; c < n; c += 32) G[(j + 1) * SLD + c] = fma(-l, G[j * SLD + c], G[(j + 1) * SLD + c]);
+                __syncwarp();
+                scale_row(j + 1);
+            }
+        } else {
+            for (int r = j + 1 + warp; r < n; r += 15) {
+                const double l = G[j * SLD + r];
+                for (int c = r + lane; c < n; c += 32) G[r * SLD + c] = fma(-l, G[j * SLD + c], G[r * SLD + c]);
+            }
+        }
+        __syncthreads();
+    }
+    const int bad = s_bad;
+    for (int idx = threadIdx.x; idx < n * n; idx += 512) {
+        const int r = idx % n, c = idx / n;
+        if (r <= c && (r < bad || (r == bad && c == bad))) A[(size_t)r + (size_t)c * lda] = G[r * SLD + c];
+    }
+    if (threadIdx.x == 0 && bad < n) atomicOr(status, ST_CHOL_BREAKDOWN);
+}
+
 __device__ int d_potrf_sink;
 
 void potrf_upper(int n, double *A, int lda, bool record_breakdown)
@@ -634,7 +825,10 @@ void potrf_upper(int n, double *A, int lda, bool record_breakdown)
         cudaGetSymbolAddress(&p, d_potrf_sink);
         st = (int *)p;
     }
-    k_potrf_upper<<<1, 256, 0, stream()>>>(n, A, lda, st);
+    if (n <= 64)
+        k_potrf_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, A, lda, st);
+    else
+        k_potrf_upper<<<1, 256, 0, stream()>>>(n, A, lda, st);
     note_launch("potrf_upper");
 }
 
@@ -674,11 +868,100 @@ __global__ void k_lu_sign(int n, double *T, int ldt, double *S, int *status)
     }
 }
 
+// The same for n <= 64 in shared memory, the pivot column one step ahead of the
+// others (as in k_potrf_small).  The pivot is -(1 + |t_kk|), so its reciprocal
+// needs no division.  64 x 64: 73 us with the two launches it replaces.  With A given, the reconstruction's other small steps too:
+// the strict lower part goes to A (and leaves zeros in T), and A's rows k with
+// S(k) = -1 are negated from the diagonal on.
+__global__ void __launch_bounds__(512) k_lu_sign_small(int n, double *T, int ldt, double *S, double *A, int lda,
+                                                       int *status)
+{
+    extern __shared__ double G[];  // column-major, SLD
+    __shared__ double s_sgn[64];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int idx = threadIdx.x; idx < n * n; idx += 512) {
+        const int r = idx % n, c = idx / n;
+        G[r + c * SLD] = T[(size_t)r + (size_t)c * ldt];
+    }
+    __syncthreads();
+    auto pivot_col = [&](int k) {  // warp 0
+        double *g = G + k * SLD;
+        const double t = g[k];
+        // |1 - t| < |1 + t| in FP64 is t > 2^-54, an integer comparison
+        const long long tb = __double_as_longlong(t);
+        const bool neg = tb > 0x3C90000000000000ll && tb <= 0x7FF0000000000000ll;
+        const long long flip = neg ? (long long)0x8000000000000000ull : 0ll;
+        const double p = __longlong_as_double(tb ^ flip) - 1.0, inv = -rcp_nr(-p);
+        __syncwarp();
+        for (int r0 = 0; r0 < n; r0 += 32) {
+            const int r = r0 + lane;
+            if (r >= n) continue;
+            const double a = __longlong_as_double(__double_as_longlong(g[r]) ^ flip);
+            double l = a;
+            if (r0 + 31 > k) {  // some row of the warp below the pivot
+                l = a * inv;
+                l = fma(fma(-l, p, a), inv, l);
+            }
+            g[r] = r < k ? a : (r == k ? p : l);
+        }
+        if (lane == 0) {
+            s_sgn[k] = neg ? -1.0 : 1.0;
+            if (p == 0.0) atomicOr(status, ST_LU_ZERO_PIVOT);
+        }
+    };
+    if (warp == 0) pivot_col(0);
+    __syncthreads();
+    for (int k = 0; k + 1 < n; k++) {
+        const double *l = G + k * SLD;
+        if (warp == 0) {
+            double *g = G + (k + 1) * SLD;
+            const double u = g[k];
+            for (int r = (k + 1) / 32 * 32 + lane; r < n; r += 32)
+                if (r > k) g[r] = fma(-l[r], u, g[r]);
+            __syncwarp();
+            pivot_col(k + 1);
+        } else {
+            for (int c = k + 1 + warp; c < n; c += 15) {
+                double *g = G + c * SLD;
+                const double u = g[k];
+                for (int r = (k + 1) / 32 * 32 + lane; r < n; r += 32)
+                    if (r > k) g[r] = fma(-l[r], u, g[r]);
+            }
+        }
+        __syncthreads();
+    }
+    for (int idx = threadIdx.x; idx < n * n; idx += 512) {
+        const int r = idx % n, c = idx / n;
+        const double v = G[r + c * SLD];
+        T[(size_t)r + (size_t)c * ldt] = A && r > c ? 0.0 : v;
+        if (A) {
+            double *a = A + (size_t)r + (size_t)c * lda;
+            if (r > c)
+                *a = v;
+            else if (s_sgn[r] == -1.0)
+                *a = -*a;
+        }
+    }
+    if (threadIdx.x < n) S[threadIdx.x] = s_sgn[threadIdx.x];
+}
+
 void lu_sign(int n, double *T, int ldt, double *S)
 {
     if (n <= 0) return;
-    k_lu_sign<<<1, 256, 0, stream()>>>(n, T, ldt, S, status_ptr());
+    if (n <= 64)
+        k_lu_sign_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, T, ldt, S, nullptr, 0, status_ptr());
+    else
+        k_lu_sign<<<1, 256, 0, stream()>>>(n, T, ldt, S, status_ptr());
     note_launch("lu_sign");
+}
+
+bool lu_sign_tile(int n, double *T, int ldt, double *S, double *A, int lda)
+{
+    if (n > 64) return false;
+    if (n <= 0) return true;
+    k_lu_sign_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, T, ldt, S, A, lda, status_ptr());
+    note_launch("lu_sign");
+    return true;
 }
 
 // LAPACK dlarfg on x(0:m): beta = -sign(alpha)*||x||, tau = (beta-alpha)/beta,

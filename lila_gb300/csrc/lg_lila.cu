@@ -341,14 +341,23 @@ void move_strict_lower_dev(int n, double *T, int ldt, double *A, int lda) { move
 // LU-with-sign reconstruction finishing steps shared by lila_dorgh2_3 and the
 // tile routine: T holds the (reduced) top block, A(n:rows) the reduced rest.
 // lila-c/lila_dorgh2_3.c:8-51.
+// rows_v rows below the block; from_q: they still stand in Q (rows n.. of Qc)
+// and go straight from there to V, with Q's signs in the same pass.
 static void reconstruct(int rows_v, int n, double *Ajj, int lda, double *Tjj, int ldt, double *Qc,
-                        int q_rows, int ldq, double *S)
+                        int q_rows, int ldq, double *S, bool from_q = false)
 {
-    lu_sign(n, Tjj, ldt, S);
-    flip_rows(n, n, S, Ajj, lda, 1);
-    flip_cols(q_rows, n, S, Qc, ldq);
-    move_strict_lower(n, Tjj, ldt, Ajj, lda);
-    trsm_right_upper(rows_v, n, 1.0, Tjj, ldt, Ajj + n, lda, S, "hr_trsm_v");
+    if (!lu_sign_tile(n, Tjj, ldt, S, Ajj, lda)) {
+        lu_sign(n, Tjj, ldt, S);
+        flip_rows(n, n, S, Ajj, lda, 1);
+        move_strict_lower(n, Tjj, ldt, Ajj, lda);
+    }
+    if (from_q) {
+        flip_cols(q_rows - rows_v, n, S, Qc, ldq);
+        trsm_right_upper_from(rows_v, n, Tjj, ldt, Qc + q_rows - rows_v, ldq, Ajj + n, lda, S, "hr_trsm_v");
+    } else {
+        flip_cols(q_rows, n, S, Qc, ldq);
+        trsm_right_upper(rows_v, n, 1.0, Tjj, ldt, Ajj + n, lda, S, "hr_trsm_v");
+    }
     trsm_right_lower_unit_trans(n, n, -1.0, Ajj, lda, Tjj, ldt);
 }
 
@@ -373,9 +382,10 @@ static void panel_hr(int m, int n, int i, int mt, double *A, int lda, double *T,
     double *Qii = Q + i + (size_t)i * ldq;
     double *Tki = T + i % mt + (size_t)i * ldt;
     cholqr(ml, n, Aii, lda, Qii, ldq, w);
-    copy2d(ml - n, n, Qii + n, ldq, Aii + n, lda);
+    const bool from_q = n <= 64;
+    if (!from_q) copy2d(ml - n, n, Qii + n, ldq, Aii + n, lda);
     copy2d(n, n, Qii, ldq, Tki, ldt);
-    reconstruct(ml - n, n, Aii, lda, Tki, ldt, Qii, ml, ldq, S);
+    reconstruct(ml - n, n, Aii, lda, Tki, ldt, Qii, ml, ldq, S, from_q);
 }
 
 static void panel(const int *lp, int m, int n, int i, int mt, double *A, int lda, double *T,
@@ -404,14 +414,16 @@ static void ormhr2(int m, int n, int i, int j, int mt, double *A, int lda, doubl
     int ldw = jw > 0 ? jw : 1;
     copy2d(jw, n, Qij, ldq, W2, ldw);
     copy2d(n, n, Qjj, ldq, Tjj, ldt);
-    copy2d(m - j - n, n, Qjj + n, ldq, Ajj + n, lda);
+    // the first tile's rows go from Q to V in one pass
+    const bool from_q = jw == 0 && n <= 64;
+    if (!from_q) copy2d(m - j - n, n, Qjj + n, ldq, Ajj + n, lda);
     if (jw > 0) {
         trsm_left_lower_unit(jw, n, Aii, lda, W2, ldw);
         gemm(n, n, jw, opnd(Aji, lda), opnd(W2, ldw), Tjj, ldt, epi(-1, 1));
         gemm(m - j - n, n, jw, opnd(Aji + n, lda), opnd(W2, ldw), Ajj + n, lda, epi(-1, 1), nullptr, 0,
              "hr_couple");
     }
-    reconstruct(m - j - n, n, Ajj, lda, Tjj, ldt, Qij, m - i, ldq, S + j);
+    reconstruct(m - j - n, n, Ajj, lda, Tjj, ldt, Qij, m - i, ldq, S + j, from_q);
 }
 
 // ---------------------------------------------------------------------------
