@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(256)
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0;
 
     double ra[LA], rb[LB];
+    chain_wait();
     auto load = [&](int k0) {
 #pragma unroll
         for (int u = 0; u < LA; u++) {
@@ -159,6 +160,10 @@ __global__ void __launch_bounds__(256)
             }
         }
     }
+    // Only now: blocks of the next kernel let in before would be placed where
+    // this one's blocks have left room, several to some SMs and none to others
+    // (opened at the start: 4000 x 1000 in tiles of 256 21.4 -> 22.3 ms).
+    chain_open();
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
@@ -178,6 +183,7 @@ __global__ void __launch_bounds__(256)
 __global__ void k_splitk_reduce(int M, int N, int splits, const double *part, double *C, int ldc,
                                 GemmEpi e)
 {
+    chain_wait();
     size_t total = (size_t)M * N;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -196,6 +202,7 @@ __global__ void k_splitk_reduce(int M, int N, int splits, const double *part, do
         for (; z < splits; z++, p += total) s += *p;
         epilogue_store(s, r, c, C, ldc, e);
     }
+    chain_open();
 }
 
 // SM count of the current device (queried once), for the grid heuristics
@@ -285,15 +292,10 @@ static bool split_pays(int M, int N, int K)
     return 38.0 + 0.175 * pad < 10.0 + 1.65 * fma;
 }
 
-void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e,
-          double *part, long long part_len, const char *tag)
+// The product, or (more than one slice returned) its K slices in `part`.
+static int gemm_parts(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e, double *part,
+                      long long part_len, const char *tag)
 {
-    if (M <= 0 || N <= 0) return;
-    if (split_pays(M, N, K)) {
-        ozgemm(M, N, K, A, B, C, ldc, e, part, part_len, "ozgemm");
-        return;
-    }
-    cudaStream_t st = stream();
     const GemmPlan p = gemm_plan(M, N, K, part ? part_len : 0, e.upper_only != 0);
     double *pp = p.splits > 1 ? part : nullptr;
     dim3 grid(ceil_div(M, p.tile), ceil_div(N, p.tile), p.splits);
@@ -307,13 +309,107 @@ void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const G
     }
     trace_begin();
     if (p.tile == 64)
-        k_gemm<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        launch_chained(k_gemm<64, 64, 16, 4, 4>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     else if (p.tile == 32)
-        k_gemm<32, 32, 16, 2, 2><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        launch_chained(k_gemm<32, 32, 16, 2, 2>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     else
-        k_gemm<16, 16, 32, 1, 1><<<grid, 256, 0, st>>>(M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        launch_chained(k_gemm<16, 16, 32, 1, 1>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
     note_launch(tag);
-    if (p.splits > 1) splitk_reduce(M, N, p.splits, part, C, ldc, e);
+    return p.splits;
+}
+
+void gemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const GemmEpi &e,
+          double *part, long long part_len, const char *tag)
+{
+    if (M <= 0 || N <= 0) return;
+    if (split_pays(M, N, K)) {
+        ozgemm(M, N, K, A, B, C, ldc, e, part, part_len, "ozgemm");
+        return;
+    }
+    const int splits = gemm_parts(M, N, K, A, B, C, ldc, e, part, part_len, tag);
+    if (splits > 1) splitk_reduce(M, N, splits, part, C, ldc, e);
+}
+
+// The sum of the product's K slices (vb x n partials; one: the product itself)
+// times op(T), `cols` columns per CTA: the sums go to shared memory, next to
+// T's triangle.  Latency bounds it (rounds of loads, then chains of up to vb
+// FMAs), so a CTA has one column while there are SMs for it, four at most, and
+// threads left over share an output's terms.  One launch instead of the slices'
+// reduction and a product of its own (6.5 + 5.8 us at 32 x 31, 6.8 us together).
+constexpr int RT_COLS = 4, RT_NTH = 128;
+__global__ void __launch_bounds__(RT_NTH) k_reduce_times_tri(int vb, int n, int cols, int splits, const double *part,
+                                                             const double *T, int ldt, int trans, double *W2)
+{
+    __shared__ double Ws[64 * RT_COLS], Ts[64 * 65], Ps[2][RT_NTH];
+    chain_wait();
+    const int c0 = blockIdx.x * cols, nc = min(cols, n - c0), out = vb * nc;
+    const size_t total = (size_t)vb * n;
+    // T's triangle as rows of op(T): Ts[r + k * 65] = op(T)(r, k)
+    {
+        const int r = threadIdx.x & 63;
+#pragma unroll 4
+        for (int c = threadIdx.x >> 6; c < vb; c += RT_NTH / 64)
+            if (r <= c) Ts[trans == TR ? c + r * 65 : r + c * 65] = T[(size_t)r + (size_t)c * ldt];
+    }
+    // P threads to an output, part p of its terms each; with P > 1 there is
+    // one round of outputs
+    const int P = out <= RT_NTH / 4 ? 4 : out <= RT_NTH / 2 ? 2 : 1;
+    const int me = P == 1 ? threadIdx.x : threadIdx.x % (RT_NTH / P), p = P == 1 ? 0 : threadIdx.x / (RT_NTH / P);
+    auto combine = [&](double *ps, double s) {
+        if (P == 1) return s;
+        ps[threadIdx.x] = s;
+        __syncthreads();
+        if (p) return 0.0;
+        s += ps[me + RT_NTH / P];
+        if (P == 4) s += ps[me + 2 * (RT_NTH / 4)] + ps[me + 3 * (RT_NTH / 4)];
+        return s;
+    };
+    for (int idx = me; idx < (P == 1 ? out : RT_NTH / P); idx += RT_NTH / P) {
+        double s = 0.0;
+        if (idx < out) {
+            const double *q = part + (size_t)c0 * vb + idx;
+            int z = p;
+            for (; z + 3 * P < splits; z += 4 * P) {
+                double v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = q[(size_t)(z + u * P) * total];
+                s += (v[0] + v[1]) + (v[2] + v[3]);
+            }
+            for (; z < splits; z += P) s += q[(size_t)z * total];
+        }
+        s = combine(Ps[0], s);
+        if (p == 0 && idx < out) Ws[idx] = s;
+    }
+    __syncthreads();
+    chain_open();
+    for (int idx = me; idx < (P == 1 ? out : RT_NTH / P); idx += RT_NTH / P) {
+        double s = 0.0;
+        if (idx < out) {
+            const int r = idx % vb, c = idx / vb;
+            const int k0 = trans == TR ? 0 : r, k1 = trans == TR ? r + 1 : vb;
+            for (int k = k0 + p; k < k1; k += P) s = fma(Ts[r + k * 65], Ws[k + c * vb], s);
+        }
+        s = combine(Ps[1], s);
+        if (p == 0 && idx < out) W2[(size_t)c0 * vb + idx] = s;
+    }
+}
+
+void gemm_times_tri(int vb, int n, int K, Operand A, Operand B, const double *T, int ldt, int trans, double *W1,
+                    double *W2, double *part, long long part_len)
+{
+    if (vb <= 0 || n <= 0) return;
+    GemmEpi e;
+    if (vb > 64 || split_pays(vb, n, K)) {
+        gemm(vb, n, K, A, B, W1, vb, e, part, part_len);
+        gemm(vb, n, vb, opnd(T, ldt, trans, M_UPPER), opnd(W1, vb), W2, vb, e);
+        return;
+    }
+    const int splits = gemm_parts(vb, n, K, A, B, W1, vb, e, part, part_len, "gemm");
+    trace_begin();
+    const int cols = std::min(ceil_div(n, num_sm()), RT_COLS);
+    launch_chained(k_reduce_times_tri, dim3(ceil_div(n, cols)), 128, 0, vb, n, cols, splits, splits > 1 ? part : W1, T,
+                   ldt, trans, W2);
+    note_launch("reduce_times_tri");
 }
 
 void splitk_reduce(int M, int N, int splits, const double *part, double *C, int ldc, const GemmEpi &e)
@@ -322,7 +418,7 @@ void splitk_reduce(int M, int N, int splits, const double *part, double *C, int 
     int blocks = ceil_div(total, 128);
     if (blocks > 8 * num_sm()) blocks = 8 * num_sm();
     trace_begin();
-    k_splitk_reduce<<<blocks, 128, 0, stream()>>>(M, N, splits, part, C, ldc, e);
+    launch_chained(k_splitk_reduce, dim3(blocks), 128, 0, M, N, splits, part, C, ldc, e);
     note_launch("splitk_reduce");
 }
 
@@ -1061,6 +1157,7 @@ __global__ void __launch_bounds__(512) k_larft_small(int k, const double *G, int
 {
     extern __shared__ double lf[];
     double *Gs = lf, *Ts = lf + 64 * LARFT_LD, *Ys = lf + 2 * 64 * LARFT_LD;
+    chain_wait();
     for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
         const int r = idx % k, c = idx / k;
         if (r < c) Gs[r + c * LARFT_LD] = G[(size_t)r + (size_t)c * ldg];
@@ -1087,6 +1184,7 @@ __global__ void __launch_bounds__(512) k_larft_small(int k, const double *G, int
         }
         __syncthreads();
     }
+    chain_open();
     for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
         const int r = idx % k, c = idx / k;
         if (r <= c) T[(size_t)r + (size_t)c * ldt] = Ts[r + c * LARFT_LD];
@@ -1100,7 +1198,7 @@ void larft_from_gram(int k, const double *G, int ldg, const double *tau, double 
     if (k <= 64) {
         constexpr int smem = 3 * 64 * LARFT_LD * (int)sizeof(double);
         cudaFuncSetAttribute(k_larft_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        k_larft_small<<<1, 512, smem, stream()>>>(k, G, ldg, tau, T, ldt);
+        launch_chained(k_larft_small, dim3(1), 512, smem, k, G, ldg, tau, T, ldt);
     } else {
         k_larft_from_gram<<<1, 256, (size_t)k * sizeof(double), stream()>>>(k, G, ldg, tau, T, ldt);
     }

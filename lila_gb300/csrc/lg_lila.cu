@@ -192,8 +192,7 @@ static void apply_qt(int m, int n, int k, int i, int mt, const double *A, int ld
         const double *V = A + a + (size_t)a * lda;
         const double *Tt = T + a % mt + (size_t)a * ldt;
         double *Ct = C + a;
-        gemm(vb, n, m - a, opnd(V, lda, TR, M_UNIT_LOWER), opnd(Ct, ldc), W1, vb, epi(1, 0), w.p, w.len);
-        gemm(vb, n, vb, opnd(Tt, ldt, TR, M_UPPER), opnd(W1, vb), W2, vb, epi(1, 0));
+        gemm_times_tri(vb, n, m - a, opnd(V, lda, TR, M_UNIT_LOWER), opnd(Ct, ldc), Tt, ldt, TR, W1, W2, w.p, w.len);
         gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), Ct, ldc, epi(-1, 1), w.p, w.len);
         a = b;
     }
@@ -226,8 +225,7 @@ static void apply_q_bz(int m, int n, int k, int i, int j, int mt, const double *
         const double *V = A + a + (size_t)a * lda;
         const double *Vbot = A + b + (size_t)a * lda;
         const double *Tt = T + a % mt + (size_t)a * ldt;
-        gemm(vb, n, m - b, opnd(Vbot, lda, TR), opnd(X + b, ldq), W1, vb, epi(1, 0), w.p, w.len);
-        gemm(vb, n, vb, opnd(Tt, ldt, NT, M_UPPER), opnd(W1, vb), W2, vb, epi(1, 0));
+        gemm_times_tri(vb, n, m - b, opnd(Vbot, lda, TR), opnd(X + b, ldq), Tt, ldt, NT, W1, W2, w.p, w.len);
         GemmEpi e = epi(-1, 1);
         e.zero_rows = vb;
         gemm(m - a, n, vb, opnd(V, lda, NT, M_UNIT_LOWER), opnd(W2, vb), X + a, ldq, e, w.p, w.len);
@@ -250,8 +248,7 @@ static void connect(int m, int n, int i, int j, int mt, const double *A, int lda
     double *Tki = T + i % mt + (size_t)i * ldt;
     double *Tji = T + (i % mt - wb) + (size_t)i * ldt;
     double *Tjj = T + (i % mt - wb) + (size_t)(i - wb) * ldt;
-    gemm(wb, vb, m - i, opnd(V1, lda, TR), opnd(V2, lda, NT, M_UNIT_LOWER), G, wb, epi(1, 0), w.p, w.len);
-    gemm(wb, vb, wb, opnd(Tjj, ldt, NT, M_UPPER), opnd(G, wb), Y, wb, epi(1, 0));
+    gemm_times_tri(wb, vb, m - i, opnd(V1, lda, TR), opnd(V2, lda, NT, M_UNIT_LOWER), Tjj, ldt, NT, G, Y, w.p, w.len);
     gemm(wb, vb, vb, opnd(Y, wb), opnd(Tki, ldt, NT, M_UPPER), Tji, ldt, epi(-1, 0));
 }
 
@@ -278,15 +275,13 @@ static void dgeqr3_dev(int m, int n, double *A, int lda, double *T, int ldt, Wor
     double *W1 = w2.take((long long)n1 * n2);
     double *W2 = w2.take((long long)n1 * n2);
     double *A12 = A + (size_t)n1 * lda;
-    gemm(n1, n2, m, opnd(A, lda, TR, M_UNIT_LOWER), opnd(A12, lda), W1, n1, epi(1, 0), w2.p, w2.len);
-    gemm(n1, n2, n1, opnd(T, ldt, TR, M_UPPER), opnd(W1, n1), W2, n1, epi(1, 0));
+    gemm_times_tri(n1, n2, m, opnd(A, lda, TR, M_UNIT_LOWER), opnd(A12, lda), T, ldt, TR, W1, W2, w2.p, w2.len);
     gemm(m, n2, n1, opnd(A, lda, NT, M_UNIT_LOWER), opnd(W2, n1), A12, lda, epi(-1, 1));
     double *A22 = A + n1 + (size_t)n1 * lda;
     double *T22 = T + n1 + (size_t)n1 * ldt;
     dgeqr3_dev(m - n1, n2, A22, lda, T22, ldt, w);
     // T12 = -T11 (Y1(n1:m)^T Y2) T22
-    gemm(n1, n2, m - n1, opnd(A + n1, lda, TR), opnd(A22, lda, NT, M_UNIT_LOWER), W1, n1, epi(1, 0), w2.p, w2.len);
-    gemm(n1, n2, n1, opnd(T, ldt, NT, M_UPPER), opnd(W1, n1), W2, n1, epi(1, 0));
+    gemm_times_tri(n1, n2, m - n1, opnd(A + n1, lda, TR), opnd(A22, lda, NT, M_UNIT_LOWER), T, ldt, NT, W1, W2, w2.p, w2.len);
     gemm(n1, n2, n2, opnd(W2, n1), opnd(T22, ldt, NT, M_UPPER), T + (size_t)n1 * ldt, ldt, epi(-1, 0));
 }
 
