@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "lg_common.cuh"
+#include "lg_house.cuh"
 #include "../../include/lila_gpu.h"
 
 namespace lg {
@@ -446,17 +447,22 @@ __global__ void __launch_bounds__(NT, 3) k_final_b(const BMInst *inst, const int
 // ---------------------------------------------------------------------------
 namespace feat {
 
-constexpr int NT = 256, LDC = 132, CH2 = 16, LD2 = 130, SMAX = 176, NB = 8;
+constexpr int NT = 256, SMAX = 176, NB = 8;
 
-// Shared memory of one size class (n <= nmax): the sketch (ld sld, odd so
-// that threads reading consecutive columns hit distinct banks; later the
-// FP32 Gram, ld nmax), a CH2-row FP64 chunk of A (later the block
-// reflector's W, 2 NB x nmax) and the same chunk in FP32 (ld LDC).
-__host__ __device__ inline int sketch_ld(int nmax) { return (min(2 * nmax, SMAX)) | 1; }
-__host__ __device__ inline size_t smem_bytes(int nmax)
-{
-    return (size_t)sketch_ld(nmax) * nmax * 8 + (size_t)CH2 * LD2 * 8 + (size_t)CH2 * LDC * 4;
-}
+// One size class, n <= 32 NW: a chunk of A is CH rows (2,048 elements in
+// flight per CTA, 1,536 for NW = 3), kept in FP64 (ld LD64) and FP32 (ld LD32);
+// the sketch has ld SLD, odd so that threads on consecutive columns hit distinct
+// banks.  Shared memory is the sketch (later the FP32 Gram, ld GLD) and the two
+// chunks (later the block reflector's sums, NT x NB doubles).
+template <int NW>
+struct Size {
+    static constexpr int NMAX = 32 * NW, CHL = NW == 1 ? 6 : NW == 2 ? 5 : 4, CH = 1 << CHL;
+    static constexpr int LD64 = NMAX + 1, LD32 = NMAX + 4, GLD = NMAX + 1;
+    static constexpr int SROWS = 2 * NMAX < SMAX ? 2 * NMAX : SMAX, SLD = SROWS | 1, RPL = SROWS / 16;
+    static constexpr int CHUNKS = CH * (LD64 * 8 + LD32 * 4), SUMS = NT * NB * 8;
+    static constexpr size_t BYTES = (size_t)SLD * NMAX * 8 + (CHUNKS > SUMS ? CHUNKS : SUMS);
+    static_assert(SLD * NMAX * 8 >= GLD * NMAX * 4 && CH * LD64 % 2 == 0 && SLD * NMAX % 2 == 0, "buffers are reused");
+};
 
 __device__ __forceinline__ uint32_t mix32(uint32_t x)
 {
@@ -482,371 +488,464 @@ __device__ __forceinline__ double wsum(double v)
     return v;
 }
 
+// x, or -x when bit 0 of b is clear.
+__device__ __forceinline__ double flip(double x, int b)
+{
+    return __hiloint2double(__double2hiint(x) ^ ((b & 1) ? 0 : 0x80000000), __double2loint(x));
+}
+
+__device__ __forceinline__ void panel_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
 // Householder QR (LAPACK dgeqrf conventions, tau = 0 for a zero column below
-// the diagonal) of the ns x nn matrix S (ld sld) in shared memory, in panels
-// of NB columns: each panel is factored column by column, then its block
-// reflector I - V T V^T (T from V^T V by the dlarft recurrence) is applied
-// to the trailing columns: W = V^T C (two threads per column, row halves),
-// W = T^T W, C -= V W (one thread per element).  R is left in the upper
-// triangle.  Wp needs 2 NB nn doubles.
+// the diagonal) of the ns x nn matrix S (ld sld) in shared memory, ns <= 16 RPL,
+// in panels of NB columns; R is left in the upper triangle.  One warp
+// instruction of FP64 holds its SM sub-partition for 64 clocks, so their count
+// per sub-partition is what a phase costs:
+//   panel: 16 lanes per column with its rows in registers, on four warps, one
+//     per sub-partition (32 lanes per column, two warps to each: 72 instructions
+//     per step instead of 45);
+//   sums: V^T [V C], a thread per column and row slice, as many slices as
+//     there are threads; the slices are added up and the triangular system of
+//     the reflectors' Gram V^T V and 1 / tau solved by one thread per column
+//     (no T, whose recurrence would be one thread's);
+//   update: C -= V W, four elements per thread at a time.
+// 176 x 95: 1.81 million clocks with a warp per column in shared memory and T,
+// 1.34 now (panels 0.42, updates 0.34); its FMAs alone are 0.65.
+template <int RPL>
 __device__ void house_qr(int ns, int nn, double *S, int sld, double *Wp)
 {
-    __shared__ double s_tau[NB], s_T[NB * NB], s_G[NB * NB];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ double s_tau[NB], s_pub[2][16 * RPL], s_ss[2];
+    const int tid = threadIdx.x, warp = tid >> 5;
     for (int j0 = 0; j0 < nn; j0 += NB) {
-        const int jb = min(NB, nn - j0);
-        for (int k = j0; k < j0 + jb; k++) {
-            double *ck = S + (size_t)sld * k;
-            if (warp == 0) {
-                double ss = 0.0;
-                for (int r = k + 1 + lane; r < ns; r += 32) ss += ck[r] * ck[r];
-                ss = wsum(ss);
-                const double alpha = ck[k];
-                double tau = 0.0, sc = 0.0, beta = alpha;
-                if (ss > 0.0) {
-                    beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-                    tau = (beta - alpha) / beta;
-                    sc = 1.0 / (alpha - beta);
+        const int jb = min(NB, nn - j0), rows = ns - j0;
+        if (warp < 4) {
+            const int g = tid >> 4, gl = tid & 15, qn = (rows + 15) >> 4;
+            double *col = S + (size_t)sld * (j0 + g) + j0 + gl;
+            double x[RPL], my_tau = 0.0, my_sc = 1.0, my_beta = 0.0;
+#pragma unroll
+            for (int q = 0; q < RPL; q++) x[q] = (g < jb && gl + 16 * q < rows) ? col[16 * q] : 0.0;
+            for (int k = 0; k < jb; k++) {
+                double *pub = s_pub[k & 1];
+                if (g == k) {
+#pragma unroll
+                    for (int q = 0; q < RPL; q++)
+                        if (q < qn) pub[gl + 16 * q] = x[q];
                 }
-                if (tau != 0.0)
-                    for (int r = k + 1 + lane; r < ns; r += 32) ck[r] *= sc;
-                __syncwarp();
-                if (lane == 0) {
-                    ck[k] = beta;
-                    s_tau[k - j0] = tau;
+                panel_bar();
+                const bool on = 2 * warp + 1 >= k;  // this warp has column k or a later one
+                double v[RPL], d = 0.0;
+                if (on) {
+                    double d1 = 0.0;
+#pragma unroll
+                    for (int q = 0; q < RPL; q++)
+                        if (q < qn) {
+                            v[q] = q || gl > k ? pub[gl + 16 * q] : 0.0;
+                            if (q & 1)
+                                d1 = fma(v[q], x[q], d1);
+                            else
+                                d = fma(v[q], x[q], d);
+                        }
+                    d = group_sum<16>(d + d1);
+                    if (g == k && gl == 0) s_ss[k & 1] = d;
                 }
+                panel_bar();
+                if (!on) continue;
+                const double ss = s_ss[k & 1], alpha = pub[k];
+                const long long sb = __double_as_longlong(ss);
+                const Reflector h = house_reflector(alpha, ss, sb > 0 && sb <= 0x7FF0000000000000LL);
+                if (g == k) {
+                    my_tau = h.tau;
+                    my_beta = h.beta;
+                    if (h.tau != 0.0) my_sc = h.sc;
+                }
+                if (__double_as_longlong(h.tau) == 0) continue;
+                const double ck = __shfl_sync(0xffffffffu, x[0], (tid & 16) + k);
+                const double w = g > k ? h.tau * fma(h.sc, d, ck) : 0.0, ws = w * h.sc;
+                const double v0 = gl > k ? ws * v[0] : gl == k ? w : 0.0;
+                x[0] -= v0;
+#pragma unroll
+                for (int q = 1; q < RPL; q++)
+                    if (q < qn) x[q] = fma(-ws, v[q], x[q]);
             }
-            __syncthreads();
-            const double tau = s_tau[k - j0];
-            const int c = k + 1 + warp;
-            if (tau != 0.0 && c < j0 + jb) {
-                double *cc = S + (size_t)sld * c;
-                double d = 0.0;
-                for (int r = k + 1 + lane; r < ns; r += 32) d += ck[r] * cc[r];
-                const double w = tau * (cc[k] + wsum(d));
-                for (int r = k + 1 + lane; r < ns; r += 32) cc[r] -= w * ck[r];
-                __syncwarp();
-                if (lane == 0) cc[k] -= w;
+            if (g < jb) {
+                if (gl == 0) s_tau[g] = my_tau;
+#pragma unroll
+                for (int q = 0; q < RPL; q++)
+                    if (gl + 16 * q < rows) {
+                        if (q || gl > g)
+                            col[16 * q] = my_sc * x[q];
+                        else
+                            col[0] = gl == g ? my_beta : x[0];
+                    }
             }
-            __syncthreads();
-        }
-        const int c0 = j0 + jb, nc = nn - c0;
-        if (nc <= 0) break;
-        // G(a, b) = v_a^T v_b, a < b (v_a: 1 at row j0 + a, S below, 0 above)
-        for (int q = warp; q < jb * jb; q += NT / 32) {
-            const int a = q % jb, b = q / jb;
-            if (a >= b) continue;
-            const double *va = S + (size_t)sld * (j0 + a), *vb = S + (size_t)sld * (j0 + b);
-            double d = 0.0;
-            for (int r = j0 + b + 1 + lane; r < ns; r += 32) d += va[r] * vb[r];
-            d = wsum(d);
-            if (lane == 0) s_G[a + NB * b] = d + va[j0 + b];
         }
         __syncthreads();
-        if (tid == 0) {
-            for (int i = 0; i < jb; i++) {
-                const double ti = s_tau[i];
-                for (int r = 0; r < i; r++) {
-                    double x = 0.0;
-                    for (int p = r; p < i; p++) x += s_T[r + NB * p] * s_G[p + NB * i];
-                    s_T[r + NB * i] = -ti * x;
-                }
-                s_T[i + NB * i] = ti;
-            }
-        }
-        // W = V^T C: thread (c, half) sums rows of its half
-        const int rows = ns - j0, hrows = (rows + 1) >> 1;
-        if (tid < 2 * nc) {
-            const int cl = tid % nc, hf = tid / nc;
-            const double *cc = S + (size_t)sld * (c0 + cl);
+        const int c0 = j0 + jb, nc = nn - c0;
+        if (nc <= 0) break;  // past here jb = NB
+        // column cl of [V C]: its sums with the NB reflectors over a slice of the rows
+        const int ncv = nc + NB, slices = NT / ncv, hrows = (rows + slices - 1) / slices;
+        const double *V = S + (size_t)sld * j0 + j0;
+        if (tid < slices * ncv) {
+            const int cl = tid % ncv, sl = tid / ncv;
+            const double *cc = V + (size_t)sld * cl;
             double acc[NB];
 #pragma unroll
             for (int i = 0; i < NB; i++) acc[i] = 0.0;
-            const int r1 = min(ns, j0 + (hf + 1) * hrows);
-            for (int r = j0 + hf * hrows; r < r1; r++) {
-                const double x = cc[r];
+            const int r1 = min(rows, (sl + 1) * hrows);
+            int r = sl * hrows;
+            for (; r < min(r1, NB); r++) {  // the reflectors' own triangle
+                const double x = cl >= NB || r > cl ? cc[r] : r == cl ? 1.0 : 0.0;
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
-                    if (i < jb) {
-                        const int d = j0 + i;
-                        const double v = r > d ? S[r + (size_t)sld * d] : (r == d ? 1.0 : 0.0);
-                        acc[i] += v * x;
-                    }
+                    const double v = r > i ? V[r + (size_t)sld * i] : r == i ? 1.0 : 0.0;
+                    acc[i] = fma(v, x, acc[i]);
                 }
             }
+#pragma unroll 2
+            for (; r < r1; r++) {
+                const double x = cc[r];
 #pragma unroll
-            for (int i = 0; i < NB; i++) Wp[(hf * NB + i) * nn + cl] = acc[i];
+                for (int i = 0; i < NB; i++) acc[i] = fma(V[r + (size_t)sld * i], x, acc[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < NB; i++) Wp[(sl * NB + i) * ncv + cl] = acc[i];
         }
         __syncthreads();
-        // W := T^T W (both halves summed)
+        for (int idx = tid; idx < NB * ncv; idx += NT) {
+            double w = Wp[idx];
+            for (int sl = 1; sl < slices; sl++) w += Wp[sl * NB * ncv + idx];
+            Wp[idx] = w;
+        }
+        __syncthreads();
         if (tid < nc) {
             double w[NB];
 #pragma unroll
-            for (int i = 0; i < NB; i++) w[i] = Wp[i * nn + tid] + Wp[(NB + i) * nn + tid];
+            for (int i = 0; i < NB; i++) w[i] = Wp[i * ncv + NB + tid];
 #pragma unroll
-            for (int i = NB - 1; i >= 0; i--) {
-                double x = 0.0;
+            for (int i = 0; i < NB; i++) {
+                w[i] *= s_tau[i];
 #pragma unroll
-                for (int p = 0; p <= i; p++) x += s_T[p + NB * i] * w[p];
-                if (i < jb) Wp[i * nn + tid] = x;
+                for (int p = i + 1; p < NB; p++) w[p] = fma(-Wp[i * ncv + p], w[i], w[p]);
             }
+#pragma unroll
+            for (int i = 0; i < NB; i++) Wp[i * ncv + NB + tid] = w[i];
         }
         __syncthreads();
-        // C -= V W, four elements per thread at a time (independent chains)
         const int tot = rows * nc;
+        double *C = S + (size_t)sld * c0 + j0;
         for (int base = tid; base < tot; base += 4 * NT) {
             int rr[4], cl[4];
             double x[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int idx = min(base + u * NT, tot - 1);
-                rr[u] = j0 + idx % rows;
                 cl[u] = idx / rows;
-                x[u] = 0.0;
+                rr[u] = idx - cl[u] * rows;
+                x[u] = C[rr[u] + (size_t)sld * cl[u]];
             }
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                if (i < jb) {
-                    const int d = j0 + i;
+            for (int i = 0; i < NB; i++)
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const double v = rr[u] > d ? S[rr[u] + (size_t)sld * d] : (rr[u] == d ? 1.0 : 0.0);
-                        x[u] += v * Wp[i * nn + cl[u]];
-                    }
+                for (int u = 0; u < 4; u++) {
+                    const double v = rr[u] > i ? V[rr[u] + (size_t)sld * i] : (rr[u] == i ? 1.0 : 0.0);
+                    x[u] = fma(-v, Wp[i * ncv + NB + cl[u]], x[u]);
                 }
-            }
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (base + u * NT < tot) S[rr[u] + (size_t)sld * (c0 + cl[u])] -= x[u];
+                if (base + u * NT < tot) C[rr[u] + (size_t)sld * cl[u]] = x[u];
         }
         __syncthreads();
     }
 }
 
-// The instances list[0 .. cnt), all with n <= nmax, one CTA per instance at a
-// time.  One pass over A in CH2-row chunks (the next chunk is loaded into
-// registers while the current one is used) feeds both the FP32 Gram (4 x 4
-// register tiles) and the FP64 sketch.  The FP32 Gram is parked in the
-// instance's Gram block (as floats, ld nmax) while the sketch is factored,
-// then read back for the FP32 Cholesky.
-__global__ void __launch_bounds__(NT, 2) k_features(const BMInst *inst, const int *list, int cnt, int nmax, float *F)
+// The upper triangle of the nn x nn S <- its inverse, its diagonal already
+// inverted: halves of 2b columns by halves of b, X12 = -X11 (R12 X22), from b = 1
+// up.  Every level's entries are independent, so all threads work and a chain
+// is b terms long (column by column, a barrier and a chain for each: 0.50
+// million clocks at n = 119, 0.20 now).  R12 X22 goes to the lower triangle,
+// transposed.
+__device__ void tri_inv_halves(int nn, double *S, int sld)
 {
-    extern __shared__ __align__(16) uint8_t fsm[];
-    __shared__ double red[NT], red2[NT];
-    __shared__ int bad;
-    const int sld = sketch_ld(nmax);
-    const int tid = threadIdx.x;
-    double *SA = (double *)fsm;
-    double *c64 = SA + (size_t)sld * nmax;
-    float *c32 = (float *)(c64 + CH2 * LD2);
-    for (int li = blockIdx.x; li < cnt; li += gridDim.x) {
-        const int t = list[li];
-        const BMInst I = inst[t];
-        const int mm = I.m, nn = I.n, ns = min(2 * nn, SMAX);
-        const int nb = (nn + 3) >> 2, nblk = nb * (nb + 1) / 2;
-        const int chunk = CH2 * nn;
-        float acc[3][16];
-#pragma unroll
-        for (int q = 0; q < 3; q++)
-#pragma unroll
-            for (int e = 0; e < 16; e++) acc[q][e] = 0.0f;
-        for (int idx = tid; idx < sld * nn; idx += NT) SA[idx] = 0.0;
-        for (int idx = tid; idx < CH2 * LDC; idx += NT) c32[idx] = 0.0f;  // columns >= nn stay zero
-        double pf[8];
-        auto load = [&](int r0) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int idx = tid + k * NT;
-                const int r = idx % CH2, c = idx / CH2;
-                pf[k] = (idx < chunk && r0 + r < mm) ? I.A[(size_t)(r0 + r) + (size_t)c * I.lda] : 0.0;
-            }
-        };
-        load(0);
-        for (int r0 = 0; r0 < mm; r0 += CH2) {
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int idx = tid + k * NT;
-                if (idx < chunk) {
-                    const int r = idx % CH2, c = idx / CH2;
-                    c64[r * LD2 + c] = pf[k];
-                    c32[r * LDC + c] = (float)pf[k];
-                }
-            }
-            __syncthreads();
-            if (r0 + CH2 < mm) load(r0 + CH2);
-#pragma unroll
-            for (int q = 0; q < 3; q++) {
-                const int blk = tid + q * NT;
-                if (blk < nblk) {
-                    int bi, bj;
-                    tile_of(blk, bi, bj);
-#pragma unroll 4
-                    for (int r = 0; r < CH2; r++) {
-                        const float4 x = *(const float4 *)(c32 + r * LDC + 4 * bi);
-                        const float4 y = *(const float4 *)(c32 + r * LDC + 4 * bj);
-                        const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-                        for (int a = 0; a < 4; a++)
-#pragma unroll
-                            for (int b = 0; b < 4; b++) acc[q][4 * a + b] = fmaf(xs[a], ys[b], acc[q][4 * a + b]);
-                    }
-                }
-            }
-            if (tid < nn) {
-                const int c = tid;
-                for (int r = 0; r < CH2 && r0 + r < mm; r++) {
-                    const uint32_t h = mix32((uint32_t)(r0 + r) * 0x9E3779B9u + 0x3C6EF372u);
-                    const int b = (int)((h >> 1) % (uint32_t)ns);
-                    const double v = c64[r * LD2 + c];
-                    SA[b + sld * c] += (h & 1u) ? v : -v;
-                }
-            }
-        }
-        // park the FP32 Gram in the instance's Gram block
-        float *Gp = (float *)I.G;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const int blk = tid + q * NT;
-            if (blk < nblk) {
-                int bi, bj;
-                tile_of(blk, bi, bj);
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        const int i = 4 * bi + a, j = 4 * bj + b;
-                        if (i < nn && j < nn) Gp[i + nmax * j] = acc[q][4 * a + b];
-                    }
-            }
+    for (int bl = 0; (1 << bl) < nn; bl++) {
+        const int b = 1 << bl, pairs = (nn + 2 * b - 1) >> (bl + 1), total = pairs << (2 * bl);
+        for (int idx = threadIdx.x; idx < total; idx += NT) {
+            const int r0 = (idx >> (2 * bl)) << (bl + 1), c0 = r0 + b;
+            const int r = r0 + (idx & (b - 1)), c = c0 + ((idx >> bl) & (b - 1));
+            if (c >= nn) continue;
+            double s = 0.0;
+            for (int q = c0; q <= c; q++) s = fma(S[r + sld * q], S[q + sld * c], s);
+            S[c + sld * r] = s;
         }
         __syncthreads();
-        // ---- the sketch's R and its 1-norm condition number
-        house_qr(ns, nn, SA, sld, c64);
-        // ||R||_1 (column sums), then R^-1 in place (column j from the already
-        // inverted leading block, as dtrti2 does) and ||R^-1||_1
-        double cr = 0.0;
-        for (int c = threadIdx.x; c < nn; c += NT) {
-            double sum = 0.0;
-            for (int r = 0; r <= c; r++) sum += fabs(SA[r + sld * c]);
-            cr = fmax(cr, sum);
-        }
-        // R^-1 as bm::tri_inv_packed does it (one barrier per column, two
-        // lanes per row, the reciprocals of the diagonal formed once), unless
-        // a diagonal entry is zero or not finite
-        __shared__ double colb[2][128], rdg[128];
-        __shared__ int sing;
-        if (threadIdx.x == 0) sing = 0;
-        __syncthreads();
-        for (int r = threadIdx.x; r < nn; r += NT) {
-            const double d = SA[r + sld * r];
-            if (d == 0.0 || !isfinite(d)) sing = 1;
-            rdg[r] = 1.0 / d;
-        }
-        if (threadIdx.x == 0 && nn > 1) colb[1][0] = SA[sld];
-        __syncthreads();
-        if (!sing) {
-            for (int r = threadIdx.x; r < nn; r += NT) SA[r + sld * r] = rdg[r];
-            __syncthreads();
-            const int r = threadIdx.x >> 1, hb = threadIdx.x & 1;
-            for (int j = 1; j < nn; j++) {
-                const double *cj = colb[j & 1];
-                double v0 = 0.0, v1 = 0.0;
-                if (r < j) {
-                    int p = r + hb;
-                    for (; p + 2 < j; p += 4) {
-                        v0 = fma(SA[r + sld * p], cj[p], v0);
-                        v1 = fma(SA[r + sld * (p + 2)], cj[p + 2], v1);
-                    }
-                    if (p < j) v0 = fma(SA[r + sld * p], cj[p], v0);
-                }
-                double v = v0 + v1;
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                if (r < j && hb == 0) SA[r + sld * j] = -rdg[j] * v;
-                if (j + 1 < nn)
-                    for (int q = threadIdx.x; q <= j; q += NT) colb[(j + 1) & 1][q] = SA[q + sld * (j + 1)];
-                __syncthreads();
-            }
-        }
-        __syncthreads();
-        double ci = 0.0;
-        for (int c = threadIdx.x; c < nn; c += NT) {
-            double sum = 0.0;
-            for (int r = 0; r <= c; r++) sum += fabs(SA[r + sld * c]);
-            ci = fmax(ci, sum);
-        }
-        if (sing || !(ci <= 1e300)) ci = INFINITY;  // singular R: no finite estimate
-        red[threadIdx.x] = cr;
-        red2[threadIdx.x] = ci;
-        __syncthreads();
-        for (int o = NT / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) {
-                red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
-                red2[threadIdx.x] = fmax(red2[threadIdx.x], red2[threadIdx.x + o]);
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            const double k1 = red[0] * red2[0];
-            F[5 * t + 3] = (isfinite(k1) ? (float)fmin(log10(fmax(k1, 1.0)), 20.0) : 20.0f) / 10.0f;
-        }
-        __syncthreads();
-        // ---- the FP32 Gram back (upper triangle, ld nmax): norms and FP32 Cholesky
-        float *G = (float *)fsm;
-        const int ldg = nmax;
-        for (int c = tid >> 5; c < nn; c += NT / 32)
-            for (int r = tid & 31; r <= c; r += 32) G[r + ldg * c] = Gp[r + nmax * c];
-        __syncthreads();
-        if (tid == 0) {
-            float mx = 0.0f, mn = 3.4e38f;
-            for (int j = 0; j < nn; j++) {
-                const float v = sqrtf(fmaxf(G[j + ldg * j], 0.0f));
-                mx = fmaxf(mx, v);
-                mn = fminf(mn, v);
-            }
-            F[5 * t + 0] = log2f((float)mm) / 12.0f;
-            F[5 * t + 1] = log2f((float)nn) / 7.0f;
-            F[5 * t + 2] = mn > 0.0f ? fminf(log10f(mx / mn) / 4.0f, 4.0f) : 4.0f;
-            bad = 0;
-        }
-        __syncthreads();
-        for (int j = 0; j < nn; j++) {
-            if (tid < 32) {
-                float d = 0.0f;
-                for (int p = tid; p < j; p += 32) d += G[p + ldg * j] * G[p + ldg * j];
-                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-                if (tid == 0) {
-                    d = G[j + ldg * j] - d;
-                    if (!(d > 0.0f))
-                        bad = 1;
-                    else
-                        G[j + ldg * j] = sqrtf(d);
-                }
-            }
-            __syncthreads();
-            if (bad) break;
-            const float dj = G[j + ldg * j];
-            for (int c = j + 1 + tid; c < nn; c += NT) {
-                float v = G[j + ldg * c];
-                for (int p = 0; p < j; p++) v -= G[p + ldg * j] * G[p + ldg * c];
-                G[j + ldg * c] = v / dj;
-            }
-            __syncthreads();
-        }
-        if (tid == 0) {
-            float f4 = 2.0f;
-            if (!bad) {
-                float mx = 0.0f, mn = 3.4e38f;
-                for (int j = 0; j < nn; j++) {
-                    mx = fmaxf(mx, G[j + ldg * j]);
-                    mn = fminf(mn, G[j + ldg * j]);
-                }
-                f4 = fminf(log10f(mx / mn) / 3.0f, 2.0f);
-            }
-            F[5 * t + 4] = f4;
+        for (int idx = threadIdx.x; idx < total; idx += NT) {
+            const int r0 = (idx >> (2 * bl)) << (bl + 1), c0 = r0 + b;
+            const int r = r0 + ((idx >> bl) & (b - 1)), c = c0 + (idx & (b - 1));
+            if (c >= nn) continue;
+            double s = 0.0;
+            for (int q = r; q < c0; q++) s = fma(S[r + sld * q], S[c + sld * q], s);
+            S[r + sld * c] = -s;
         }
         __syncthreads();
     }
+}
+
+// The instances list[0 .. gridDim.x), all with n <= 32 NW, one CTA each.  One
+// pass over A in CH-row chunks (the next chunk is loaded into registers while
+// the current one is used) feeds both the FP32 Gram (4 x 4 register tiles) and
+// the FP64 sketch, whose buckets are shared out over the warps a column block
+// has.  The FP32 Gram is parked in the instance's Gram block (as floats, ld
+// NMAX) while the sketch is factored, then read back for the FP32 Cholesky.
+// The launches of a call are independent and chained: a class starts where the
+// one before leaves SMs free, and the last block of each waits for the launch
+// before, so that the last launch ends after all.  1,000 instances (n to 128,
+// m to 4,096): 11.55 -> 5.99 ms, of which the passes over A are about 2.3.
+template <int NW>
+__global__ void __launch_bounds__(NT, NW == 1 ? 3 : NW == 2 ? 2 : 1) k_features(const BMInst *inst, const int *list, float *F)
+{
+    using Z = Size<NW>;
+    constexpr int CH = Z::CH, TILES = (8 * NW) * (8 * NW + 1) / 2, Q = (TILES + NT - 1) / NT, PF = CH * Z::NMAX / NT;
+    extern __shared__ __align__(16) uint8_t fsm[];
+    __shared__ double red[NT], red2[NT], rdg[Z::NMAX];
+    __shared__ int bad, sing, s_b[CH];
+    constexpr int sld = Z::SLD;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double *SA = (double *)fsm;
+    double *c64 = SA + (size_t)sld * Z::NMAX;
+    float *c32 = (float *)(c64 + CH * Z::LD64);
+    chain_open();
+    const int t = list[blockIdx.x];
+    const BMInst I = inst[t];
+    const int mm = I.m, nn = I.n, ns = min(2 * nn, SMAX);
+    const int nb = (nn + 3) >> 2, nblk = nb * (nb + 1) / 2;
+    const int chunk = CH * nn;
+    float acc[Q][16];
+    int xo[Q], yo[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        int bi = 0, bj = 0;
+        if (tid + q * NT < nblk) tile_of(tid + q * NT, bi, bj);
+        xo[q] = 4 * bi;
+        yo[q] = 4 * bj;
+#pragma unroll
+        for (int e = 0; e < 16; e++) acc[q][e] = 0.0f;
+    }
+    for (int idx = tid; idx < sld * nn; idx += NT) SA[idx] = 0.0;
+    for (int idx = tid; idx < CH * Z::LD32; idx += NT) c32[idx] = 0.0f;  // columns >= nn stay zero
+    double pf[PF];
+    auto load = [&](int r0) {
+#pragma unroll
+        for (int k = 0; k < PF; k++) {
+            const int idx = tid + k * NT;
+            const int r = idx % CH, c = idx / CH;
+            pf[k] = (idx < chunk && r0 + r < mm) ? I.A[(size_t)(r0 + r) + (size_t)c * I.lda] : 0.0;
+        }
+    };
+    // buckets = bgrp modulo `groups` are this warp's, for the columns 32 cblk ..
+    constexpr int groups = 8 / NW;  // a power of two (NW = 3: two warps have none)
+    const int cblk = warp % NW, bgrp = warp / NW;
+    const int sc = 32 * cblk + lane;
+    load(0);
+    for (int r0 = 0; r0 < mm; r0 += CH) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PF; k++) {
+            const int idx = tid + k * NT;
+            if (idx < chunk) {
+                const int r = idx % CH, c = idx / CH;
+                c64[r * Z::LD64 + c] = pf[k];
+                c32[r * Z::LD32 + c] = (float)pf[k];
+            }
+        }
+        if (tid < CH) {
+            const uint32_t h = mix32((uint32_t)(r0 + tid) * 0x9E3779B9u + 0x3C6EF372u);
+            s_b[tid] = r0 + tid < mm ? (int)(2 * ((h >> 1) % (uint32_t)ns) + (h & 1u)) : -1;
+        }
+        __syncthreads();
+        if (r0 + CH < mm) load(r0 + CH);
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            if (tid + q * NT < nblk) {
+#pragma unroll 4
+                for (int r = 0; r < CH; r++) {
+                    const float4 x = *(const float4 *)(c32 + r * Z::LD32 + xo[q]);
+                    const float4 y = *(const float4 *)(c32 + r * Z::LD32 + yo[q]);
+                    const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for (int a = 0; a < 4; a++)
+#pragma unroll
+                        for (int b = 0; b < 4; b++) acc[q][4 * a + b] = fmaf(xs[a], ys[b], acc[q][4 * a + b]);
+                }
+            }
+        }
+        // this warp's rows in order, two at a time: their sums are independent
+        // unless they share a bucket
+        if (bgrp < groups) {
+#pragma unroll
+            for (int r32 = 0; r32 < CH; r32 += 32) {
+                const int mine = r32 + lane < CH ? s_b[r32 + lane] : -1;
+                unsigned todo = __ballot_sync(0xffffffffu, mine >= 0 && ((mine >> 1) & (groups - 1)) == bgrp);
+                while (todo) {
+                    const int p = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int q = todo ? __ffs(todo) - 1 : p;
+                    todo &= todo - 1;
+                    const int bp = __shfl_sync(0xffffffffu, mine, p), bq = __shfl_sync(0xffffffffu, mine, q);
+                    if (sc < nn) {
+                        double *ap = SA + (bp >> 1) + sld * sc, *aq = SA + (bq >> 1) + sld * sc;
+                        const double vp = flip(c64[(r32 + p) * Z::LD64 + sc], bp), vq = flip(c64[(r32 + q) * Z::LD64 + sc], bq);
+                        if (p == q) {
+                            *ap += vp;
+                        } else if (ap == aq) {
+                            *ap = (*ap + vp) + vq;
+                        } else {
+                            const double x = *ap, y = *aq;
+                            *ap = x + vp;
+                            *aq = y + vq;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    // park the FP32 Gram in the instance's Gram block
+    float *Gp = (float *)I.G;
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        if (tid + q * NT < nblk) {
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const int i = xo[q] + a, j = yo[q] + b;
+                    if (i < nn && j < nn) Gp[i + Z::NMAX * j] = acc[q][4 * a + b];
+                }
+        }
+    }
+    __syncthreads();
+    // ---- the sketch's R and its 1-norm condition number
+    house_qr<Z::RPL>(ns, nn, SA, sld, c64);
+    // ||R||_1 (column sums), then R^-1 in place and ||R^-1||_1, unless a
+    // diagonal entry is zero or not finite
+    double cr = 0.0;
+    for (int c = tid; c < nn; c += NT) {
+        double sum = 0.0;
+        for (int r = 0; r <= c; r++) sum += fabs(SA[r + sld * c]);
+        cr = fmax(cr, sum);
+    }
+    if (tid == 0) sing = 0;
+    __syncthreads();
+    for (int r = tid; r < nn; r += NT) {
+        const double d = SA[r + sld * r];
+        if (d == 0.0 || !isfinite(d)) sing = 1;
+        rdg[r] = 1.0 / d;
+    }
+    __syncthreads();
+    if (!sing) {
+        for (int r = tid; r < nn; r += NT) SA[r + sld * r] = rdg[r];
+        __syncthreads();
+        tri_inv_halves(nn, SA, sld);
+    }
+    double ci = 0.0;
+    for (int c = tid; c < nn; c += NT) {
+        double sum = 0.0;
+        for (int r = 0; r <= c; r++) sum += fabs(SA[r + sld * c]);
+        ci = fmax(ci, sum);
+    }
+    if (sing || !(ci <= 1e300)) ci = INFINITY;  // singular R: no finite estimate
+    red[tid] = cr;
+    red2[tid] = ci;
+    __syncthreads();
+    for (int o = NT / 2; o > 0; o >>= 1) {
+        if (tid < o) {
+            red[tid] = fmax(red[tid], red[tid + o]);
+            red2[tid] = fmax(red2[tid], red2[tid + o]);
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        const double k1 = red[0] * red2[0];
+        F[5 * t + 3] = (isfinite(k1) ? (float)fmin(log10(fmax(k1, 1.0)), 20.0) : 20.0f) / 10.0f;
+    }
+    // ---- the FP32 Gram back (upper triangle, ld GLD, odd): norms and FP32
+    // Cholesky by rows, every entry's terms in row order; the pivot's sum of
+    // squares is formed anew from its column
+    float *G = (float *)fsm;
+    constexpr int ldg = Z::GLD;
+    for (int c = warp; c < nn; c += NT / 32)
+        for (int r = lane; r <= c; r += 32) G[r + ldg * c] = Gp[r + Z::NMAX * c];
+    if (tid == 0) bad = 0;
+    __syncthreads();
+    auto diag_range = [&](bool root, float &mx, float &mn) {
+        mx = 0.0f;
+        mn = 3.4e38f;
+        for (int j = lane; j < nn; j += 32) {
+            const float v = root ? sqrtf(fmaxf(G[j + ldg * j], 0.0f)) : G[j + ldg * j];
+            mx = fmaxf(mx, v);
+            mn = fminf(mn, v);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        }
+    };
+    float mx, mn;
+    if (warp == 0) {
+        diag_range(true, mx, mn);
+        if (lane == 0) {
+            F[5 * t + 0] = log2f((float)mm) / 12.0f;
+            F[5 * t + 1] = log2f((float)nn) / 7.0f;
+            F[5 * t + 2] = mn > 0.0f ? fminf(log10f(mx / mn) / 4.0f, 4.0f) : 4.0f;
+        }
+    }
+    __syncthreads();
+    for (int j = 0; j < nn; j++) {
+        if (warp == 0) {
+            float d = 0.0f;
+            for (int p = lane; p < j; p += 32) d += G[p + ldg * j] * G[p + ldg * j];
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if (lane == 0) {
+                d = G[j + ldg * j] - d;
+                if (!(d > 0.0f))
+                    bad = 1;
+                else
+                    G[j + ldg * j] = sqrtf(d);
+            }
+        }
+        __syncthreads();
+        if (bad) break;
+        const float dj = G[j + ldg * j];
+        for (int c = j + 1 + tid; c < nn; c += NT) G[j + ldg * c] = G[j + ldg * c] / dj;
+        __syncthreads();
+        for (int r = j + 1 + warp; r < nn; r += NT / 32) {
+            const float x = G[j + ldg * r];
+            for (int c = r + 1 + lane; c < nn; c += 32) G[r + ldg * c] -= x * G[j + ldg * c];
+        }
+        // the next pivot's column (rows <= j) is complete; its row's updates are
+        // seen after the barrier that follows the pivot
+    }
+    if (warp == 0) {
+        float f4 = 2.0f;
+        if (!bad) {
+            diag_range(false, mx, mn);
+            f4 = fminf(log10f(mx / mn) / 3.0f, 2.0f);
+        }
+        if (lane == 0) F[5 * t + 4] = f4;
+    }
+    if (blockIdx.x == gridDim.x - 1) chain_wait();
+}
+
+// One class's launch; the first of a call is an ordinary one.
+template <int NW>
+static void launch_features(const BMInst *inst, const int *list, int cnt, float *F, bool chained)
+{
+    constexpr int bytes = (int)Size<NW>::BYTES;
+    cudaFuncSetAttribute(k_features<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    trace_begin();
+    if (chained)
+        launch_chained(k_features<NW>, dim3(cnt), NT, bytes, inst, list, F);
+    else
+        k_features<NW><<<cnt, NT, bytes, stream()>>>(inst, list, F);
+    note_launch("gels_features");
 }
 
 }  // namespace feat
@@ -1387,7 +1486,9 @@ int lila_gels_mixed_features(void *handle, float *F)
     // instances the mixed variants cannot take keep zero features (the
     // solve routes them to the FP64 solver whatever the selector says); the
     // others run one launch per size class (n <= 32, 64, 96, 128) with that
-    // class's shared memory, so that small instances share an SM
+    // class's shared memory, so that small instances share an SM; the largest
+    // class and the longest instances of each first, so that the short ones fill
+    // the SMs at the end
     cudaStream_t st = lg::stream();
     cudaMemsetAsync(F, 0, sizeof(float) * 5 * (size_t)H->count, st);
     std::vector<int> order;
@@ -1396,25 +1497,22 @@ int lila_gels_mixed_features(void *handle, float *F)
     const int ne = (int)order.size();
     if (ne == 0) return 0;
     auto cls = [&](int t) { return (H->h[t].n - 1) >> 5; };
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cls(a) < cls(b); });
+    // per row about 3 n clocks of the pass, then about 1.2 n^3 / 3 (n to 128) for the sketch
+    auto cost = [&](int t) {
+        const long long n = H->h[t].n;
+        return n * (3LL * H->h[t].m + 100 * n);
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return cls(a) != cls(b) ? cls(a) > cls(b) : cost(a) > cost(b);
+    });
     cudaMemcpyAsync(H->d_list, order.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, st);
-    cudaFuncSetAttribute(feat::k_features, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)feat::smem_bytes(BM_NMAX));
     for (int a = 0; a < ne;) {
         int b = a;
         while (b < ne && cls(order[b]) == cls(order[a])) b++;
-        const int nmax = 32 * (cls(order[a]) + 1);
-        const size_t sm = feat::smem_bytes(nmax);
-        int per_sm = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, feat::k_features, feat::NT, sm) != cudaSuccess ||
-            per_sm < 1) {
-            cudaGetLastError();
-            per_sm = 1;
-        }
-        const int grid = std::min(b - a, per_sm * sm_count());
-        trace_begin();
-        feat::k_features<<<grid, feat::NT, sm, st>>>(H->d_inst, H->d_list + a, b - a, nmax, F);
-        note_launch("gels_features");
+        const int c = cls(order[a]);
+        (c == 0 ? feat::launch_features<1> : c == 1 ? feat::launch_features<2> : c == 2 ? feat::launch_features<3>
+                                                                                       : feat::launch_features<4>)(
+            H->d_inst, H->d_list + a, b - a, F, a > 0);
         a = b;
     }
     return 0;

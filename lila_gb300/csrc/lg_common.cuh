@@ -256,9 +256,10 @@ int mixed_leaf_entry(int m, int n, int i, int mt, double *A, int lda, double *T,
 // Programmatic dependent launch of the chains of small kernels: a kernel
 // launched by launch_chained may be placed on the SMs while the one before it
 // drains, and waits in chain_wait (before its first read or write of global
-// memory) until that one has completed.  chain_open lets the next one in once every
-// block has come to it or ended.  691 such launches of a 1413 x 692 recursive QR:
-// 10.03 -> 8.12 ms, with the fused reduction of gemm_times_tri.  Both do nothing in a kernel launched otherwise.
+// memory) until that one has completed.  chain_open lets the next one in once
+// every block has come to it or ended.  691 such launches of a 1413 x 692 recursive QR:
+// 10.03 -> 8.12 ms, with the fused reduction of gemm_times_tri.  Both do
+// nothing in a kernel launched otherwise.
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
