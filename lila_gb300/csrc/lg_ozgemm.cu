@@ -1200,11 +1200,29 @@ __global__ void __launch_bounds__(GW_NT, 1) k_gram_w(const GramW *jobs, int njob
             }
         };
         int last_commit = -1;
+        // Adds the window that ends with stage `last` up, once that stage's MMAs
+        // (and so all before) are complete.  Called after the next window's first
+        // stage has been split: the tensor core runs meanwhile (with the fold at the
+        // window's own end the two Gram kernels took 9.32 ms on 2,000 instances, 8.57
+        // now).
+        auto fold = [&](int last) {
+            if (!tc::wait_abort_warp(&empty_b[last & 1], (last >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) return false;
+            tc::fence_after_sync();
+            flush_acc(tbase, q, h, acc_hi, acc_lo);
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tfree);
+            return true;
+        };
+        bool ok_all = nch > 0;
         load_stage(0);
         for (int ch = 0; ch < nch; ch++) {
             const int buf = ch & 1;
             // the buffer's previous stage (ch - 2) has been read by the tensor core
-            if (ch >= NSTAGE && !tc::wait_abort_warp(&empty_b[buf], ((ch - NSTAGE) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) break;
+            if (ch >= NSTAGE && !tc::wait_abort_warp(&empty_b[buf], ((ch - NSTAGE) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) {
+                ok_all = false;
+                break;
+            }
             uint8_t *stA = smem + (size_t)buf * STAGE_BYTES;
             uint8_t *stB = stA + A_BYTES;
             const int k0 = ch * KC;
@@ -1238,6 +1256,10 @@ __global__ void __launch_bounds__(GW_NT, 1) k_gram_w(const GramW *jobs, int njob
             tc::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&full_b[buf]);
+            if (ch > 0 && ch % FLUSH == 0 && !fold(ch - 1)) {
+                ok_all = false;
+                break;
+            }
             if (warp == GW_ISSUER && lane == 0) {
                 bool ok = tc::wait_abort(&full_b[buf], (ch >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
                 const bool window_start = (ch % FLUSH) == 0;
@@ -1265,17 +1287,12 @@ __global__ void __launch_bounds__(GW_NT, 1) k_gram_w(const GramW *jobs, int njob
                     last_commit = ch;
                 }
             }
-            if (__any_sync(0xffffffffu, *s_abort)) break;
-            if (((ch + 1) % FLUSH) == 0 || ch == nch - 1) {
-                // every MMA of the window is complete once this stage's commit is
-                if (!tc::wait_abort_warp(&empty_b[buf], (ch >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) break;
-                tc::fence_after_sync();
-                flush_acc(tbase, q, h, acc_hi, acc_lo);
-                tc::fence_before_sync();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&tfree);
+            if (__any_sync(0xffffffffu, *s_abort)) {
+                ok_all = false;
+                break;
             }
         }
+        if (ok_all) fold(nch - 1);
         // after an abort the issuer's last MMAs may still run: wait (bounded)
         // for its last commit before the accumulators are released
         if (last_commit >= 0) tc::mbar_wait(&empty_b[last_commit & 1], (last_commit >> 1) & 1);
@@ -1376,13 +1393,55 @@ __global__ void __launch_bounds__(OZT, 1) k_gram_stacked(const GramW *jobs, int 
         };
         const bool issuer = warp == OZT / 32 - 1 && lane == 0;
         int last_commit = -1;
+        // as in k_gram_w: a window is added up after the next one's first stage is split
+        auto fold = [&](int last) {
+            if (!tc::wait_abort_warp(&empty_b[last % GS_STAGES], (last / GS_STAGES) & 1, s_abort, status,
+                                     ST_WAIT_TIMEOUT))
+                return false;
+            tc::fence_after_sync();
+            // top lanes: order d in block d; bottom lanes: order d in
+            // block d - 1 (their order 0 is absent: a zero word)
+#pragma unroll
+            for (int hc = 0; hc < 2; hc++)
+#pragma unroll
+                for (int g4 = 0; g4 < 2; g4++) {
+                    uint32_t v[4][8];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int d = 4 * g4 + e;
+                        const int blk = top ? d : d - 1;
+                        if (blk >= 0)
+                            tc::tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * blk + 16 * h + 8 * hc),
+                                         v[e]);
+                        else
+#pragma unroll
+                            for (int j = 0; j < 8; j++) v[e][j] = 0u;
+                    }
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const long long x = oz::combine4(v[0][j], v[1][j], v[2][j], v[3][j]);
+                        if (g4 == 0)
+                            acc_hi[8 * hc + j] += x;
+                        else
+                            acc_lo[8 * hc + j] += x;
+                    }
+                }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tfree);
+            return true;
+        };
+        bool ok_all = nch > 0;
         load_stage(0);
         for (int ch = 0; ch < nch; ch++) {
             const int buf = ch % GS_STAGES;
             if (ch >= GS_STAGES &&
                 !tc::wait_abort_warp(&empty_b[buf], ((ch - GS_STAGES) / GS_STAGES) & 1, s_abort, status,
-                                     ST_WAIT_TIMEOUT))
+                                     ST_WAIT_TIMEOUT)) {
+                ok_all = false;
                 break;
+            }
             uint8_t *stg = smem + (size_t)buf * GS_STAGE_BYTES;
             {
                 uint32_t w01[NS], w23[NS];
@@ -1394,6 +1453,10 @@ __global__ void __launch_bounds__(OZT, 1) k_gram_stacked(const GramW *jobs, int 
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&full_b[buf]);
             const bool window_start = (ch % FLUSH) == 0;
+            if (ch > 0 && ch % FLUSH == 0 && !fold(ch - 1)) {
+                ok_all = false;
+                break;
+            }
             if (issuer) {
                 bool ok = tc::wait_abort(&full_b[buf], (ch / GS_STAGES) & 1, s_abort, status, ST_WAIT_TIMEOUT);
                 if (ok && window_start && ch > 0)
@@ -1420,44 +1483,12 @@ __global__ void __launch_bounds__(OZT, 1) k_gram_stacked(const GramW *jobs, int 
                     last_commit = ch;
                 }
             }
-            if (__any_sync(0xffffffffu, *s_abort)) break;
-            if (((ch + 1) % FLUSH) == 0 || ch == nch - 1) {
-                if (!tc::wait_abort_warp(&empty_b[buf], (ch / GS_STAGES) & 1, s_abort, status, ST_WAIT_TIMEOUT))
-                    break;
-                tc::fence_after_sync();
-                // top lanes: order d in block d; bottom lanes: order d in
-                // block d - 1 (their order 0 is absent: a zero word)
-#pragma unroll
-                for (int hc = 0; hc < 2; hc++)
-#pragma unroll
-                    for (int g4 = 0; g4 < 2; g4++) {
-                        uint32_t v[4][8];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int d = 4 * g4 + e;
-                            const int blk = top ? d : d - 1;
-                            if (blk >= 0)
-                                tc::tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * blk + 16 * h + 8 * hc),
-                                             v[e]);
-                            else
-#pragma unroll
-                                for (int j = 0; j < 8; j++) v[e][j] = 0u;
-                        }
-                        tc::tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const long long x = oz::combine4(v[0][j], v[1][j], v[2][j], v[3][j]);
-                            if (g4 == 0)
-                                acc_hi[8 * hc + j] += x;
-                            else
-                                acc_lo[8 * hc + j] += x;
-                        }
-                    }
-                tc::fence_before_sync();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&tfree);
+            if (__any_sync(0xffffffffu, *s_abort)) {
+                ok_all = false;
+                break;
             }
         }
+        if (ok_all) fold(nch - 1);
         if (last_commit >= 0) tc::mbar_wait(&empty_b[last_commit % GS_STAGES], (last_commit / GS_STAGES) & 1);
     }
     __syncthreads();
@@ -1633,23 +1664,64 @@ __global__ void __launch_bounds__(OZT, 1) k_map_items(const MapItem *items, int 
             }
             if (st == 0) rx = live ? J.rexp[grow] : 0;
         };
-        load(0, 0);
-        for (int tile = 0; tile < ntiles; tile++) {
-            const int row0 = tile * BM;
-            const int rr = 32 * q + lane, grow_e = row0 + rr;
-            const int er = grow_e < J.m ? J.rexp[grow_e] : 0;  // in flight during the stages
-            const int emax = rx;  // loaded with this tile's first stage
-            long long acc_hi[16], acc_lo[16];
+        long long acc_hi[16], acc_lo[16];
+        // A tile's MMAs end with stage `last`; they are added up after the next
+        // tile's first stage has been split, so the tensor core runs meanwhile,
+        // and its outputs are written after that stage's MMAs have been issued
+        // (folded at the tile's own end: 2,000 instances 5.65 ms, 4.88 now).
+        auto fold = [&](int last) {
+            if (!tc::wait_abort_warp(&empty_b[last & 1], (last >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) return false;
+            tc::fence_after_sync();
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 acc_hi[j] = 0;
                 acc_lo[j] = 0;
             }
+            flush_acc(tbase, q, h, acc_hi, acc_lo);
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tfree);
+            W++;
+            return true;
+        };
+        // TMEM lane 32 q + lane = output row, columns 16 h + j of the block
+        auto store = [&](int tile, int er) {
+            const int grow_e = tile * BM + 32 * q + lane;
+            if (grow_e < J.m && er) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int c = 16 * h + j;
+                    if (c >= J.ncols) continue;
+                    const int ec = s_cexp[c];
+                    double v;
+                    if (er == 0x7FF || ec == 0x7FF)
+                        v = __longlong_as_double(0x7FF8000000000000ll);
+                    else
+                        v = ec ? oz::assemble_fast(acc_hi[j], acc_lo[j], (er - 1022) + (ec - 1022) - 63) : 0.0;
+                    J.out[(size_t)grow_e + (size_t)(J.col0 + c) * J.ldo] = v;
+                }
+            } else if (grow_e < J.m) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int c = 16 * h + j;
+                    if (c < J.ncols) J.out[(size_t)grow_e + (size_t)(J.col0 + c) * J.ldo] = 0.0;
+                }
+            }
+        };
+        int er_prev = 0;
+        bool ok_all = ntiles > 0;
+        load(0, 0);
+        for (int tile = 0; tile < ntiles && ok_all; tile++) {
+            const int grow_e = tile * BM + 32 * q + lane;
+            const int er = grow_e < J.m ? J.rexp[grow_e] : 0;  // in flight during the stages
+            const int emax = rx;  // loaded with this tile's first stage
             for (int st = 0; st < nst; st++, G++) {
                 const int buf = G & 1;
                 if (G >= 2 &&
-                    !tc::wait_abort_warp(&empty_b[buf], ((G - 2) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT))
+                    !tc::wait_abort_warp(&empty_b[buf], ((G - 2) >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) {
+                    ok_all = false;
                     break;
+                }
                 {
                     uint32_t w01[NS], w23[NS];
                     digits4(ra, emax, w01, w23);
@@ -1666,6 +1738,10 @@ __global__ void __launch_bounds__(OZT, 1) k_map_items(const MapItem *items, int 
                 tc::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&full_b[buf]);
+                if (st == 0 && tile > 0 && !fold(G - 1)) {
+                    ok_all = false;
+                    break;
+                }
                 if (issuer) {
                     bool ok = tc::wait_abort(&full_b[buf], (G >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
                     if (ok && st == 0 && W > 0) ok = tc::wait_abort(&tfree, (W - 1) & 1, s_abort, status, ST_WAIT_TIMEOUT);
@@ -1690,41 +1766,15 @@ __global__ void __launch_bounds__(OZT, 1) k_map_items(const MapItem *items, int 
                         last_commit = G;
                     }
                 }
-                if (__any_sync(0xffffffffu, *s_abort)) break;
-                if (st + 1 == nst) {
-                    // the tile's last commit covers all its MMAs
-                    if (!tc::wait_abort_warp(&empty_b[buf], (G >> 1) & 1, s_abort, status, ST_WAIT_TIMEOUT)) break;
-                    tc::fence_after_sync();
-                    flush_acc(tbase, q, h, acc_hi, acc_lo);
-                    tc::fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) tc::mbar_arrive(&tfree);
+                if (__any_sync(0xffffffffu, *s_abort)) {
+                    ok_all = false;
+                    break;
                 }
+                if (st == 0 && tile > 0) store(tile - 1, er_prev);
             }
-            if (__any_sync(0xffffffffu, *s_abort)) break;
-            W++;
-            // epilogue: TMEM lane rr = output row, columns 16 h + j of the block
-            if (grow_e < J.m && er) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int c = 16 * h + j;
-                    if (c >= J.ncols) continue;
-                    const int ec = s_cexp[c];
-                    double v;
-                    if (er == 0x7FF || ec == 0x7FF)
-                        v = __longlong_as_double(0x7FF8000000000000ll);
-                    else
-                        v = ec ? oz::assemble_fast(acc_hi[j], acc_lo[j], (er - 1022) + (ec - 1022) - 63) : 0.0;
-                    J.out[(size_t)grow_e + (size_t)(J.col0 + c) * J.ldo] = v;
-                }
-            } else if (grow_e < J.m) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int c = 16 * h + j;
-                    if (c < J.ncols) J.out[(size_t)grow_e + (size_t)(J.col0 + c) * J.ldo] = 0.0;
-                }
-            }
+            er_prev = er;
         }
+        if (ok_all && fold(G - 1)) store(ntiles - 1, er_prev);
     }
     // after an abort the issuer's last MMAs may still run: wait (bounded)
     if (last_commit >= 0) tc::mbar_wait(&empty_b[last_commit & 1], (last_commit >> 1) & 1);
