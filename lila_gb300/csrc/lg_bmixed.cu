@@ -71,11 +71,14 @@ __device__ __forceinline__ double warp_sum(double v)
 // Upper Cholesky of the packed n x n S in place, right-looking with the
 // pivot one step ahead (as the tall leaf's factor pass): in step j warp 0
 // applies row j of R to row j + 1, takes that row's pivot (its 1 / sqrt by
-// rsqrt_nr) and scales the row, while the warps of the other three SM
-// sub-partitions (warp % 4 != 0) apply row j to rows j + 2 .. n - 1, one
-// element of the trailing triangle per thread and step; a step ends with one
-// block barrier.  False on a non-positive pivot (the pivot is then replaced
-// by 1 so that the factor stays finite).
+// rsqrt_nr) and scales the row, while the other seven warps apply row j to rows
+// j + 2 .. n - 1, one element of the trailing triangle per thread and step; a
+// step ends with one block barrier.  The FP64 instructions of the updates bound
+// it when several CTAs share an SM, so all lanes have an element (a column per
+// warp leaves a quarter of them empty: k_factor 2.81 -> 4.5 ms on 2,000
+// instances) and warp 4 helps on the pivot's sub-partition (2.99 without it).
+// False on a non-positive pivot (the pivot is then replaced by 1 so that the
+// factor stays finite).
 __device__ bool chol_packed(int n, double *S)
 {
     __shared__ int bad;
@@ -86,7 +89,8 @@ __device__ bool chol_packed(int n, double *S)
     // j + lane + 32 q), factored and scaled
     auto pivot_row = [&](int j, const double (&v)[4]) {
         double d = __shfl_sync(0xffffffffu, v[0], 0);
-        if (!(d > 0.0) || !isfinite(d)) {
+        const long long db = __double_as_longlong(d);
+        if (db <= 0 || db >= 0x7FF0000000000000LL) {  // not a positive finite number
             if (lane == 0) bad = 1;
             d = 1.0;
         }
@@ -118,12 +122,12 @@ __device__ bool chol_packed(int n, double *S)
                 v[q] = c < n ? fma(-a, S[pk(j, c)], S[pk(j + 1, c)]) : 0.0;
             }
             pivot_row(j + 1, v);
-        } else if (warp & 3) {
+        } else {
             // rows p = j + 2 .. n - 1: element e = cc (cc + 1) / 2 + q of the
             // trailing upper triangle (columns cc = 0 .. w - 1, rows q <= cc, offset j + 2)
-            const int wid = warp - (warp >> 2) - 1;  // 0 .. 5
+            const int wid = warp - 1;
             const int w = n - j - 2, tot = w * (w + 1) / 2;
-            for (int e = wid * 32 + lane; e < tot; e += 192) {
+            for (int e = wid * 32 + lane; e < tot; e += 224) {
                 int cc = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
                 if (cc * (cc + 1) / 2 > e) cc--;
                 if ((cc + 1) * (cc + 2) / 2 <= e) cc++;
@@ -137,38 +141,69 @@ __device__ bool chol_packed(int n, double *S)
     return bad == 0;
 }
 
-// S := S^-1 in place for the packed upper n x n S (n <= 128; column j from
-// the already inverted leading block, as LAPACK's dtrti2:
-// X(r, j) = -(sum_{p=r}^{j-1} X(r, p) R(p, j)) / R(j, j)).  The reciprocals
-// of the diagonal are formed once into the shared rd (BM_LD doubles) and
-// written over the diagonal first; two lanes share each row's dot product
-// (even and odd p, two accumulators each); the next column of R is copied
-// aside while the current one is formed, so a column costs one barrier.
+// S := S^-1 in place for the packed upper n x n S (n <= 128).  The reciprocals
+// of the diagonal are formed once into the shared rd (BM_LD doubles) and written
+// over the diagonal; then halves of 2b columns by halves of b, X12 = -X11 (R12
+// X22), from b = 1 up: a level's entries are independent (n b / 2 of them, at
+// most 16 per thread, kept in registers until all have been formed).  One column
+// at a time, a barrier and a chain for each: k_factor 3.87 ms on 2,000
+// instances, 2.98 by halves.
 __device__ void tri_inv_packed(int n, double *S, double *rd)
 {
-    __shared__ double colb[2][BM_LD];
     for (int r = threadIdx.x; r < n; r += NT) rd[r] = 1.0 / S[pk(r, r)];
-    if (threadIdx.x == 0 && n > 1) colb[1][0] = S[pk(0, 1)];
     __syncthreads();
     for (int r = threadIdx.x; r < n; r += NT) S[pk(r, r)] = rd[r];
     __syncthreads();
-    const int r = threadIdx.x >> 1, hb = threadIdx.x & 1;
-    for (int j = 1; j < n; j++) {
-        const double *cj = colb[j & 1];
-        double v0 = 0.0, v1 = 0.0;
-        if (r < j) {
-            int p = r + hb;
-            for (; p + 2 < j; p += 4) {
-                v0 = fma(S[pk(r, p)], cj[p], v0);
-                v1 = fma(S[pk(r, p + 2)], cj[p + 2], v1);
+    for (int bl = 0; (1 << bl) < n; bl++) {
+        const int b = 1 << bl, total = ((n + 2 * b - 1) >> (bl + 1)) << (2 * bl);
+        double y[16];
+        // R12 X22, rows over the lanes
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+            const int idx = threadIdx.x + u * NT;
+            if (u * NT >= total) continue;
+            const int r0 = (idx >> (2 * bl)) << (bl + 1), c0 = r0 + b;
+            const int r = r0 + (idx & (b - 1)), c = c0 + ((idx >> bl) & (b - 1));
+            double v = 0.0;
+            if (idx < total && c < n) {
+                const double *x = S + pk(0, c);
+                for (int q = c0, o = pk(r, c0); q <= c; o += ++q) v = fma(S[o], x[q], v);
             }
-            if (p < j) v0 = fma(S[pk(r, p)], cj[p], v0);
+            y[u] = v;
         }
-        double v = v0 + v1;
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if (r < j && hb == 0) S[pk(r, j)] = -rd[j] * v;
-        if (j + 1 < n)
-            for (int q = threadIdx.x; q <= j; q += NT) colb[(j + 1) & 1][q] = S[pk(q, j + 1)];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+            const int idx = threadIdx.x + u * NT;
+            if (u * NT >= total) continue;
+            const int r0 = (idx >> (2 * bl)) << (bl + 1);
+            const int r = r0 + (idx & (b - 1)), c = r0 + b + ((idx >> bl) & (b - 1));
+            if (idx < total && c < n) S[pk(r, c)] = y[u];
+        }
+        __syncthreads();
+        // -X11 (R12 X22), columns over the lanes
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+            const int idx = threadIdx.x + u * NT;
+            if (u * NT >= total) continue;
+            const int r0 = (idx >> (2 * bl)) << (bl + 1), c0 = r0 + b;
+            const int r = r0 + ((idx >> bl) & (b - 1)), c = c0 + (idx & (b - 1));
+            double v = 0.0;
+            if (idx < total && c < n) {
+                const double *x = S + pk(0, c);
+                for (int q = r, o = pk(r, r); q < c0; o += ++q) v = fma(S[o], x[q], v);
+            }
+            y[u] = -v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 16; u++) {
+            const int idx = threadIdx.x + u * NT;
+            if (u * NT >= total) continue;
+            const int r0 = (idx >> (2 * bl)) << (bl + 1);
+            const int r = r0 + ((idx >> bl) & (b - 1)), c = r0 + b + (idx & (b - 1));
+            if (idx < total && c < n) S[pk(r, c)] = y[u];
+        }
         __syncthreads();
     }
 }
@@ -223,20 +258,32 @@ __device__ void store_packed(int n, const double *S, double *D, int ldd, bool ze
 }
 
 // y := R^-T y (forward substitution) for the packed upper R, one right-hand
-// side (ld BM_LD in y) per warp; rd holds 1 / R(r, r).
+// side (ld BM_LD in y) per warp, four entries per lane in registers: entry r is
+// finished, sent to all lanes and taken out of the later ones (a chain of three
+// FP64 operations per entry instead of a dot product and its reduction); rd
+// holds 1 / R(r, r).
 __device__ void solve_rt(int n, const double *S, const double *rd, double *y, int nrhs)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int j = warp; j < nrhs; j += NT / 32) {
         double *yj = y + BM_LD * j;
-        for (int r = 0; r < n; r++) {
-            const double *sr = S + pk(0, r);
-            double s = 0.0;
-            for (int p = lane; p < r; p += 32) s += sr[p] * yj[p];
-            s = warp_sum(s);
-            if (lane == 0) yj[r] = (yj[r] - s) * rd[r];
-            __syncwarp();
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = lane + 32 * q < n ? yj[lane + 32 * q] : 0.0;
+#pragma unroll
+        for (int q0 = 0; q0 < 4; q0++) {
+            const int re = min(n, 32 * (q0 + 1));
+            for (int r = 32 * q0; r < re; r++) {
+                const double z = __shfl_sync(0xffffffffu, v[q0], r & 31) * rd[r];
+                if (lane == (r & 31)) yj[r] = z;
+#pragma unroll
+                for (int q = q0; q < 4; q++) {
+                    const int p = lane + 32 * q;
+                    if (32 * q < n && 32 * q + 31 > r) v[q] = fma(p > r && p < n ? -S[pk(r, p)] : 0.0, z, v[q]);
+                }
+            }
         }
+        __syncwarp();
     }
 }
 
