@@ -427,6 +427,7 @@ void splitk_reduce(int M, int N, int splits, const double *part, double *C, int 
 // ---------------------------------------------------------------------------
 __global__ void k_copy2d(int m, int n, const double *src, int lds, double *dst, int ldd)
 {
+    chain_wait();
     size_t total = (size_t)m * n;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -447,6 +448,7 @@ __global__ void k_copy2d_trans(int m, int n, const double *src, int lds, double 
 
 __global__ void k_set2d(int m, int n, double off, double diag, double *dst, int ldd, int uplo)
 {
+    chain_wait();
     size_t total = (size_t)m * n;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -469,6 +471,7 @@ __global__ void k_sub2d(int m, int n, const double *src, int lds, double *dst, i
 
 __global__ void k_flip_rows(int nrows, int n, const double *S, double *X, int ldx, int upper)
 {
+    chain_wait();
     size_t total = (size_t)nrows * n;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -480,6 +483,7 @@ __global__ void k_flip_rows(int nrows, int n, const double *S, double *X, int ld
 
 __global__ void k_flip_cols(int m, int n, const double *S, double *X, int ldx)
 {
+    chain_wait();
     size_t total = (size_t)m * n;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -498,7 +502,7 @@ void copy2d(int m, int n, const double *src, int lds, double *dst, int ldd)
 {
     if (m <= 0 || n <= 0) return;
     trace_begin();
-    k_copy2d<<<ew_blocks((long long)m * n), 256, 0, stream()>>>(m, n, src, lds, dst, ldd);
+    launch_chained(k_copy2d, dim3(ew_blocks((long long)m * n)), 256, 0, m, n, src, lds, dst, ldd);
     note_launch("copy2d");
 }
 void copy2d_trans(int m, int n, const double *src, int lds, double *dst, int ldd)
@@ -510,7 +514,7 @@ void copy2d_trans(int m, int n, const double *src, int lds, double *dst, int ldd
 void set2d(int m, int n, double off, double diag, double *dst, int ldd, int uplo)
 {
     if (m <= 0 || n <= 0) return;
-    k_set2d<<<ew_blocks((long long)m * n), 256, 0, stream()>>>(m, n, off, diag, dst, ldd, uplo);
+    launch_chained(k_set2d, dim3(ew_blocks((long long)m * n)), 256, 0, m, n, off, diag, dst, ldd, uplo);
     note_launch("set2d");
 }
 void sub2d(int m, int n, const double *src, int lds, double *dst, int ldd)
@@ -522,14 +526,14 @@ void sub2d(int m, int n, const double *src, int lds, double *dst, int ldd)
 void flip_rows(int nrows, int n, const double *S, double *X, int ldx, int upper)
 {
     if (nrows <= 0 || n <= 0) return;
-    k_flip_rows<<<ew_blocks((long long)nrows * n), 256, 0, stream()>>>(nrows, n, S, X, ldx, upper);
+    launch_chained(k_flip_rows, dim3(ew_blocks((long long)nrows * n)), 256, 0, nrows, n, S, X, ldx, upper);
     note_launch("flip_rows");
 }
 void flip_cols(int m, int n, const double *S, double *X, int ldx)
 {
     if (m <= 0 || n <= 0) return;
     trace_begin();
-    k_flip_cols<<<ew_blocks((long long)m * n), 256, 0, stream()>>>(m, n, S, X, ldx);
+    launch_chained(k_flip_cols, dim3(ew_blocks((long long)m * n)), 256, 0, m, n, S, X, ldx);
     note_launch("flip_cols");
 }
 
@@ -554,6 +558,7 @@ __global__ void k_trsm_left_lower_unit(int M, int N, const double *L, int ldl, d
 __global__ void __launch_bounds__(128) k_trsm_left_lower_unit_warp(int M, int N, const double *L, int ldl, double *B,
                                                                    int ldb)
 {
+    chain_wait();
     const int lane = threadIdx.x & 31, c = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (c >= N) return;
     double *b = B + (size_t)c * ldb;
@@ -573,7 +578,7 @@ void trsm_left_lower_unit(int M, int N, const double *L, int ldl, double *B, int
 {
     if (M <= 1 || N <= 0) return;
     if (M <= 64) {
-        k_trsm_left_lower_unit_warp<<<ceil_div(N, 4), 128, 0, stream()>>>(M, N, L, ldl, B, ldb);
+        launch_chained(k_trsm_left_lower_unit_warp, dim3(ceil_div(N, 4)), 128, 0, M, N, L, ldl, B, ldb);
         note_launch("trsm_left_lower_unit");
         return;
     }
@@ -746,6 +751,7 @@ __global__ void k_trsm_right_lower_unit_trans(int M, int N, double alpha, const 
 __global__ void __launch_bounds__(256) k_trsm_right_lower_unit_trans_warp(int M, int N, double alpha, const double *L,
                                                                           int ldl, double *B, int ldb)
 {
+    chain_wait();
     __shared__ double Ls[64 * 64];
     for (int idx = threadIdx.x; idx < N * N; idx += 256) {
         const int r = idx % N, c = idx / N;
@@ -771,7 +777,7 @@ void trsm_right_lower_unit_trans(int M, int N, double alpha, const double *L, in
 {
     if (M <= 0 || N <= 0) return;
     if (N <= 64) {
-        k_trsm_right_lower_unit_trans_warp<<<ceil_div(M, 8), 256, 0, stream()>>>(M, N, alpha, L, ldl, B, ldb);
+        launch_chained(k_trsm_right_lower_unit_trans_warp, dim3(ceil_div(M, 8)), 256, 0, M, N, alpha, L, ldl, B, ldb);
         note_launch("trsm_right_lower_unit_trans");
         return;
     }
@@ -856,6 +862,8 @@ constexpr int SLD = 65;  // leading dimension of the 64 x 64 blocks in shared me
 // reduction and columns of dependent global loads), 64 us here.
 __global__ void __launch_bounds__(512) k_potrf_small(int n, double *A, int lda, int *status)
 {
+    chain_open();
+    chain_wait();
     extern __shared__ double G[];  // (r, c) at r * SLD + c: a warp's lanes run along a row
     __shared__ int s_bad;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -922,7 +930,7 @@ void potrf_upper(int n, double *A, int lda, bool record_breakdown)
         st = (int *)p;
     }
     if (n <= 64)
-        k_potrf_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, A, lda, st);
+        launch_chained(k_potrf_small, dim3(1), 512, 64 * SLD * sizeof(double), n, A, lda, st);
     else
         k_potrf_upper<<<1, 256, 0, stream()>>>(n, A, lda, st);
     note_launch("potrf_upper");
@@ -972,6 +980,8 @@ __global__ void k_lu_sign(int n, double *T, int ldt, double *S, int *status)
 __global__ void __launch_bounds__(512) k_lu_sign_small(int n, double *T, int ldt, double *S, double *A, int lda,
                                                        int *status)
 {
+    chain_open();
+    chain_wait();
     extern __shared__ double G[];  // column-major, SLD
     __shared__ double s_sgn[64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1045,7 +1055,7 @@ void lu_sign(int n, double *T, int ldt, double *S)
 {
     if (n <= 0) return;
     if (n <= 64)
-        k_lu_sign_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, T, ldt, S, nullptr, 0, status_ptr());
+        launch_chained(k_lu_sign_small, dim3(1), 512, 64 * SLD * sizeof(double), n, T, ldt, S, nullptr, 0, status_ptr());
     else
         k_lu_sign<<<1, 256, 0, stream()>>>(n, T, ldt, S, status_ptr());
     note_launch("lu_sign");
@@ -1055,7 +1065,7 @@ bool lu_sign_tile(int n, double *T, int ldt, double *S, double *A, int lda)
 {
     if (n > 64) return false;
     if (n <= 0) return true;
-    k_lu_sign_small<<<1, 512, 64 * SLD * sizeof(double), stream()>>>(n, T, ldt, S, A, lda, status_ptr());
+    launch_chained(k_lu_sign_small, dim3(1), 512, 64 * SLD * sizeof(double), n, T, ldt, S, A, lda, status_ptr());
     note_launch("lu_sign");
     return true;
 }

@@ -33,6 +33,7 @@ namespace oz {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_colmax_exp(int m, int n, const double *A, int lda, int *colexp, int *status)
 {
+    chain_wait();
     const int c = blockIdx.y;
     const unsigned long long *col = (const unsigned long long *)(A + (size_t)c * lda);
     const size_t nth = (size_t)gridDim.x * blockDim.x, t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -121,6 +122,7 @@ constexpr int GRAM_NT = 512;
 
 __global__ void __launch_bounds__(GRAM_NT, 1) k_ozaki_gram(GramArgs g, int *status)
 {
+    chain_wait();
     if (g.pred && !*g.pred) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t empty_b[G_STAGES], full_b[G_STAGES], tfree;
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(GRAM_NT, 1) k_ozaki_gram(GramArgs g, int *stat
 __global__ void k_gram_reduce(int n, int nparts, const long long *partial, const int *colexp, double *G, int ldg,
                               const int *pred)
 {
+    chain_wait();
     if (pred && !*pred) return;
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int idx = gid >> 3, l = gid & 7;
@@ -391,6 +394,7 @@ constexpr int MAP_NT = 512;
 
 __global__ void __launch_bounds__(MAP_NT, 1) k_ozaki_map(MapArgs args, int *status)
 {
+    chain_wait();
     if (args.pred && !*args.pred) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sA = smem;
@@ -635,6 +639,7 @@ __global__ void __launch_bounds__(MAP_NT, 1) k_ozaki_map(MapArgs args, int *stat
 template <bool kScales>
 __global__ void __launch_bounds__(MAP_NT, 1) k_ozaki_map_pre(MapArgs args, int *status)
 {
+    chain_wait();
     if (args.pred && !*args.pred) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sA = smem;
@@ -906,6 +911,7 @@ __global__ void __launch_bounds__(MAP_NT, 1) k_ozaki_map_pre(MapArgs args, int *
 __global__ void __launch_bounds__(256) k_scales_rc(int m, int n, const double *A, int lda, int *colexp, int *rexp,
                                                    int *status)
 {
+    chain_wait();
     __shared__ int s_cmax[64];
     if (threadIdx.x < 64) s_cmax[threadIdx.x] = 0;
     __syncthreads();
@@ -1012,10 +1018,10 @@ int ozaki_gram(int m, int n, const double *A, int lda, double *G, int ldg, doubl
         if (rexp_out) {
             // the row scales too, for a following row map of A
             const int tiles = (m + 2047) / 2048, gx = tiles < sm_count() * 8 ? tiles : sm_count() * 8;
-            oz::k_scales_rc<<<gx > 0 ? gx : 1, 256, 0, st>>>(m, n, A, lda, colexp, rexp_out, status_ptr());
+            launch_chained(oz::k_scales_rc, dim3(gx > 0 ? gx : 1), 256, 0, m, n, A, lda, colexp, rexp_out, status_ptr());
         } else {
             const int gx = (sm_count() * 8 + n - 1) / n;  // ~8 CTAs per SM over all columns
-            oz::k_colmax_exp<<<dim3(gx, n), 256, 0, st>>>(m, n, A, lda, colexp, status_ptr());
+            launch_chained(oz::k_colmax_exp, dim3(gx, n), 256, 0, m, n, A, lda, colexp, status_ptr());
         }
         note_launch("ozaki_colmax");
     }
@@ -1027,7 +1033,7 @@ int ozaki_gram(int m, int n, const double *A, int lda, double *G, int ldg, doubl
     if (rows_per_override > 0) rows_per = (rows_per_override + oz::G_KC - 1) / oz::G_KC * oz::G_KC;
     if (g_map_path != 1 && ozaki_gram_tma(m, n, A, lda, rows_per, colexp, partial, parts, pred)) {
         trace_begin();
-        oz::k_gram_reduce<<<(n * n * 8 + 255) / 256, 256, 0, st>>>(n, parts, partial, colexp, G, ldg, pred);
+        launch_chained(oz::k_gram_reduce, dim3((n * n * 8 + 255) / 256), 256, 0, n, parts, partial, colexp, G, ldg, pred);
         note_launch("ozaki_gram_reduce");
         return 0;
     }
@@ -1041,10 +1047,10 @@ int ozaki_gram(int m, int n, const double *A, int lda, double *G, int ldg, doubl
     ga.colexp = colexp;
     ga.partial = partial;
     ga.pred = pred;
-    oz::k_ozaki_gram<<<parts, oz::GRAM_NT, smem, st>>>(ga, status_ptr());
+    launch_chained(oz::k_ozaki_gram, dim3(parts), oz::GRAM_NT, smem, ga, status_ptr());
     note_launch("ozaki_gram");
     trace_begin();
-    oz::k_gram_reduce<<<(n * n * 8 + 255) / 256, 256, 0, st>>>(n, parts, partial, colexp, G, ldg, pred);
+    launch_chained(oz::k_gram_reduce, dim3((n * n * 8 + 255) / 256), 256, 0, n, parts, partial, colexp, G, ldg, pred);
     note_launch("ozaki_gram_reduce");
     return 0;
 }
@@ -1084,11 +1090,11 @@ int ozaki_map(int m, int n, const double *A, int lda, const double *X, int ldx, 
             attr = true;
         }
         if (colexp_out || rexp_out)
-            oz::k_ozaki_map_pre<true><<<grid, oz::MAP_NT, smem, stream()>>>(ma, status_ptr());
+            launch_chained(oz::k_ozaki_map_pre<true>, dim3(grid), oz::MAP_NT, smem, ma, status_ptr());
         else
-            oz::k_ozaki_map_pre<false><<<grid, oz::MAP_NT, smem, stream()>>>(ma, status_ptr());
+            launch_chained(oz::k_ozaki_map_pre<false>, dim3(grid), oz::MAP_NT, smem, ma, status_ptr());
     } else {
-        oz::k_ozaki_map<<<grid, oz::MAP_NT, smem, stream()>>>(ma, status_ptr());
+        launch_chained(oz::k_ozaki_map, dim3(grid), oz::MAP_NT, smem, ma, status_ptr());
     }
     note_launch("ozaki_map");
     return 0;

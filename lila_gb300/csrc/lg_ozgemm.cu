@@ -12,9 +12,10 @@
 // exact integer sum assembled once to FP64 (rounded to nearest).  The error of
 // an entry is below 2^-50 (max|a| sum|b| + sum|a| max|b|) over its K range.
 //
-// CTA = 256 threads, output tile 128 x 64, K in stages of 32 through a
+// CTA = 512 threads, output tile 128 x 64, K in stages of 32 through a
 // two-stage SMEM ring (96 KB per stage: A digits 8 x 128 x 32 BF16, B digits
 // 8 x 64 x 32), so the split of stage k+1 overlaps the MMAs of stage k.
+// Operands that several tiles use are split once beforehand and copied.
 // Split-K (grid z) writes FP64 partial products; a reduction kernel adds them
 // and applies the epilogue, as the FP64 GEMM does.
 #include <math.h>

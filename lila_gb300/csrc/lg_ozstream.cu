@@ -96,6 +96,7 @@ template <bool kIntAsm>
 __global__ void __launch_bounds__(TR_THREADS, 1)
     k_map_tma(const __grid_constant__ CUtensorMap tmA, const MapTmaArgs a, int *status)
 {
+    chain_wait();
     if (a.pred && !*a.pred) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t raw_full[TR_NRAW], raw_empty[TR_NRAW], dig_full[TR_NDIG], dig_empty[TR_NDIG],
@@ -468,6 +469,7 @@ struct GramTmaArgs {
 __global__ void __launch_bounds__(GT_NT, 1)
     k_gram_tma(const __grid_constant__ CUtensorMap tmA, const GramTmaArgs g, int *status)
 {
+    chain_wait();
     if (g.pred && !*g.pred) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t empty_b[GT_DIG], full_b[GT_DIG], raw_full[GT_RAW], raw_empty[GT_RAW], tfree;
@@ -761,9 +763,9 @@ bool ozaki_map_tma(int m, int n, const double *A, int lda, const double *X, int 
     ozs::MapTmaArgs args{m, n, X, ldx, nout, out, ldo, colexp_out, pred};
     trace_begin();
     if (int_asm)
-        ozs::k_map_tma<true><<<grid, ozs::TR_THREADS, ozs::TR_SMEM, stream()>>>(tm, args, status_ptr());
+        launch_chained(ozs::k_map_tma<true>, dim3(grid), ozs::TR_THREADS, ozs::TR_SMEM, tm, args, status_ptr());
     else
-        ozs::k_map_tma<false><<<grid, ozs::TR_THREADS, ozs::TR_SMEM, stream()>>>(tm, args, status_ptr());
+        launch_chained(ozs::k_map_tma<false>, dim3(grid), ozs::TR_THREADS, ozs::TR_SMEM, tm, args, status_ptr());
     note_launch("ozaki_map");
     return true;
 }
@@ -783,7 +785,7 @@ bool ozaki_gram_tma(int m, int n, const double *A, int lda, int rows_per, const 
     }
     ozs::GramTmaArgs args{m, n, rows_per, colexp, partial, pred};
     trace_begin();
-    ozs::k_gram_tma<<<parts, ozs::GT_NT, ozs::GT_SMEM, stream()>>>(tm, args, status_ptr());
+    launch_chained(ozs::k_gram_tma, dim3(parts), ozs::GT_NT, ozs::GT_SMEM, tm, args, status_ptr());
     note_launch("ozaki_gram");
     return true;
 }

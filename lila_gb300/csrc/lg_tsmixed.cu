@@ -118,6 +118,7 @@ static int sample_count(int ml, int stride) { return (ml + stride - 1) / stride;
 
 __global__ void k_gather_rows(int ns, int n, int stride, const double *A, int lda, double *As)
 {
+    chain_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ns) return;
     const size_t r = (size_t)s * stride;
@@ -131,6 +132,7 @@ __global__ void k_gather_rows(int ns, int n, int stride, const double *A, int ld
 __global__ void __launch_bounds__(128) k_res_sample(int ns, int n, int stride, const double *As, const double *Q,
                                                     int ldq, const double *R, int ldr, double *acc)
 {
+    chain_wait();
     __shared__ double Rs[64 * 64];
     __shared__ double red[2][4];
     for (int k = threadIdx.x; k < 64 * 64; k += blockDim.x) {
@@ -186,6 +188,8 @@ __global__ void __launch_bounds__(128) k_res_sample(int ns, int n, int stride, c
 __global__ void k_check_decide(int n, const double *E, int lde, double *acc, double tol, const PassCtl *ctl,
                                int *status, int fail_bits)
 {
+    chain_open();
+    chain_wait();
     __shared__ double red[8];
     double v = 0.0;
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
@@ -293,6 +297,8 @@ static void reconstruct_small(int n, int i0, int mt, MixedWs &w, double *T, int 
 // ---------------------------------------------------------------------------
 __global__ void k_pass_init(PassCtl *c)
 {
+    chain_open();
+    chain_wait();
     c->active = 1;
     c->plain_run = 0;
     c->passes = 0;
@@ -477,6 +483,8 @@ __global__ void __launch_bounds__(FP_NT, 1)
     k_factor_pass(int n, const double *G, int ldg, double *Rk, int ldk, double *X, int ldx, PassCtl *ctl,
                   int variant, double shift_factor, double cond_limit, int *status)
 {
+    chain_open();
+    chain_wait();
     if (!ctl->active) {
         if (threadIdx.x == 0) ctl->ran = 0;
         return;
@@ -563,6 +571,7 @@ __global__ void __launch_bounds__(FP_NT, 1)
 // ran: CTA j forms column j (thread i: sum_{q = i}^{j} Rk(i, q) R(q, j)).
 __global__ void k_rk_r(int n, const double *Rk, double *R, const PassCtl *ctl)
 {
+    chain_wait();
     if (!ctl->ran) return;
     __shared__ double col[64];
     const int j = blockIdx.x, i = threadIdx.x;
@@ -588,11 +597,11 @@ static void factor_pass_dev(int n, MixedWs &w, PassCtl *ctl, int variant, double
 {
     factor_pass_attr();
     trace_begin();
-    k_factor_pass<<<1, FP_NT, FP_SMEM, stream()>>>(n, w.G, n, w.Rk, n, w.X, n, ctl, variant, shift_factor, 1e7,
+    launch_chained(k_factor_pass, dim3(1), FP_NT, FP_SMEM, n, w.G, n, w.Rk, n, w.X, n, ctl, variant, shift_factor, 1e7,
                                                    status_ptr());
     note_launch("factor_pass");
     trace_begin();
-    k_rk_r<<<n, 64, 0, stream()>>>(n, w.Rk, w.R, ctl);
+    launch_chained(k_rk_r, dim3(n), 64, 0, n, w.Rk, w.R, ctl);
     note_launch("factor_rk_r");
 }
 
@@ -612,7 +621,12 @@ __device__ PassCtl d_prim_ctl;
 // The pass control of the last leaf, kept for lila_gpu_last_variant /
 // lila_gpu_last_passes (copied on the device when the leaf ends).
 __device__ PassCtl d_last_ctl;
-__global__ void k_keep_ctl(const PassCtl *c) { d_last_ctl = *c; }
+__global__ void k_keep_ctl(const PassCtl *c)
+{
+    chain_open();
+    chain_wait();
+    d_last_ctl = *c;
+}
 
 // Read on the library stream (stream-ordered, so that it waits for nothing
 // but this thread's own work, not for copies on other streams).
@@ -661,10 +675,10 @@ static int check_result(int ml, int n, const double *Qii, int ldq, const double 
     cudaMemsetAsync(w.chk, 0, 2 * sizeof(double), st);
     trace_break();
     trace_begin();
-    k_res_sample<<<(ns + 31) / 32, 128, 0, st>>>(ns, n, stride, w.As, Qii, ldq, Rtop, ldr, w.chk);
+    launch_chained(k_res_sample, dim3((ns + 31) / 32), 128, 0, ns, n, stride, w.As, Qii, ldq, Rtop, ldr, w.chk);
     note_launch("check_residual");
     trace_begin();
-    k_check_decide<<<1, 256, 0, st>>>(n, E, n, w.chk, tol, ctl, status_ptr(), fail_bits);
+    launch_chained(k_check_decide, dim3(1), 256, 0, n, E, n, w.chk, tol, ctl, status_ptr(), fail_bits);
     note_launch("check_decide");
     // one read of res, orth, the verdict and the pass control's end state, into
     // page-locked memory of this host thread
@@ -696,7 +710,7 @@ static int mixed_leaf(int m, int n, int i, int mt, double *A, int lda, double *T
     // R = I
     set2d(n, n, 0.0, 1.0, w.R, n, 0);
     trace_begin();
-    k_pass_init<<<1, 1, 0, stream()>>>(w.ctl);
+    launch_chained(k_pass_init, dim3(1), 1, 0, w.ctl);
     note_launch("pass_init");
     // kMaxPasses passes are enqueued; those after the last one the device
     // decides on do nothing.  The candidate is A for the first pass and the
@@ -720,7 +734,7 @@ static int mixed_leaf(int m, int n, int i, int mt, double *A, int lda, double *T
         }
     }
     trace_begin();
-    k_keep_ctl<<<1, 1, 0, stream()>>>(w.ctl);
+    launch_chained(k_keep_ctl, dim3(1), 1, 0, w.ctl);
     note_launch("pass_keep");
     g_last_fallback = 0;
     g_last_check[0] = g_last_check[1] = -1.0;
@@ -734,7 +748,7 @@ static int mixed_leaf(int m, int n, int i, int mt, double *A, int lda, double *T
     if (level > 0) {
         // A is intact until the V map below writes over it
         trace_begin();
-        k_gather_rows<<<(ns + 127) / 128, 128, 0, stream()>>>(ns, n, stride, Aii, lda, w.As);
+        launch_chained(k_gather_rows, dim3((ns + 127) / 128), 128, 0, ns, n, stride, Aii, lda, w.As);
         note_launch("check_gather");
     }
     if (ml > n) ozaki_map(ml - n, n, Qii + n, ldq, w.MV, n, n, Aii + n, lda, nullptr, nullptr, rexp ? rexp + n : nullptr);
