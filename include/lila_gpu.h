@@ -30,8 +30,8 @@ int lila_gpu_sync(void);
 int lila_gpu_status(void);
 int lila_gpu_clear_status(void);
 int lila_gpu_version(void);
-/* Clock-cycle limit of the device-side grid-barrier waits of the cooperative
- * Householder panel (default 4e9, about 2 s at 2 GHz): a wait that reaches it
+/* Clock-cycle limit of the device-side waits of the cooperative Householder
+ * panel's CTAs for one another (default 4e9, about 2 s at 2 GHz): a wait that reaches it
  * sets LILA_ST_WAIT_TIMEOUT and its kernel returns.  cycles <= 0 keeps the
  * setting.  Returns the previous limit. */
 long long lila_gpu_set_wait_limit(long long cycles);
@@ -144,12 +144,13 @@ int lila_gpu_tsqr_autotune(int m, int n, double *A, int lda, double *T, int ldt,
 
 /* Batched least squares: count independent problems min ||A_t x - B_t||
  * (A_t m_t x n_t with m_t >= n_t, nrhs <= 8 right-hand sides), the reference's
- * least-squares driver per instance (least-squares/main_ls_qr3.c:94-119) in
- * one persistent launch.  m, n, lda, ldb and the pointer arrays A, B (device
+ * least-squares driver per instance (least-squares/main_ls_qr3.c:94-119) in up
+ * to three launches: instances that would outlast the others on one SM go to
+ * clusters of eight or four CTAs, the rest to one CTA each.  m, n, lda, ldb and the pointer arrays A, B (device
  * addresses) are host arrays; x overwrites B_t(0:n_t, :), V and R overwrite
  * A_t, info[t] (device) is 0 or k when R(k,k) is exactly zero.  prepare uploads
  * the batch description into work (lila_query_dgels_batched(count) bytes);
- * run is one capturable launch; graph captures run into a CUDA graph that
+ * run only enqueues (it can be captured); graph captures run into a CUDA graph that
  * lila_gpu_graph_launch replays. */
 long long lila_query_dgels_batched(int count);
 int lila_dgels_batched_prepare(int count, const int *m, const int *n, int nrhs, double *const *A,
@@ -159,7 +160,7 @@ int lila_dgels_batched_run(int count, int nrhs, void *work, int *info);
 void *lila_dgels_batched_graph(int count, int nrhs, void *work, int *info);
 int lila_gpu_graph_launch(void *exec);
 int lila_gpu_graph_destroy(void *exec);
-/* Autotuner of the persistent launch (threads per CTA, CTAs per SM): times the
+/* Autotuner of the one-CTA launch (threads per CTA, CTAs per SM): times the
  * candidates on the prepared batch, restoring A and B from the saved copies
  * before each, and keeps the fastest; returns threads * 100 + CTAs per SM. */
 int lila_gpu_gels_autotune(int count, int nrhs, void *work, int *info, double *const *Asave,

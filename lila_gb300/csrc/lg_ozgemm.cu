@@ -652,6 +652,7 @@ __global__ void __launch_bounds__(OZT, 1)
     k_ozgemm(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e, double *part,
              int *status)
 {
+    chain_wait();
     OZG_SHARED;
     const int kbeg = blockIdx.z * kchunk;
     tile<false>(x, M, N, blockIdx.x * BM, blockIdx.y * BN, kbeg, min(K, kbeg + kchunk), A, B, C, ldc, e,
@@ -665,6 +666,7 @@ __global__ void __launch_bounds__(OZT, 1)
     k_ozgemm_pre(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e, double *part,
                  int *status, PreSplit preA, PreSplit preB, const int *rexp, const int *cexp)
 {
+    chain_wait();
     OZG_SHARED;
     const int kbeg = blockIdx.z * kchunk;
     tile<true>(x, M, N, blockIdx.x * BM, blockIdx.y * BN, kbeg, min(K, kbeg + kchunk), A, B, C, ldc, e,
@@ -690,6 +692,7 @@ __global__ void __launch_bounds__(OZT + 32, 1)
     k_ozgemm_pp(int M, int N, int K, double *C, int ldc, GemmEpi e, int *status, PreSplit preA, PreSplit preB,
                 const int *rexp, const int *cexp, int tiles_m, int total)
 {
+    chain_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t copy_b[NSTAGE], empty_b[NSTAGE], acc_b, tfree;
     __shared__ uint32_t tmem_base_s;
@@ -860,6 +863,7 @@ constexpr int PRE_KP = 64;   // K values per CTA of the scale pass
 
 __global__ void __launch_bounds__(256) k_pre_scales(PreJobs P)
 {
+    chain_wait();
     const PreJob J = P.j[blockIdx.z];
     const int ppc = (P.kchunk + PRE_KP - 1) / PRE_KP, z = blockIdx.y / ppc;
     const int k0 = z * P.kchunk + (blockIdx.y % ppc) * PRE_KP;
@@ -886,6 +890,7 @@ __global__ void __launch_bounds__(256) k_pre_scales(PreJobs P)
 // 64 rows x 32 K values per CTA (256 units of 8 values, one per thread).
 __global__ void __launch_bounds__(256) k_pre_split(PreJobs P)
 {
+    chain_wait();
     const PreJob J = P.j[blockIdx.z];
     const int st = blockIdx.y, k0 = st * KC, z = k0 / P.kchunk, x0 = blockIdx.x * 64;
     const int pad = (J.rows + J.tile - 1) / J.tile * J.tile;
@@ -1021,10 +1026,10 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
         cudaMemsetAsync(exps, 0, nexp * sizeof(int), st);
         const int xb = cdiv(P.j[0].dig && (!P.j[1].dig || M > N) ? cdiv(M, ozg::BM) * ozg::BM : cdiv(N, ozg::BN) * ozg::BN, 64);
         trace_begin();
-        ozg::k_pre_scales<<<dim3(xb, splits * cdiv(kchunk, ozg::PRE_KP), 2), 256, 0, st>>>(P);
+        launch_chained(ozg::k_pre_scales, dim3(xb, splits * cdiv(kchunk, ozg::PRE_KP), 2), 256, 0, P);
         note_launch("ozgemm_pre_scales");
         trace_begin();
-        ozg::k_pre_split<<<dim3(xb, cdiv(K, ozg::KC), 2), 256, 0, st>>>(P);
+        launch_chained(ozg::k_pre_split, dim3(xb, cdiv(K, ozg::KC), 2), 256, 0, P);
         note_launch("ozgemm_pre_split");
         const ozg::PreSplit sA{P.j[0].dig, cdiv(K, ozg::KC)}, sB{P.j[1].dig, cdiv(K, ozg::KC)};
         cudaFuncSetAttribute(ozg::k_ozgemm_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
@@ -1034,15 +1039,15 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
             const long long total = (long long)grid.x * grid.y;
             const int ctas = total < sm_count() ? (int)total : sm_count();
-            kern<<<ctas, ozg::OZT + 32, ozg::SMEM, st>>>(M, N, K, C, ldc, e, status_ptr(), sA, sB, P.j[0].exps, P.j[1].exps,
+            launch_chained(kern, dim3(ctas), ozg::OZT + 32, ozg::SMEM, M, N, K, C, ldc, e, status_ptr(), sA, sB, P.j[0].exps, P.j[1].exps,
                                                         (int)grid.x, (int)total);
         } else
-            ozg::k_ozgemm_pre<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr(), sA, sB,
+            launch_chained(ozg::k_ozgemm_pre, grid, ozg::OZT, ozg::SMEM, M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr(), sA, sB,
                                                             P.j[0].exps, P.j[1].exps);
     } else {
         cudaFuncSetAttribute(ozg::k_ozgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
         trace_begin();
-        ozg::k_ozgemm<<<grid, ozg::OZT, ozg::SMEM, st>>>(M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr());
+        launch_chained(ozg::k_ozgemm, grid, ozg::OZT, ozg::SMEM, M, N, K, kchunk, A, B, C, ldc, e, p, status_ptr());
     }
     note_launch(tag);
     if (splits > 1) splitk_reduce(M, N, splits, part, C, ldc, e);
