@@ -257,11 +257,11 @@ int mixed_leaf_entry(int m, int n, int i, int mt, double *A, int lda, double *T,
 // launched by launch_chained may be placed on the SMs while the one before it
 // drains, and waits in chain_wait (before its first read or write of global
 // memory) until that one has completed.  chain_open lets the next one in once
-// every block has come to it or ended.  691 such launches of a 1413 x 692 recursive QR:
-// 10.03 -> 8.12 ms, with the fused reduction of gemm_times_tri; the tall leaf's
-// 78 on 20,001 x 48: 0.94 -> 0.79 ms.  A kernel of one block opens at its start,
+// every block has come to it or ended: a kernel of one block opens at its start,
 // one that fills the SMs after its main loop or not at all (its end).  Both do
-// nothing in a kernel launched otherwise.
+// nothing in a kernel launched otherwise.  691 such launches of a 1413 x 692
+// recursive QR: 10.03 -> 8.12 ms, with the fused reduction of gemm_times_tri; the
+// tall leaf's 78 on 20,001 x 48: 0.94 -> 0.79 ms.
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
