@@ -22,7 +22,7 @@
 // but costs G FP64 additions per column and CTA: 7.1 us per column at 4000 x
 // 64 against 4.8 us this way (11.7 us before, with 5 shuffle additions per
 // column and a counter barrier).
-// The exchange has no separate barrier: a value travels as two 8-byte words
+// The exchange has no separate barrier: a value travels as two 64-bit words
 // of (32 data bits, 32-bit column tag), and its reader polls until both tags
 // are column j's.  Slots alternate between two buffers: a slot of column j is
 // written again for column j + 2 only by a CTA that has every total of column
@@ -56,53 +56,68 @@ __host__ __device__ inline int lanes_for(int threads, int n)
 __host__ __device__ inline int pad_ld(int rows, int lanes) { return ((rows - lanes + 15) / 16 * 16) + lanes; }
 
 // ---- tagged slots -----------------------------------------------------------
-__device__ __forceinline__ void slot_put(uint4 *p, double v, uint32_t tag)
+// A slot is two 64-bit words, (tag, low half) and (tag, high half) of the value:
+// flags travelling in the data words, as NCCL's published low-latency (LL)
+// protocol has them.  The vector accesses are of 64-bit elements because only an
+// element is a single access (PTX, vector data types): a word comes with its own
+// tag or not at all, whereas four 32-bit elements may be seen one without the
+// other.
+struct __align__(16) Slot {
+    unsigned long long lo, hi;
+};
+__device__ __forceinline__ void slot_put(Slot *p, double v, uint32_t tag)
 {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(tag),
-                 "r"(__double2hiint(v)), "r"(tag)
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.volatile.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (uint32_t)__double2loint(v)),
+                 "l"(t | (uint32_t)__double2hiint(v))
                  : "memory");
 }
-__device__ __forceinline__ uint4 slot_get(const uint4 *p)
+__device__ __forceinline__ Slot slot_get(const Slot *p)
 {
-    uint4 w;
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p) : "memory");
+    Slot w;
+    asm volatile("ld.volatile.global.v2.b64 {%0, %1}, [%2];" : "=l"(w.lo), "=l"(w.hi) : "l"(p) : "memory");
     return w;
 }
+__device__ __forceinline__ bool slot_ready(const Slot &w, uint32_t tag)
+{
+    return (uint32_t)(w.lo >> 32) == tag && (uint32_t)(w.hi >> 32) == tag;
+}
+__device__ __forceinline__ double slot_value(const Slot &w) { return __hiloint2double((int)w.hi, (int)w.lo); }
 
 // The value of slot p once it holds `tag`; false when the wait gave up.
-__device__ __forceinline__ bool slot_wait(const uint4 *p, uint32_t tag, long long limit, double &v)
+__device__ __forceinline__ bool slot_wait(const Slot *p, uint32_t tag, long long limit, double &v)
 {
-    uint4 w = slot_get(p);
-    if (w.y != tag || w.w != tag) {
+    Slot w = slot_get(p);
+    if (!slot_ready(w, tag)) {
         const long long t0 = clock64();
         do {
             if (clock64() - t0 > limit) return false;
             w = slot_get(p);
-        } while (w.y != tag || w.w != tag);
+        } while (!slot_ready(w, tag));
     }
-    v = __hiloint2double((int)w.z, (int)w.x);
+    v = slot_value(w);
     return true;
 }
 
 // Sum over the warp of the slots p[0 .. G) once each holds `tag` (lane l adds
 // p[l], p[l + 32], .., then a butterfly); false when the wait gave up.
-__device__ __forceinline__ bool slots_sum(const uint4 *p, int lane, int G, uint32_t tag, long long limit, double &sum)
+__device__ __forceinline__ bool slots_sum(const Slot *p, int lane, int G, uint32_t tag, long long limit, double &sum)
 {
     constexpr int B = 5;  // loads in flight: 160 CTAs
     sum = 0.0;
     bool ok = true;
     for (int q0 = 0; q0 < G && ok; q0 += B * 32) {
-        uint4 w[B];
+        Slot w[B];
         const long long t0 = clock64();
         for (;;) {
             bool ready = true;
 #pragma unroll
             for (int u = 0; u < B; u++) {
-                w[u] = make_uint4(0, tag, 0, tag);
+                w[u] = Slot{(unsigned long long)tag << 32, (unsigned long long)tag << 32};
                 if (q0 + u * 32 + lane < G) w[u] = slot_get(p + q0 + u * 32 + lane);
             }
 #pragma unroll
-            for (int u = 0; u < B; u++) ready = ready && w[u].y == tag && w[u].w == tag;
+            for (int u = 0; u < B; u++) ready = ready && slot_ready(w[u], tag);
             if (__all_sync(0xffffffffu, ready)) break;
             if (__any_sync(0xffffffffu, clock64() - t0 > limit)) {
                 ok = false;
@@ -111,7 +126,7 @@ __device__ __forceinline__ bool slots_sum(const uint4 *p, int lane, int G, uint3
         }
 #pragma unroll
         for (int u = 0; u < B; u++)
-            if (q0 + u * 32 < G) sum += __hiloint2double((int)w[u].z, (int)w[u].x);
+            if (q0 + u * 32 < G) sum += slot_value(w[u]);
     }
     sum = group_sum<32>(sum);
     return ok;
@@ -123,7 +138,7 @@ __host__ __device__ inline long long slot_buffer(int nb, int G) { return (long l
 
 template <int LG>
 __global__ void __launch_bounds__(NT, 1)
-    k_panel(int m, int nb, int rpb, double *A, int lda, double *tau, double *Gram, uint4 *slots, int *status,
+    k_panel(int m, int nb, int rpb, double *A, int lda, double *tau, double *Gram, Slot *slots, int *status,
             long long limit, uint32_t tag_skew)
 {
     extern __shared__ double X[];  // nb columns, ld
@@ -143,8 +158,8 @@ __global__ void __launch_bounds__(NT, 1)
     // one past the warp's last column, 0 for a warp without columns
     const int wc1 = warp * (32 / LG) < nb ? min(nb, (warp + 1) * (32 / LG)) : 0;
     for (int j = 0; j < nb; j++) {
-        uint4 *buf = slots + (size_t)(j & 1) * slot_buffer(nb, G);
-        uint4 *total = buf + (size_t)nb * G, *pivot = total + nb;
+        Slot *buf = slots + (size_t)(j & 1) * slot_buffer(nb, G);
+        Slot *total = buf + (size_t)nb * G, *pivot = total + nb;
         const uint32_t tag = j + 1 + tag_skew;
         const bool owner = j >= r0 && j < r0 + nr;
         const double *xj = X + j * ld;
@@ -437,7 +452,7 @@ static bool panel_coop_launch(int m, int nb, double *A, int lda, double *T, int 
     double *tau = work;
     double *Gram = tau + nb;
     // slots on a 16-byte boundary (work is at least 8-byte aligned)
-    uint4 *slots = (uint4 *)(((uintptr_t)(Gram + (size_t)nb * nb) + 15) & ~(uintptr_t)15);
+    pnl::Slot *slots = (pnl::Slot *)(((uintptr_t)(Gram + (size_t)nb * nb) + 15) & ~(uintptr_t)15);
     const long long nslots = 2 * pnl::slot_buffer(nb, G);
     const int lg = pnl::lanes_for(pnl::NT, nb);
     const size_t smem = (size_t)pnl::pad_ld(rpb, lg) * nb * sizeof(double);
@@ -449,7 +464,7 @@ static bool panel_coop_launch(int m, int nb, double *A, int lda, double *T, int 
         return false;
     }
     trace_break();
-    cudaMemsetAsync(slots, 0, (size_t)nslots * sizeof(uint4), st);
+    cudaMemsetAsync(slots, 0, (size_t)nslots * sizeof(pnl::Slot), st);
     int *status = status_ptr();
     long long limit = wait_limit();
     void *args[] = {(void *)&m,    (void *)&nb,    (void *)&rpb,    (void *)&A,     (void *)&lda,     (void *)&tau,
