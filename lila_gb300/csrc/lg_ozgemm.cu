@@ -356,8 +356,9 @@ __device__ __forceinline__ void ctx_close(TileCtx &x)
     // normally every commit has been waited on by the flushes; after an
     // abort wait (bounded) for the issuer's last MMAs before freeing TMEM
     if (x.last_commit >= 0) tc::mbar_wait(&x.empty_b[x.last_commit & 1], (x.last_commit >> 1) & 1);
-    // and for the copies still writing shared memory
-    if (x.last_copy >= 0) tc::mbar_wait(&x.copy_b[x.last_copy & 1], (x.last_copy >> 1) & 1);
+    // and for the copies still writing shared memory, one per buffer at most
+    // (the MMAs waited for theirs; those of a stage given up did not)
+    for (int s = x.last_copy; s >= 0 && s > x.last_copy - NSTAGE; s--) tc::mbar_wait(&x.copy_b[s & 1], (s >> 1) & 1);
     tc::fence_before_sync();
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(x.tbase, 512);
@@ -758,12 +759,11 @@ __global__ void __launch_bounds__(OZT + 32, 1)
                     // refill the other buffer once its MMAs are done
                     if (g >= 1) ok = make();
                 }
-            // a give-up leaves copies and MMAs in flight: wait (bounded) for them
-            if (!ok) {
-                if (made > 0) tc::mbar_wait(&copy_b[(made - 1) & 1], ((made - 1) >> 1) & 1);
-                if (made > 1) tc::mbar_wait(&copy_b[(made - 2) & 1], ((made - 2) >> 1) & 1);
-                if (g > 0) tc::mbar_wait(&empty_b[(g - 1) & 1], ((g - 1) >> 1) & 1);
-            }
+            // whatever was started is over before shared and tensor memory are
+            // given up, whichever thread gave up (bounded; done already in a run
+            // that went through)
+            for (int s = made - 1; s >= 0 && s >= made - NSTAGE; s--) tc::mbar_wait(&copy_b[s & 1], (s >> 1) & 1);
+            if (g > 0) tc::mbar_wait(&empty_b[(g - 1) & 1], ((g - 1) >> 1) & 1);
         }
         __syncwarp();
     } else {
