@@ -20,6 +20,8 @@
 // and applies the epilogue, as the FP64 GEMM does.
 #include <math.h>
 
+#include <algorithm>
+
 #include "lg_common.cuh"
 #include "lg_tc.cuh"
 #include "lg_ozdigits.cuh"
@@ -861,55 +863,61 @@ __device__ __forceinline__ bool along_x(const PreJob &J) { return J.isA ? J.X.tr
 
 constexpr int PRE_KP = 64;   // K values per CTA of the scale pass
 
-__global__ void __launch_bounds__(256) k_pre_scales(PreJobs P)
+// Both passes walk their K steps over grid.y, which holds 65,535 blocks at most
+// (two million K values of the digits, four of the scales).
+__global__ void __launch_bounds__(256) k_pre_scales(PreJobs P, int steps)
 {
     chain_wait();
     const PreJob J = P.j[blockIdx.z];
-    const int ppc = (P.kchunk + PRE_KP - 1) / PRE_KP, z = blockIdx.y / ppc;
-    const int k0 = z * P.kchunk + (blockIdx.y % ppc) * PRE_KP;
-    const int k1 = min(min(k0 + PRE_KP, (z + 1) * P.kchunk), P.K), x0 = blockIdx.x * 64;
-    if (!J.dig || x0 >= J.rows || k0 >= k1) return;
-    int *out = J.exps + (size_t)z * J.rows;
-    if (along_x(J)) {
-        const int x = x0 + (threadIdx.x & 63);
-        int mx = 0;
-#pragma unroll 4
-        for (int k = k0 + (threadIdx.x >> 6); k < k1; k += 4) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
-        if (x < J.rows && mx) atomicMax(&out[x], mx);
-    } else {
-        for (int x = x0 + (threadIdx.x >> 5); x < min(x0 + 64, J.rows); x += 8) {
+    const int ppc = (P.kchunk + PRE_KP - 1) / PRE_KP, x0 = blockIdx.x * 64;
+    if (!J.dig || x0 >= J.rows) return;
+    for (int step = blockIdx.y; step < steps; step += gridDim.y) {
+        const int z = step / ppc, k0 = z * P.kchunk + (step % ppc) * PRE_KP;
+        const int k1 = min(min(k0 + PRE_KP, (z + 1) * P.kchunk), P.K);
+        if (k0 >= k1) continue;
+        int *out = J.exps + (size_t)z * J.rows;
+        if (along_x(J)) {
+            const int x = x0 + (threadIdx.x & 63);
             int mx = 0;
 #pragma unroll 4
-            for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
-            mx = __reduce_max_sync(0xffffffffu, mx);
-            if ((threadIdx.x & 31) == 0 && mx) atomicMax(&out[x], mx);
+            for (int k = k0 + (threadIdx.x >> 6); k < k1; k += 4) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
+            if (x < J.rows && mx) atomicMax(&out[x], mx);
+        } else {
+            for (int x = x0 + (threadIdx.x >> 5); x < min(x0 + 64, J.rows); x += 8) {
+                int mx = 0;
+#pragma unroll 4
+                for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) mx = max(mx, oz::bexp(pre_bits(J, x, k, k1)));
+                mx = __reduce_max_sync(0xffffffffu, mx);
+                if ((threadIdx.x & 31) == 0 && mx) atomicMax(&out[x], mx);
+            }
         }
     }
 }
 
-// 64 rows x 32 K values per CTA (256 units of 8 values, one per thread).
+// 64 rows x 32 K values per CTA and stage (256 units of 8 values, one per thread).
 __global__ void __launch_bounds__(256) k_pre_split(PreJobs P)
 {
     chain_wait();
     const PreJob J = P.j[blockIdx.z];
-    const int st = blockIdx.y, k0 = st * KC, z = k0 / P.kchunk, x0 = blockIdx.x * 64;
+    const int stages = (P.K + KC - 1) / KC, x0 = blockIdx.x * 64;
     const int pad = (J.rows + J.tile - 1) / J.tile * J.tile;
-    if (!J.dig || x0 >= pad || k0 >= P.K) return;
-    const int kend = min(P.K, (z + 1) * P.kchunk);
+    if (!J.dig || x0 >= pad) return;
     const int kg = along_x(J) ? threadIdx.x >> 6 : threadIdx.x & 3, xi = along_x(J) ? threadIdx.x & 63 : threadIdx.x >> 2;
-    const int x = x0 + xi, emax = x < J.rows ? J.exps[(size_t)z * J.rows + x] : 0;
-    unsigned long long v[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = pre_bits(J, x, k0 + kg * 8 + i, kend);
-    uint32_t a01[NS], a23[NS], b01[NS], b23[NS];
-    digits4(v, emax, a01, a23);
-    digits4(v + 4, emax, b01, b23);
+    const int x = x0 + xi, idx = x % J.tile;
     const uint32_t slice = J.isA ? A_SLICE : B_SLICE, bytes = J.isA ? A_BYTES : B_BYTES;
-    const int idx = x % J.tile;
-    uint8_t *base = J.dig + ((size_t)(x / J.tile) * ((P.K + KC - 1) / KC) + st) * bytes + (idx >> 3) * SBO + kg * LBO +
-                    (idx & 7) * 16;
+    for (int st = blockIdx.y; st < stages; st += gridDim.y) {
+        const int k0 = st * KC, z = k0 / P.kchunk, kend = min(P.K, (z + 1) * P.kchunk);
+        const int emax = x < J.rows ? J.exps[(size_t)z * J.rows + x] : 0;
+        unsigned long long v[8];
 #pragma unroll
-    for (int s = 0; s < NS; s++) *(uint4 *)(base + s * slice) = make_uint4(a01[s], a23[s], b01[s], b23[s]);
+        for (int i = 0; i < 8; i++) v[i] = pre_bits(J, x, k0 + kg * 8 + i, kend);
+        uint32_t a01[NS], a23[NS], b01[NS], b23[NS];
+        digits4(v, emax, a01, a23);
+        digits4(v + 4, emax, b01, b23);
+        uint8_t *base = J.dig + ((size_t)(x / J.tile) * stages + st) * bytes + (idx >> 3) * SBO + kg * LBO + (idx & 7) * 16;
+#pragma unroll
+        for (int s = 0; s < NS; s++) *(uint4 *)(base + s * slice) = make_uint4(a01[s], a23[s], b01[s], b23[s]);
+    }
 }
 
 // Grouped form: CTA b runs tile b - prefix[g] of group g, prefix[g] <= b <
@@ -1026,10 +1034,11 @@ void ozgemm(int M, int N, int K, Operand A, Operand B, double *C, int ldc, const
         cudaMemsetAsync(exps, 0, nexp * sizeof(int), st);
         const int xb = cdiv(P.j[0].dig && (!P.j[1].dig || M > N) ? cdiv(M, ozg::BM) * ozg::BM : cdiv(N, ozg::BN) * ozg::BN, 64);
         trace_begin();
-        launch_chained(ozg::k_pre_scales, dim3(xb, splits * cdiv(kchunk, ozg::PRE_KP), 2), 256, 0, P);
+        const int steps = splits * cdiv(kchunk, ozg::PRE_KP);
+        launch_chained(ozg::k_pre_scales, dim3(xb, std::min(steps, 65535), 2), 256, 0, P, steps);
         note_launch("ozgemm_pre_scales");
         trace_begin();
-        launch_chained(ozg::k_pre_split, dim3(xb, cdiv(K, ozg::KC), 2), 256, 0, P);
+        launch_chained(ozg::k_pre_split, dim3(xb, std::min(cdiv(K, ozg::KC), 65535), 2), 256, 0, P);
         note_launch("ozgemm_pre_split");
         const ozg::PreSplit sA{P.j[0].dig, cdiv(K, ozg::KC)}, sB{P.j[1].dig, cdiv(K, ozg::KC)};
         cudaFuncSetAttribute(ozg::k_ozgemm_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ozg::SMEM);
