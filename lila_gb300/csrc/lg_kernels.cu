@@ -690,13 +690,12 @@ __global__ void __launch_bounds__(128) k_trsm_right_upper_rows(int M, int N, dou
             double t = v[c];
 #pragma unroll
             for (int p = 0; p < c; p++) t = fma(-v[p], Us[p + c * 64], t);
-            const double inv = s_inv[c], d = s_d[c];
-            if (s_plain[c]) {
-                v[c] = t * inv;
-                v[c] = fma(fma(-v[c], d, t), inv, v[c]);
-            } else {
+            const double inv = s_inv[c], d = s_d[c], q = t * inv;
+            // the residual of an infinite quotient is no number
+            if (s_plain[c] && ((__double2hiint(q) >> 20) & 0x7FF) != 0x7FF)
+                v[c] = fma(fma(-q, d, t), inv, q);
+            else
                 v[c] = t / d;
-            }
             b[(size_t)c * ldb] = v[c];
         }
     }

@@ -1,0 +1,43 @@
+"""Quotients that leave the FP64 range in the kernels that multiply by a
+reciprocal and correct by the residual: an overflow is an infinity, as a division
+gives it, and what is finite is unaffected."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(got, exp, tol):
+    """The same infinities and NaNs, finite entries within tol of their column's largest."""
+    assert np.array_equal(np.isnan(got), np.isnan(exp))
+    inf, fin = np.isinf(exp), np.isfinite(exp)
+    assert np.array_equal(np.isinf(got), inf) and np.array_equal(got[inf], exp[inf])
+    assert np.all(np.abs(got[fin] - exp[fin]) <= tol * np.abs(exp[fin]).max())
+
+
+@pytest.mark.parametrize("n", [1, 3, 33, 64])
+def test_triangular_solve_of_many_rows(gpu_lib, n):
+    """x U = b row by row in divisions: 2^600 / 2^-600 and an infinite b."""
+    import torch
+
+    L = gpu_lib
+    m = 5000
+    rng = np.random.default_rng(n)
+    U = np.asfortranarray(np.triu(rng.uniform(-1.0, 1.0, (n, n)), 1) / n + np.diag(rng.uniform(1.0, 2.0, n)))
+    U[n - 1, n - 1] = -(2.0 ** -600)
+    B = rng.uniform(1.0, 2.0, (m, n)) * np.where(rng.random((m, n)) < 0.5, -1.0, 1.0)
+    B[::7, n - 1] *= 2.0 ** 600
+    B[1, 0], B[2, n // 2], B[3, n - 1] = np.inf, -np.inf, np.nan
+    B = np.asfortranarray(B)
+    X = B.copy()
+    with np.errstate(all="ignore"):
+        for c in range(n):
+            for p in range(c):
+                X[:, c] -= X[:, p] * U[p, c]
+            X[:, c] /= U[c, c]
+    assert np.isinf(X[::7, n - 1]).any()
+    dU, dB = L.to_device_colmajor(U), L.to_device_colmajor(B)
+    assert L.prim_trsm_right_upper(m, n, 1.0, dU, n, dB, m, None) == 0
+    torch.cuda.synchronize()
+    # n products and a quotient of entries of one size, each rounded once
+    _same(L.from_device(dB), X, 4 * n * 2.0 ** -53)
