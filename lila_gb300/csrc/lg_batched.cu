@@ -475,10 +475,13 @@ struct Solver {
             for (int k = nk - 1; k >= 0; k--) {
                 const double cur = col;
                 if (k > 0 && on) col = A[(size_t)r + (size_t)(32 * q + k - 1) * lda];
-                // lane k: y / d, the quotient corrected by one residual step
+                // lane k: y / d, the quotient corrected by one residual step (an
+                // infinite one has none)
                 double x = y * inv;
-                if (plain) x = fma(fma(-x, d, y), inv, x);
-                if (!plain) x = is_bad ? NAN : y / d;
+                if (plain && bexp_of(x) != 0x7FF)
+                    x = fma(fma(-x, d, y), inv, x);
+                else
+                    x = is_bad ? NAN : y / d;
                 x = __shfl_sync(0xffffffffu, x, k);
                 if (lane == k) y = x;
                 if (lane < k) y = fma(-cur, x, y);

@@ -41,3 +41,31 @@ def test_triangular_solve_of_many_rows(gpu_lib, n):
     torch.cuda.synchronize()
     # n products and a quotient of entries of one size, each rounded once
     _same(L.from_device(dB), X, 4 * n * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 40])
+def test_batched_back_substitution(gpu_lib, n):
+    """R x = y with x_n = 2^600 / 2^-600, A its own R (nothing below a diagonal)."""
+    import torch
+
+    L = gpu_lib
+    R = np.diag(np.arange(1.0, n + 1.0))
+    R[n - 1, n - 1] = 2.0 ** -600
+    R[: n - 1, n - 1] = np.where(np.arange(n - 1) % 3 == 0, -2.0, 0.5)
+    b = np.arange(2.0, n + 2.0)[:, None]
+    b[n - 1] = 2.0 ** 600
+    x = b.copy()
+    with np.errstate(all="ignore"):
+        for k in range(n - 1, -1, -1):  # column by column, as BLAS solves it
+            x[k] /= R[k, k]
+            x[:k, 0] -= R[:k, k] * x[k, 0]
+    assert np.isinf(x[n - 1])
+    dA, dB = L.to_device_colmajor(np.asfortranarray(R)), L.to_device_colmajor(np.asfortranarray(b))
+    nb = L.lib().lila_query_dgels_batched(1)
+    work = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    info = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    assert L.dgels_batched_prepare(1, [n], [n], 1, [dA], [n], [dB], [n], work, nb) == 0
+    assert L.dgels_batched_run(1, 1, work, info) == 0
+    torch.cuda.synchronize()
+    assert info.item() == 0
+    assert np.array_equal(L.from_device(dB), x, equal_nan=True)
