@@ -879,14 +879,20 @@ __global__ void __launch_bounds__(512) k_potrf_small(int n, double *A, int lda, 
             if (lane == 0) s_bad = j;
             return;
         }
-        const double y = rsqrt_nr(d);
-        double root = d * y;
-        root = fma(0.5 * y, fma(-root, root, d), root);
+        // an infinite pivot is its own root, and the row then holds what t / inf is
+        const bool finite = __double2hiint(d) != 0x7FF00000;
+        const double y = finite ? rsqrt_nr(d) : 0.0;
+        double root = d;
+        if (finite) {
+            root = d * y;
+            root = fma(0.5 * y, fma(-root, root, d), root);
+        }
         __syncwarp();
         for (int c = j + lane; c < n; c += 32) {
             const double t = G[j * SLD + c];
             double u = t * y;
-            u = fma(fma(-u, root, t), y, u);  // t / root to rounding level
+            // t / root to rounding level (an infinite quotient has no residual)
+            if (finite && ((__double2hiint(u) >> 20) & 0x7FF) != 0x7FF) u = fma(fma(-u, root, t), y, u);
             G[j * SLD + c] = c == j ? root : u;
         }
     };

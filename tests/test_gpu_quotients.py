@@ -8,11 +8,11 @@ pytestmark = pytest.mark.gpu
 
 
 def _same(got, exp, tol):
-    """The same infinities and NaNs, finite entries within tol of their column's largest."""
+    """The same infinities and NaNs, finite entries within tol of the largest."""
     assert np.array_equal(np.isnan(got), np.isnan(exp))
     inf, fin = np.isinf(exp), np.isfinite(exp)
     assert np.array_equal(np.isinf(got), inf) and np.array_equal(got[inf], exp[inf])
-    assert np.all(np.abs(got[fin] - exp[fin]) <= tol * np.abs(exp[fin]).max())
+    assert np.all(np.abs(got[fin] - exp[fin]) <= tol * np.abs(exp[fin]).max(initial=0.0))
 
 
 @pytest.mark.parametrize("n", [1, 3, 33, 64])
@@ -69,3 +69,30 @@ def test_batched_back_substitution(gpu_lib, n):
     torch.cuda.synchronize()
     assert info.item() == 0
     assert np.array_equal(L.from_device(dB), x, equal_nan=True)
+
+
+@pytest.mark.parametrize("n,k", [(1, 0), (2, 0), (33, 5), (64, 31), (64, 63), (70, 5)])
+def test_cholesky_with_an_infinite_pivot(gpu_lib, n, k):
+    """An infinite diagonal entry is a positive pivot: its row is zero right of
+    the root, the rows below go on, and nothing breaks down."""
+    import torch
+
+    L = gpu_lib
+    rng = np.random.default_rng(n + k)
+    X = rng.standard_normal((n, 2 * n))
+    A = np.asfortranarray(X @ X.T)
+    A[k, k] = np.inf
+    R = np.triu(A)
+    for j in range(n):
+        R[j, j] = np.sqrt(R[j, j])
+        R[j, j + 1:] /= R[j, j]
+        for r in range(j + 1, n):
+            R[r, r:] -= R[j, r] * R[j, r:]
+    assert np.isfinite(np.delete(R.diagonal(), k)).all()
+    dA = L.to_device_colmajor(A)
+    L.gpu_clear_status()
+    assert L.prim_potrf_upper(n, dA, n) == 0
+    torch.cuda.synchronize()
+    assert L.gpu_status() == 0
+    # n products and a quotient per entry; the matrix is well conditioned
+    _same(np.triu(L.from_device(dA)), R, 64 * n * 2.0 ** -53)
