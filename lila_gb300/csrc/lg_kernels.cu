@@ -998,9 +998,11 @@ __global__ void __launch_bounds__(512) k_lu_sign_small(int n, double *T, int ldt
     auto pivot_col = [&](int k) {  // warp 0
         double *g = G + k * SLD;
         const double t = g[k];
-        // |1 - t| < |1 + t| in FP64 is t > 2^-54, an integer comparison
+        // |1 - t| < |1 + t| in FP64 is t > 2^-54, an integer comparison, up to
+        // 2^53; past that the rounding of both sides decides
         const long long tb = __double_as_longlong(t);
-        const bool neg = tb > 0x3C90000000000000ll && tb <= 0x7FF0000000000000ll;
+        const bool wide = ((tb >> 52) & 0x7FF) >= 1023 + 53;
+        const bool neg = wide ? fabs(1.0 - t) < fabs(1.0 + t) : tb > 0x3C90000000000000ll;
         const long long flip = neg ? (long long)0x8000000000000000ull : 0ll;
         const double p = __longlong_as_double(tb ^ flip) - 1.0, inv = -rcp_nr(-p);
         __syncwarp();
@@ -1011,7 +1013,10 @@ __global__ void __launch_bounds__(512) k_lu_sign_small(int n, double *T, int ldt
             double l = a;
             if (r0 + 31 > k) {  // some row of the warp below the pivot
                 l = a * inv;
-                l = fma(fma(-l, p, a), inv, l);
+                if (wide)
+                    l = a / p;
+                else if (((__double2hiint(l) >> 20) & 0x7FF) != 0x7FF)  // an infinity has no residual
+                    l = fma(fma(-l, p, a), inv, l);
             }
             g[r] = r < k ? a : (r == k ? p : l);
         }

@@ -96,3 +96,41 @@ def test_cholesky_with_an_infinite_pivot(gpu_lib, n, k):
     assert L.gpu_status() == 0
     # n products and a quotient per entry; the matrix is well conditioned
     _same(np.triu(L.from_device(dA)), R, 64 * n * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("n", [4, 64, 70])
+@pytest.mark.parametrize("lower", [0, 1])
+def test_sign_lu_with_large_entries(gpu_lib, n, lower):
+    """The sign of a column is the one for which |s t - 1| as FP64 rounds it is not
+    the smaller, also where t is so large that both sides round alike."""
+    import torch
+
+    L = gpu_lib
+    rng = np.random.default_rng(n + lower)
+    d = rng.uniform(-1.0, 1.0, n)
+    big = [2.0 ** 60, -(2.0 ** 60), 2.0 ** 53 + 4, 2.0 ** 53 + 2, 2.0 ** 53, 2.0 ** 53 - 1, 1e300, np.inf, -np.inf,
+           2.0 ** -54, 2.0 ** -54 * (1 + 2.0 ** -52), -(2.0 ** -54)]
+    d[: len(big)] = big[:n]
+    # nothing is subtracted: the strict triangle is quotients, or stays
+    W = rng.uniform(-1.0, 1.0, (n, n))
+    T = np.asfortranarray((np.tril(W, -1) if lower else np.triu(W, 1)) + np.diag(d))
+    if lower:
+        T[n - 1, 0] = np.inf
+    E, S = T.copy(order="F"), np.zeros(n)
+    with np.errstate(all="ignore"):
+        for k in range(n):
+            S[k] = -1.0 if abs(1.0 - E[k, k]) < abs(1.0 + E[k, k]) else 1.0
+            E[:, k] *= S[k]
+            E[k, k] -= 1.0
+            E[k + 1:, k] /= E[k, k]
+            E[k + 1:, k + 1:] -= np.outer(E[k + 1:, k], E[k, k + 1:])
+    dT, dS = L.to_device_colmajor(T), torch.zeros(n, dtype=torch.float64, device="cuda")
+    assert L.prim_lu_sign(n, dT, n, dS) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(dS.cpu().numpy(), S)
+    got = L.from_device(dT)
+    assert np.array_equal(np.isnan(got), np.isnan(E))
+    # one quotient per entry
+    ok = ~np.isnan(E)
+    with np.errstate(invalid="ignore"):
+        assert np.all((got[ok] == E[ok]) | (np.abs(got[ok] - E[ok]) <= 4 * 2.0 ** -53 * np.abs(E[ok])))
