@@ -135,6 +135,11 @@ __device__ __forceinline__ bool slots_sum(const Slot *p, int lane, int G, uint32
 // Slots of one buffer: column c's partial of CTA q at c G + q, its total at
 // nb G + c, the pivot row's entry at nb (G + 1) + c.
 __host__ __device__ inline long long slot_buffer(int nb, int G) { return (long long)nb * (G + 2); }
+// Behind the two buffers those of a column taken again: partials and totals as
+// above, then the CTAs' largest exponents.  One set is enough: the next column
+// taken again writes it after that column's own exchange, so after every CTA has
+// left this one.
+__host__ __device__ inline long long slot_count(int nb, int G) { return 2 * slot_buffer(nb, G) + (long long)nb * (G + 1) + G; }
 
 template <int LG>
 __global__ void __launch_bounds__(NT, 1)
@@ -143,13 +148,14 @@ __global__ void __launch_bounds__(NT, 1)
 {
     extern __shared__ double X[];  // nb columns, ld
     __shared__ double s_tau, s_f, s_sc[MAXNB], s_beta[MAXNB], s_d[MAXNB], s_p[MAXNB];
-    __shared__ int s_fail;
     constexpr int NW = NT / 32;
+    __shared__ int s_shift, s_below, s_e[NW], s_nz[NW];
+    __shared__ int2 s_stop;  // a wait gave up; the column has to be taken again
     const int G = gridDim.x, b = blockIdx.x;
     const int r0 = b * rpb, nr = min(m - r0, rpb), ld = pad_ld(rpb, LG);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = threadIdx.x / LG, g = threadIdx.x % LG;  // this thread's column and its lane in the group
-    if (threadIdx.x == 0) s_fail = 0;
+    if (threadIdx.x == 0) s_stop = make_int2(0, 0);
     for (int cc = warp; cc < nb; cc += NW)
         for (int r = lane; r < nr; r += 32) X[r + cc * ld] = A[(size_t)(r0 + r) + (size_t)cc * lda];
     __syncthreads();
@@ -162,15 +168,18 @@ __global__ void __launch_bounds__(NT, 1)
         Slot *total = buf + (size_t)nb * G, *pivot = total + nb;
         const uint32_t tag = j + 1 + tag_skew;
         const bool owner = j >= r0 && j < r0 + nr;
-        const double *xj = X + j * ld;
+        double *xj = X + j * ld;
         const int first = max(0, j + 1 - r0);
         // this CTA's partials (the warps of columns before j would be idle
         // now: the products for T cost nothing extra)
-        if (wc1 > 0) {
+        auto product = [&] {
             double d = 0.0;
 #pragma unroll 4
             for (int r = first + g; r < nr; r += LG) d = fma(xj[r], xc[r], d);
-            d = group_sum<LG>(d);
+            return group_sum<LG>(d);
+        };
+        if (wc1 > 0) {
+            const double d = product();
             if (mine && g == 0) {
                 slot_put(buf + (size_t)c * G + b, d, j + 1);
                 if (owner) slot_put(pivot + c, xc[j - r0], j + 1);
@@ -195,7 +204,11 @@ __global__ void __launch_bounds__(NT, 1)
         if (wc1 > j) {
             if (mine && c >= j) ok = slot_wait(pivot + c, tag, limit, pr) && slot_wait(total + c, tag, limit, d) && ok;
             if (c == j && g == 0) {
-                const Reflector h = house_reflector(pr, d, d != 0.0);
+                // house_in_range by the exponents alone, beside the reflector's
+                // chain (an FP64 compare in it cost 80 ns per column); a sum of
+                // zero is out of range, so there is something below here
+                s_stop.y = bexp_of(d) < 1023 - 930 || bexp_of(d) > 1023 + 929 || bexp_of(pr) > 1023 + 463;
+                const Reflector h = house_reflector(pr, d, true);
                 s_tau = h.tau;
                 s_f = h.tau * h.sc;
                 s_sc[j] = h.sc;
@@ -203,11 +216,85 @@ __global__ void __launch_bounds__(NT, 1)
                 if (owner) tau[j] = h.tau;
             }
         }
-        if (!ok) s_fail = 1;
+        if (!ok) s_stop.x = 1;
         __syncthreads();
-        if (s_fail) {
+        const int2 stop = s_stop;
+        if (stop.x) {
             if (threadIdx.x == 0) atomicOr(status, ST_WAIT_TIMEOUT);
             return;
+        }
+        if (stop.y) {
+            // rare, and the same in every CTA (they have the same total and pivot):
+            // rows j.. of the column by 2^-k, k its largest exponent, and the column
+            // again, as in k_qr_small
+            Slot *part = slots + 2 * slot_buffer(nb, G), *sum = part + (size_t)nb * G, *exps = sum + nb;
+            int e = 0, nz = 0;
+            for (int r = max(0, j - r0) + threadIdx.x; r < nr; r += NT) {
+                const int x = house_exponent(xj[r]);
+                if (r0 + r > j && x) nz = 1;
+                e = max(e, x);
+            }
+            e = __reduce_max_sync(0xffffffffu, e);
+            nz = __any_sync(0xffffffffu, nz);
+            if (lane == 0) {
+                s_e[warp] = e;
+                s_nz[warp] = nz;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                e = __reduce_max_sync(0xffffffffu, lane < NW ? s_e[lane] : 0);
+                nz = __any_sync(0xffffffffu, lane < NW && s_nz[lane]);
+                if (lane == 0) slot_put(exps + b, __hiloint2double(nz, e), j + 1);
+                for (int q = lane; q < G && ok; q += 32) {
+                    double v = 0.0;
+                    ok = slot_wait(exps + q, tag, limit, v);
+                    e = max(e, __double2loint(v));
+                    nz |= __double2hiint(v);
+                }
+                e = __reduce_max_sync(0xffffffffu, e);
+                nz = __any_sync(0xffffffffu, nz);
+                if (lane == 0) {
+                    s_shift = house_shift(e);
+                    s_below = nz;
+                }
+                if (!ok) s_stop.x = 1;
+            }
+            __syncthreads();
+            const int k = s_shift;
+            for (int r = max(0, j - r0) + threadIdx.x; r < nr; r += NT) xj[r] = scalbn(xj[r], -k);
+            __syncthreads();
+            if (wc1 > 0 && !s_stop.x) {
+                const double dk = product();
+                if (mine && g == 0) slot_put(part + (size_t)c * G + b, dk, j + 1);
+            }
+            for (int cc = b + warp * G; cc < nb && !s_stop.x; cc += NW * G) {
+                double dk;
+                ok = slots_sum(part + (size_t)cc * G, lane, G, tag, limit, dk) && ok;
+                if (lane == 0) {
+                    if (cc >= j)
+                        slot_put(sum + cc, dk, j + 1);
+                    else
+                        s_d[cc] = dk;
+                }
+            }
+            if (wc1 > j && !s_stop.x) {
+                if (mine && c >= j) ok = slot_wait(sum + c, tag, limit, d) && ok;
+                if (c == j && g == 0) {
+                    const Reflector h = house_reflector(scalbn(pr, -k), d, s_below != 0);
+                    s_tau = h.tau;
+                    s_f = h.tau * h.sc;
+                    s_sc[j] = h.sc;
+                    s_beta[j] = scalbn(h.beta, k);
+                    if (owner) tau[j] = h.tau;
+                }
+            }
+            __syncthreads();
+            if (!ok) s_stop.x = 1;
+            __syncthreads();
+            if (s_stop.x) {
+                if (threadIdx.x == 0) atomicOr(status, ST_WAIT_TIMEOUT);
+                return;
+            }
         }
         const double tj = s_tau, sc = s_sc[j];
         if (wc1 > j + 1 && tj != 0.0 && mine && c > j) {
@@ -419,8 +506,7 @@ __global__ void __launch_bounds__(NTS, 1)
 }  // namespace pnl
 
 // Doubles of workspace panel_coop needs for an nb-column panel (tau, the
-// Gram V^T V and the exchange slots: two buffers of 16-byte slots; the rest
-// is kept so that the workspace queries' answers stay).
+// Gram V^T V and the 16-byte exchange slots; the rest is kept so that the workspace queries' answers stay).
 long long panel_coop_work(int nb)
 {
     const long long G = sm_count();
@@ -453,7 +539,7 @@ static bool panel_coop_launch(int m, int nb, double *A, int lda, double *T, int 
     double *Gram = tau + nb;
     // slots on a 16-byte boundary (work is at least 8-byte aligned)
     pnl::Slot *slots = (pnl::Slot *)(((uintptr_t)(Gram + (size_t)nb * nb) + 15) & ~(uintptr_t)15);
-    const long long nslots = 2 * pnl::slot_buffer(nb, G);
+    const long long nslots = pnl::slot_count(nb, G);
     const int lg = pnl::lanes_for(pnl::NT, nb);
     const size_t smem = (size_t)pnl::pad_ld(rpb, lg) * nb * sizeof(double);
     const void *kern = lg == 4 ? (const void *)pnl::k_panel<4>
