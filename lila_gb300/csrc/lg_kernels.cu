@@ -63,8 +63,17 @@ __device__ __forceinline__ void epilogue_store(double v, int r, int c, double *C
 // 32 x 32 tiles with 256-deep K slices and unpipelined loads: the 617 products
 // of a 1413 x 692 recursive QR 22.1 -> 7.1 ms, the 133 of 4000 x 1000 (tiles
 // of 256) 21.6 -> 16.1 ms, the upper 64 x 64 Gram of 262,144 rows 2.23 -> 1.4 ms.
+// PARTS (K slices of more than 2 SUB terms): an output is summed in chains of SUB
+// terms, whose rounding errors grow with the chain.  The plan takes K slices for
+// their time alone, so without this the Gram's chains were as long as 4,384; with
+// it the leaf's errors fall by a quarter (262,144 x 64, A 3.3e-16 -> 2.4e-16 of
+// the largest entry, root mean square over 10 matrices) at the same time (3.62
+// ms), as the additions are outside the loop over K steps (inside it: 3.66).  The
+// 64 x 64 tile has no registers for a second set of sums; it is taken where the
+// output has many tiles.
+constexpr int SUB = 256;
 constexpr int UPPER_TILES = 2;  // upper_only on a grid without the tiles below the diagonal
-template <int BM, int BN, int BK, int TM, int TN>
+template <int BM, int BN, int BK, int TM, int TN, bool PARTS>
 __global__ void __launch_bounds__(256)
     k_gemm(int M, int N, int K, int kchunk, Operand A, Operand B, double *C, int ldc, GemmEpi e,
            double *part)
@@ -104,6 +113,20 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0;
 
+    // PARTS: sums of SUB terms, added up in `sum`
+    double sum[PARTS ? TM : 1][PARTS ? TN : 1] = {};
+    auto add_up = [&] {
+        if constexpr (PARTS) {
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) {
+                    sum[i][j] += acc[i][j];
+                    acc[i][j] = 0.0;
+                }
+        }
+    };
+
     double ra[LA], rb[LB];
     chain_wait();
     auto load = [&](int k0) {
@@ -124,41 +147,54 @@ __global__ void __launch_bounds__(256)
     };
     load(kbeg);
     int buf = 0;
-    for (int k0 = kbeg; k0 < kend; k0 += BK, buf ^= 1) {
+    int kstop = PARTS ? min(kend, kbeg + SUB) : kend;
+    for (int k0 = kbeg;;) {
+        for (; k0 < kstop; k0 += BK, buf ^= 1) {
 #pragma unroll
-        for (int u = 0; u < LA; u++) {
-            const int idx = tid + u * NTH;
-            if (A.trans == NT)
-                As[buf][idx / BM][idx % BM] = ra[u];
-            else
-                As[buf][idx % BK][idx / BK] = ra[u];
-        }
+            for (int u = 0; u < LA; u++) {
+                const int idx = tid + u * NTH;
+                if (A.trans == NT)
+                    As[buf][idx / BM][idx % BM] = ra[u];
+                else
+                    As[buf][idx % BK][idx / BK] = ra[u];
+            }
 #pragma unroll
-        for (int u = 0; u < LB; u++) {
-            const int idx = tid + u * NTH;
-            if (B.trans == NT)
-                Bs[buf][idx % BK][idx / BK] = rb[u];
-            else
-                Bs[buf][idx / BN][idx % BN] = rb[u];
-        }
-        // one barrier per step: the buffer written two steps later was last
-        // read before the barrier of the step between
-        __syncthreads();
-        if (k0 + BK < kend) load(k0 + BK);
-        if (live) {
+            for (int u = 0; u < LB; u++) {
+                const int idx = tid + u * NTH;
+                if (B.trans == NT)
+                    Bs[buf][idx % BK][idx / BK] = rb[u];
+                else
+                    Bs[buf][idx / BN][idx % BN] = rb[u];
+            }
+            // one barrier per step: the buffer written two steps later was last
+            // read before the barrier of the step between
+            __syncthreads();
+            if (k0 + BK < kend) load(k0 + BK);
+            if (live) {
 #pragma unroll
-            for (int k = 0; k < BK; k++) {
-                double a[TM], b[TN];
+                for (int k = 0; k < BK; k++) {
+                    double a[TM], b[TN];
 #pragma unroll
-                for (int i = 0; i < TM; i++) a[i] = As[buf][k][tr + i * RT];
+                    for (int i = 0; i < TM; i++) a[i] = As[buf][k][tr + i * RT];
 #pragma unroll
-                for (int j = 0; j < TN; j++) b[j] = Bs[buf][k][tc + j * CT];
+                    for (int j = 0; j < TN; j++) b[j] = Bs[buf][k][tc + j * CT];
 #pragma unroll
-                for (int i = 0; i < TM; i++)
+                    for (int i = 0; i < TM; i++)
 #pragma unroll
-                    for (int j = 0; j < TN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                        for (int j = 0; j < TN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                }
             }
         }
+        if (!PARTS) break;
+        add_up();
+        if (kstop == kend) break;
+        kstop = min(kend, kstop + SUB);
+    }
+    if constexpr (PARTS) {
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+            for (int j = 0; j < TN; j++) acc[i][j] = sum[i][j];
     }
     // Only now: blocks of the next kernel let in before would be placed where
     // this one's blocks have left room, several to some SMs and none to others
@@ -308,12 +344,14 @@ static int gemm_parts(int M, int N, int K, Operand A, Operand B, double *C, int 
         grid.y = 1;
     }
     trace_begin();
+    auto launch = [&](auto kern) { launch_chained(kern, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp); };
+    const bool parts = p.kchunk > 2 * SUB;
     if (p.tile == 64)
-        launch_chained(k_gemm<64, 64, 16, 4, 4>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        launch(k_gemm<64, 64, 16, 4, 4, false>);
     else if (p.tile == 32)
-        launch_chained(k_gemm<32, 32, 16, 2, 2>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        parts ? launch(k_gemm<32, 32, 16, 2, 2, true>) : launch(k_gemm<32, 32, 16, 2, 2, false>);
     else
-        launch_chained(k_gemm<16, 16, 32, 1, 1>, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp);
+        parts ? launch(k_gemm<16, 16, 32, 1, 1, true>) : launch(k_gemm<16, 16, 32, 1, 1, false>);
     note_launch(tag);
     return p.splits;
 }
