@@ -1201,6 +1201,44 @@ def run_reference(args, rank, world):
     }
 
 
+# What the result line keeps of the measurements beside the headline; stderr has
+# all of them.
+BRIEF = ("value", "ms_per_step", "ms_per_matrix", "ms_per_batch_median", "mats_per_s", "gflops", "gflops_credited",
+         "fallback_rate_of_all", "mixed_over_plain", "best_mixed_over_plain", "learned_over_plain",
+         "learned_over_best_fixed_variant", "passes", "res", "orth", "tol", "error")
+
+
+def _brief(x):
+    if isinstance(x, dict):
+        kept = {k: _brief(v) for k, v in x.items() if k in BRIEF or (isinstance(v, dict) and "kernels" not in k)}
+        return {k: v for k, v in kept.items() if v != {}}
+    return float("%.5g" % x) if isinstance(x, float) else x
+
+
+def result_line(out):
+    """The one-line result: the headline whole, of everything else the values (a
+    reader of the line may take a few KB only)."""
+    line = {k: v for k, v in out.items() if k != "kernels"}
+    for key in ("plain_fp64", "tsqr_fp64", "out_of_core", "workloads", "accuracy"):
+        if key in line:
+            line[key] = _brief(line[key])
+    if "e2e" in line:
+        line["e2e"] = {k: v for k, v in line["e2e"].items()
+                       if k in ("value", "unit", "ms_per_step", "steps", "h2d_bytes_per_step", "d2h_bytes_per_step",
+                                "copies_of_one_step_concurrently_ms")}
+    if "cpu_baseline" in line:
+        line["cpu_baseline"] = {k: v for k, v in line["cpu_baseline"].items()
+                                if k in ("value", "unit", "cores", "kind", "sample")}
+    if "roofline" in line:
+        line["roofline"] = {k: v for k, v in line["roofline"].items() if k != "traffic_source"}
+    # the per-condition-number times and accuracy close the line, so that
+    # a record that keeps only the line's tail still shows them
+    for key in ("per_kappa_ms", "accuracy"):
+        if key in line:
+            line[key] = line.pop(key)
+    return line
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1255,12 +1293,8 @@ def main():
                     out["workloads"][w] = run_extra(args, w)
                 except Exception as e:  # reported, never hidden: the headline line still prints
                     out["workloads"][w] = {"error": "%s: %s" % (type(e).__name__, e)}
-        # the per-condition-number times and accuracy close the line, so that
-        # a record that keeps only the line's tail still shows them
-        for key in ("per_kappa_ms", "accuracy"):
-            if key in out:
-                out[key] = out.pop(key)
-        print(json.dumps(out))
+        print("detail: " + json.dumps(out), file=sys.stderr)
+        print(json.dumps(result_line(out)))
     if world > 1:
         import torch.distributed as dist
 
