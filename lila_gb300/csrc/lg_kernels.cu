@@ -64,15 +64,19 @@ __device__ __forceinline__ void epilogue_store(double v, int r, int c, double *C
 // 32 x 32 tiles with 256-deep K slices and unpipelined loads: the 617 products
 // of a 1413 x 692 recursive QR 22.1 -> 7.1 ms, the 133 of 4000 x 1000 (tiles
 // of 256) 21.6 -> 16.1 ms, the upper 64 x 64 Gram of 262,144 rows 2.23 -> 1.4 ms.
-// PARTS (K slices of more than 2 SUB terms): an output is summed in chains of SUB
-// terms, whose rounding errors grow with the chain.  The plan takes K slices for
-// their time alone, so without this the Gram's chains were as long as 4,384; with
-// it the leaf's errors fall by a quarter (262,144 x 64, A 3.3e-16 -> 2.4e-16 of
-// the largest entry, root mean square over 10 matrices) at the same time (3.62
-// ms), as the additions are outside the loop over K steps (inside it: 3.66).  The
-// 64 x 64 tile has no registers for a second set of sums; it is taken where the
-// output has many tiles.
-constexpr int SUB = 256;
+// PARTS (K > 512, slices of more than SUB terms): an output is summed in chains
+// of SUB terms, whose rounding errors grow with the chain.  The plan takes K
+// slices for their time alone, so without this the Gram's chains were as long as
+// 4,384 and a product of 520 terms was one chain.  Errors with it against
+// double-double products (root mean square, of the largest entry): Q^T C of 520 x
+// 600 x 33 in tiles of 32 7.7e-17 -> 6.5e-17, 775 x 1852 x 40 6.4e-17 -> 5.4e-17,
+// the Cholesky QR leaf of 262,144 x 64 a quarter less (A 3.3e-16 -> 2.4e-16).  It
+// costs nothing (3.62 and 3.63 ms, 1413 x 692 8.09 ms both), as the additions are
+// outside the loop over K steps; inside it the leaf took 3.66 ms.  Chains of 160
+// take 3.634 ms, of 256 lose what is gained at 520 terms.  The 64 x 64 tile has
+// no registers for a second set of sums; it is taken where the output has many
+// tiles.
+constexpr int SUB = 192;
 constexpr int UPPER_TILES = 2;  // upper_only on a grid without the tiles below the diagonal
 template <int BM, int BN, int BK, int TM, int TN, bool PARTS>
 __global__ void __launch_bounds__(256)
@@ -346,7 +350,7 @@ static int gemm_parts(int M, int N, int K, Operand A, Operand B, double *C, int 
     }
     trace_begin();
     auto launch = [&](auto kern) { launch_chained(kern, grid, 256, 0, M, N, K, p.kchunk, A, B, C, ldc, ek, pp); };
-    const bool parts = p.kchunk > 2 * SUB;
+    const bool parts = K > 512 && p.kchunk > SUB;
     if (p.tile == 64)
         launch(k_gemm<64, 64, 16, 4, 4, false>);
     else if (p.tile == 32)

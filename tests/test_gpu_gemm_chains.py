@@ -1,5 +1,5 @@
 """The FP64 GEMM's long sums (Grams and updates of tall blocks) run in chains of
-256 terms: equal terms whose running sum rounds the same way every time, against
+at most 256 terms: equal terms whose running sum rounds the same way every time, against
 the exact sum.  A chain of n terms may be off by n u: 256 of them, at most 64
 chains in a K slice here and at most 128 slices."""
 import pytest
