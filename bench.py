@@ -966,7 +966,7 @@ def run_batched(L, torch, count=10000, steps=3, warmup=1, klo=1.0, khi=12.0, p_r
     flops = sum(b.flops() for b in batches) / len(batches)
     out["flops_per_batch"] = flops
     b0 = batches[0]
-    # ---- plain FP64: the batched Householder solver, one persistent launch in a CUDA graph
+    # ---- plain FP64: the batched Householder solver, up to three launches in a CUDA graph
     wbytes = L.lib().lila_query_dgels_batched(count)
     work = torch.empty(wbytes, dtype=torch.uint8, device="cuda")
     info = torch.zeros(count, dtype=torch.int32, device="cuda")
@@ -981,7 +981,7 @@ def run_batched(L, torch, count=10000, steps=3, warmup=1, klo=1.0, khi=12.0, p_r
         L.gpu_graph_destroy(graph)
     plain_acc = _ls_summary(batches[-1], skip_rankdef=True)
     pm = float(np.median(plain_ms))
-    out["plain_fp64"] = {"path": "lila_dgels_batched (FP64 Householder, persistent kernel, CUDA graph)",
+    out["plain_fp64"] = {"path": "lila_dgels_batched (FP64 Householder, CUDA graph)",
                          "ms_per_batch_median": pm, "mats_per_s": count / (pm * 1e-3),
                          "gflops": flops / (pm * 1e-3) / 1e9, "accuracy": plain_acc}
 

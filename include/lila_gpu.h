@@ -44,7 +44,8 @@ int lila_gpu_trace_summary(char *buf, int len);
 
 /* Precision of the library's large products (FP64 GEMMs of the block
  * reflector updates, panels, explicit Q; those of M, N, K >= 16 that are
- * faster there, from about 25 million multiply-adds): LILA_PRECISION_FP64
+ * faster there, from about 19 million multiply-adds where the dimensions fill
+ * the 128 x 64 x 32 tiles, later where they do not): LILA_PRECISION_FP64
  * (default) runs them on the FP64 CUDA cores; LILA_PRECISION_SPLIT runs them as FP64-grade split-precision products
  * on the BF16 tensor cores (eight base-128 digits per value, exact integer
  * accumulation, error below 2^-50 (max|a| sum|b| + sum|a| max|b|) per entry).

@@ -32,7 +32,7 @@ int lila_prim_potrf_upper(int n, double *A, int lda);
 int lila_prim_lu_sign(int n, double *T, int ldt, double *S);
 int lila_prim_larfg(int m, double *x, double *tau);
 /* The pivot step of the split leaf's FP64 factor: out[k] = 1 / sqrt(d[k])
- * (Newton-Raphson from a single-precision estimate, within about 1.5 ulp);
+ * (one third-order step from the hardware's estimate, within about 1.5 ulp);
  * 0 where d[k] is not positive and finite. */
 int lila_prim_rsqrt(int n, const double *d, double *out);
 /* One pass's factor of the split leaf (n <= 64): from the Gram G the upper

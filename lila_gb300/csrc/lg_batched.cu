@@ -1,7 +1,8 @@
 // lg_batched.cu -- thousands of independent least-squares problems
 // min ||A_t x - b_t|| (A_t m_t x n_t, m_t >= n_t, nrhs right-hand sides) in
-// one persistent launch (and one of clusters beside it when a few large
-// instances would outlast the rest).
+// up to three launches side by side: a persistent one, and before it one of
+// clusters of eight CTAs and one of four for the large instances that would
+// outlast the rest (batches of up to 32 instances per SM).
 //
 // Per instance the algorithm is the reference's least-squares driver
 // (least-squares/main_ls_qr3.c:94-119): Householder QR of A, Q^T applied to
@@ -726,7 +727,7 @@ int lila_dgels_batched_prepare(int count, const int *m, const int *n, int nrhs, 
     return 0;
 }
 
-// One persistent launch over every prepared instance (stream-capturable).
+// Up to three launches over the prepared instances (stream-capturable).
 int lila_dgels_batched_run(int count, int nrhs, void *work, int *info)
 {
     if (count <= 0) return 0;

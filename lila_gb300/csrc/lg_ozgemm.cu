@@ -682,11 +682,12 @@ __global__ void __launch_bounds__(OZT, 1)
 // Both operands split beforehand, no K slices: nothing is left for the tile's
 // warps but its outputs, so a persistent CTA gives copies and MMAs to one thread
 // of a 17th warp and the other 16 warps only fold tensor memory and assemble.
-// The MMAs of a tile start as soon as the previous tile's sums are in registers:
-// its 8,192 outputs (an int64 -> FP64 conversion and a beta FMA each, ~10,000
-// clocks of the FP64 pipe) are assembled while the next 128 K are multiplied
-// (~12,000 clocks).  16384 x 8192 x 128: 2,674 us with a CTA per tile, which does
-// one after the other, 1,152 this way.
+// The MMAs of a tile (12,000 clocks) start as soon as the previous tile's sums
+// are in registers, so that its 8,192 outputs are assembled beside them; folding
+// the sums, which the next MMAs wait for, is not hidden, and a tile takes 22,000
+// clocks.  No unit is full (8192 x 8192 x 128: tensor pipe 46 %, FP64 26 %, L2
+// 23 %, DRAM 24 %, leading stall the wait for loads).  16384 x 8192 x 128: 2,674 us
+// with a CTA per tile, 1,152 this way.
 // ONE: K <= 128, a single window per tile: its sums go straight into one 64-bit
 // integer per output, which leaves registers for C's values, loaded while the
 // tile's MMAs run (4096 x 4864 x 128: 212 -> 185 us).

@@ -11,7 +11,7 @@
 
 namespace lg {
 
-// Clock-cycle limit of the cooperative panel's grid-barrier waits
+// Clock-cycle limit of the cooperative panel's waits for one another's slots
 // (lila_gpu_set_wait_limit); ~2 s at 2 GHz by default.
 long long g_wait_limit = 4000000000LL;
 long long wait_limit() { return g_wait_limit; }

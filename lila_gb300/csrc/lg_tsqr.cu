@@ -36,7 +36,7 @@ namespace tsqr {
 // the block in shared memory, one warp per column and a five-step shuffle
 // reduction per dot product, 131,072 x 32 (512 blocks of 256 rows, groups of 4):
 // QR 2.10 -> 0.82 ms, backward sweep 1.96 -> 0.80 ms; the 512 blocks run with
-// the FP64 pipe 65 % (QR) and 80 % (sweep) busy, the five levels above them are
+// the FP64 pipe 73 % (QR) and 95 % (sweep) busy, the five levels above them are
 // bound by their columns' chains (91 us per level, 150 before the interleaving
 // and 35 us per sweep).
 constexpr int CH = 4;  // registers skipped together
